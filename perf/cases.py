@@ -422,7 +422,7 @@ def _pm_exact(case, seed):
     on = torch.ones(nlocal, dtype=torch.bool, device=pos.device) if tag is None else tag == 1
     p = pos[:, on]
     i = (p * n).long()
-    w = (p - (i + 0.5) / n) * n
+    w = (p - (i.double() + 0.5) / n) * n
     side = torch.where(w > 0, i + 1, i - 1)
     idx = [torch.remainder(i, n), torch.remainder(side, n)]
     wt = [1.0 - w.abs(), w.abs()]
