@@ -16,6 +16,7 @@
 #include "photons_p2p.h"
 #include "p2p_internal.h"
 #include "p2p_fit.h"
+#include "p2p_fit64.h"
 #include "p2p_args.h"
 #include "p2p_launch.h"
 #include "p2p_host_shared.h"
@@ -84,6 +85,7 @@ struct p2p_session {
     std::map<std::tuple<const void *, int, size_t>, int> occupancy;
     p2p_params params{};
     PolyFit fit;
+    Fit64 fit64{};  // FP64 form
     // device buffers
     DevBuf task_t2, task_s2;  // second buffer pair of pipelined submits
     DevBuf pos, mass, leaf_ip, leaf_np, task_t, task_s, meta, pos4, counts, fill, row_off,
@@ -215,6 +217,14 @@ int default_stage(const p2p_params &p) {
     return p.stage_sources ? p.stage_sources : (p.form == P2P_FORM_PLAIN_FP64 ? 128 : 256);
 }
 
+// Warps per block. The FP64 kernel's warps share a sink leaf's row: with so
+// few leaves that the rows' length and not their number decides, eight take
+// 0.144 ms where four take 0.220 (12^3, 900 leaves); from 32^3 (3,900 leaves:
+// 0.361 ms at four, 0.379 at eight) to 110^3 four are as good or better.
+int default_warps(const p2p_session *s, const p2p_params &p) {
+    return p.form == P2P_FORM_PLAIN_FP64 && s->fit64.nfar && s->nleaf <= 16 * s->sm_count ? 8 : 4;
+}
+
 // Dispatch to the lane mapping's launcher (p2p_pair_*.cu).
 int launch_pair(p2p_session *s, const PairArgs &a) {
     const p2p_params &p = s->params;
@@ -225,12 +235,13 @@ int launch_pair(p2p_session *s, const PairArgs &a) {
     L.masses = a.mass != nullptr;
     L.acc = p.form == P2P_FORM_KAHAN_FP32 ? ACC_KAHAN : (p.form == P2P_FORM_NAIVE_FP32 ? ACC_F32 : ACC_F64);
     L.ncoef = s->fit.ncoef_kernel;
-    L.warps = p.warps_per_block ? p.warps_per_block : 4;
+    L.warps = p.warps_per_block ? p.warps_per_block : default_warps(s, p);
     L.stage = default_stage(p);
     L.blocks_per_sm = p.blocks_per_sm;
     L.dry_run = s->dry_run;
     L.occ = &s->occupancy;
     L.sink_pairs = p.kernel_variant == P2P_VARIANT_SOURCE_LANES_X2_S16 ? 8 : 16;
+    L.fit64 = &s->fit64;
     L.sreg_spl = p.kernel_variant == P2P_VARIANT_SINK_REGS8 ? 8 : 4;
     PairLaunchResult r;
     if (p.form == P2P_FORM_PLAIN_FP64)
@@ -547,6 +558,8 @@ P2P_API int p2p_session_set_params(p2p_session *s, const p2p_params *params) {
     if (s->in_pass) return fail(P2P_ERR_STATE, "cannot change parameters inside a pass");
     P2P_TRY(validate_params(params));
     s->params = *params;
+    if (params->form == P2P_FORM_PLAIN_FP64)
+        s->fit64 = fit64(params->x_cut, params->split_radius, params->soften);
     if (is_fp32_form(params->form)) {
         s->fit = fit_h(fit_umax(params->x_cut), params->poly_tol > 0.0 ? params->poly_tol : kDefaultPolyTol);
     } else {

@@ -15,6 +15,8 @@ namespace p2p {
 
 using OccupancyCache = std::map<std::tuple<const void *, int, size_t>, int>;
 
+struct Fit64;  // p2p_fit64.h
+
 struct PairLaunch {
     cudaStream_t stream;
     int sm_count;
@@ -28,6 +30,7 @@ struct PairLaunch {
     OccupancyCache *occ;
     int max_blocks = 0; // > 0: cap on the persistent grid (a share of the GPU)
     int sink_pairs = 16; // packed source-lane kernel: sink pairs per slice (16 or 8)
+    const Fit64 *fit64 = nullptr;  // FP64 form: the pair factor's polynomials (null or nfar 0: general kernel)
     int sreg_spl = 4;    // sink-register kernel: sinks per lane (4: 32-sink slices, 8: 64)
 };
 
@@ -42,6 +45,10 @@ inline size_t pair_smem_split(int warps, int stage, bool source_lanes) {
     return (size_t)warps * (stage + (source_lanes ? 32 : 0)) * 16;
 }
 inline size_t pair_smem_plain(int warps, int stage) { return (size_t)warps * stage * 32; }
+// FP64 kernel with fitted cutoff: per warp its sources and lane sums
+inline size_t pair_smem_fp64(int warps, int stage) {
+    return (size_t)warps * ((size_t)stage * 32 + 32 * 12 * 8);
+}
 // packed source-lane kernel: sink pairs, band corrections, staged sources + their indices
 inline size_t pair_smem_x2(int warps, int stage) { return (size_t)warps * (stage + 64 + stage / 4) * 16; }
 // packed sink-lane kernel: staged sources as two float4 + index, 32 padding slots

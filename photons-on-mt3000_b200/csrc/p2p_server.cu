@@ -41,6 +41,7 @@
 #include "photons_p2p.h"
 #include "p2p_args.h"
 #include "p2p_fit.h"
+#include "p2p_fit64.h"
 #include "p2p_host_shared.h"
 #include "p2p_internal.h"
 #include "p2p_launch.h"
@@ -262,6 +263,7 @@ struct p2p_server {
     int device = 0, sm_count = 0;
     p2p_params shape{};
     PolyFit fit;
+    Fit64 fit64{};  // FP64 form
     p2p_server_config cfg{};
     bool fp32 = true;
     // arena
@@ -587,6 +589,7 @@ int launch_pack(p2p_server *S, Slot &sl, const std::vector<Job> &jobs) {
     L.masses = false;
     L.acc = p.form == P2P_FORM_KAHAN_FP32 ? ACC_KAHAN : (p.form == P2P_FORM_NAIVE_FP32 ? ACC_F32 : ACC_F64);
     L.ncoef = S->fit.ncoef_kernel;
+    L.fit64 = &S->fit64;
     L.warps = p.warps_per_block ? p.warps_per_block : 4;
     L.stage = p.stage_sources ? p.stage_sources : (p.form == P2P_FORM_PLAIN_FP64 ? 128 : 256);
     L.blocks_per_sm = p.blocks_per_sm;
@@ -946,6 +949,7 @@ P2P_API int p2p_server_create(int device, const p2p_params *shape, const p2p_ser
     S->shape.mass = 1.0;
     S->cfg = c;
     S->fp32 = shape->form != P2P_FORM_PLAIN_FP64;
+    if (!S->fp32) S->fit64 = fit64(shape->x_cut, shape->split_radius, shape->soften);
     if (S->fp32)
         S->fit = fit_h(fit_umax(shape->x_cut), shape->poly_tol > 0.0 ? shape->poly_tol : kDefaultPolyTol);
     auto cleanup = [&](int st) {
