@@ -189,7 +189,7 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
     R.leaf_cap = cap;
 
     tree_init_kernel<<<init_blocks, kTreeThreads, 0, st>>>(d_pos, n, P, blo, bhi);
-    tree_root_box_kernel<<<1, 32, 0, st>>>(blo, bhi, init_blocks, boxsize, R, 0);
+    tree_root_box_kernel<<<1, 96, 0, st>>>(blo, bhi, init_blocks, boxsize, R, 0);
     launches += 2;
 
     // ---- nodes above kTreeSmall particles, level by level (host-driven) ----
@@ -232,7 +232,11 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
         TREE_CUDA(cudaMemcpyAsync(d_segs, segs.data(), sizeof(TreeSeg) * nseg, cudaMemcpyHostToDevice, st));
         TREE_CUDA(cudaMemcpyAsync(d_tile_seg, tile_seg.data(), sizeof(int) * ntile, cudaMemcpyHostToDevice, st));
         TREE_CUDA(cudaMemcpyAsync(d_tile_off, tile_off.data(), sizeof(int) * ntile, cudaMemcpyHostToDevice, st));
-        tree_seg_mean_kernel<<<nseg, kTreeThreads, 0, st>>>(d_segs, P, R);
+        const int64_t nchain = std::count_if(segs.begin(), segs.end(),
+                                             [&](const TreeSeg &g) { return tree_takes_chain(g.length, nseg); });
+        if (nchain < nseg) tree_seg_mean_kernel<<<nseg, kTreeThreads, 0, st>>>(d_segs, nseg, P, R);
+        if (nchain > 0) tree_seg_chain_kernel<<<(nseg + 3) / 4, 128, 0, st>>>(d_segs, nseg, P, R);
+        launches += (nchain < nseg ? 1 : 0) + (nchain > 0 ? 1 : 0) - 1;
         tree_tile_count_kernel<<<ntile, kTreeThreads, 0, st>>>(d_segs, d_tile_seg, d_tile_off, P, d_tile_small);
         launches += 2;
         std::vector<int> tsmall(ntile), tpre(ntile);
@@ -299,7 +303,7 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
         TREE_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(TreeTask) * tasks.size(), cudaMemcpyHostToDevice, st));
         TREE_CUDA(cudaFuncSetAttribute(tree_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kTreeSmallSmem));
-        tree_small_kernel<<<(int)tasks.size(), kTreeThreads, kTreeSmallSmem, st>>>(d_tasks, P, R, maxleaf);
+        tree_small_kernel<<<(int)tasks.size(), kTreeSmallThreads, kTreeSmallSmem, st>>>(d_tasks, P, R, maxleaf);
         launches += 1;
         TREE_CUDA(cudaGetLastError());
     }

@@ -28,7 +28,6 @@ namespace p2p {
 constexpr int kTreeSmall = 2048;       // subtrees up to this size are built by one block
 constexpr int kTreeTile = 2048;        // slots per tile of the level-wide partition
 constexpr int kTreeThreads = 256;
-constexpr int kTreeMaxStack = kTreeSmall;
 
 // Status bits of the tree build.
 enum : int {
@@ -71,15 +70,94 @@ __device__ __forceinline__ void tree_swap(TreeParts &P, int i, int j) {
     P.x[j] = tx; P.y[j] = ty; P.z[j] = tz; P.id[j] = ti;
 }
 
-// The reference's split value of a node of length >= 3: the sampled mean,
-// summed in slot order (src/fmm.c:88-97).
-__device__ __forceinline__ double tree_mean(const double *c, int length) {
-    int mul = 1;
-    if (length > 100000) mul = length / 100000;
-    double mean = 0.0;
-    for (int n = 0; n < length; n += mul) mean = __dadd_rn(mean, c[n]);
-    mean = __ddiv_rn(mean, (double)length);
-    return __dmul_rn(mean, (double)mul);
+// ------------------------------------------------------ the split value ---
+//
+// The reference's split value of a node of length >= 3 is the sampled mean,
+// summed in slot order (src/fmm.c:88-97), so its rounding is that of a chain of
+// up to 2e5 dependent FP64 additions. One thread makes one in 10 cycles (the
+// addition takes 8.4), 0.87 ms a level of a 256^3 tree as it was and 12 of the
+// tree's 26 ms. Short nodes keep the chain, many side by side; for long ones its
+// result is found in parallel, bit for bit: while the running sum stays in one
+// binade its unit in the last place u does not change, adding x moves it by x
+// rounded to a multiple of u, which (S + x) - S gives exactly for any S of that
+// binade, unless x lies half way between two multiples, where the chain rounds
+// by its own parity. Those moves and their sums are multiples of u below 2^53
+// of them, so FP64 adds them exactly in any order. A group of samples is
+// therefore applied at once when it holds no half and S stays inside its binade
+// whatever the order of the group's moves up and down; a group that might leave
+// it goes through in shorter groups and, where need be, in the chain. Binades
+// are left, and halves met, about log2(samples) times each.
+
+// S after the n samples at s (shared memory: every lane reads the same word),
+// added one by one.
+__device__ __forceinline__ double mean_chain(const double *s, int n, double S) {
+#pragma unroll 16
+    for (int i = 0; i < n; ++i) S = __dadd_rn(S, s[i]);
+    return S;
+}
+
+// The moves of a group of samples.
+struct MeanMoves {
+    double sum, size;  // their sum, and the sum of their magnitudes
+    bool half;         // one of the samples rounds by parity
+};
+
+// S's binade as [lo, 2 lo) and half its unit; false where a chain must be
+// followed sample by sample (zero, near-subnormal, huge or not finite).
+__device__ __forceinline__ bool mean_binade(double S, double &lo, double &half_u) {
+    const int e = (__double2hiint(S) >> 20) & 0x7ff;
+    lo = __hiloint2double(e << 20, 0);
+    half_u = __hiloint2double((e - 53) << 20, 0);
+    return e >= 100 && e <= 2000;
+}
+
+__device__ __forceinline__ void mean_add(MeanMoves &g, double x, double S, double half_u) {
+    const double move = __dsub_rn(__dadd_rn(S, x), S);
+    g.sum = __dadd_rn(g.sum, move);
+    g.size = __dadd_rn(g.size, fabs(move));
+    g.half = g.half || fabs(__dsub_rn(x, move)) == half_u;
+}
+
+// Whether a group of moves may be applied to S at once (NaN and infinity fail):
+// size + sum and size - sum are twice its moves up and down, exactly.
+__device__ __forceinline__ bool mean_fits(double S, double lo, double sum, double size) {
+    const double along = S < 0.0 ? -sum : sum, m = fabs(S);
+    const double less = __dmul_rn(0.5, __dsub_rn(size, along)), more = __dmul_rn(0.5, __dadd_rn(size, along));
+    return __dsub_rn(m, less) > lo && __dadd_rn(m, more) < __dadd_rn(lo, lo);
+}
+
+// The lanes' moves together (in every lane); half also where S might leave its
+// binade under them.
+__device__ __forceinline__ MeanMoves mean_gather(MeanMoves m, double S, double lo) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        m.sum = __dadd_rn(m.sum, __shfl_xor_sync(0xffffffffu, m.sum, off));
+        m.size = __dadd_rn(m.size, __shfl_xor_sync(0xffffffffu, m.size, off));
+    }
+    m.half = __any_sync(0xffffffffu, m.half) || !mean_fits(S, lo, m.sum, m.size);
+    return m;
+}
+
+// S after one warp's n samples at s (shared memory), 128 at a time.
+__device__ __forceinline__ double mean_warp(const double *s, int n, double S) {
+    const int lane = threadIdx.x & 31;
+    for (int b = 0; b < n; b += 128) {
+        const int m = min(128, n - b);
+        double lo, half_u;
+        if (mean_binade(S, lo, half_u)) {
+            MeanMoves g = {0.0, 0.0, false};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (32 * i + lane < m) mean_add(g, s[b + 32 * i + lane], S, half_u);
+            g = mean_gather(g, S, lo);
+            if (!g.half) {
+                S = __dadd_rn(S, g.sum);
+                continue;
+            }
+        }
+        S = mean_chain(s + b, m, S);
+    }
+    return S;
 }
 
 // -------------------------------------------------------------- inputs ---
@@ -124,17 +202,23 @@ __global__ void tree_init_kernel(const double *__restrict__ pos, int n, TreePart
 }
 
 // The root box: boxL = min(boxsize, min float coordinate) - 1e-6 boxsize,
-// boxH = max(0, max float coordinate) + 1e-6 boxsize, per axis (one thread).
-__global__ void tree_root_box_kernel(const float *__restrict__ block_lo, const float *__restrict__ block_hi,
-                                     int nblocks, double boxsize, TreeRec R, int root) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int d = 0; d < 3; ++d) {
-        double lo = boxsize, hi = 0.0;
-        for (int b = 0; b < nblocks; ++b) {
-            const double l = (double)block_lo[3 * b + d], h = (double)block_hi[3 * b + d];
-            if (lo > l) lo = l;
-            if (hi < h) hi = h;
-        }
+// boxH = max(0, max float coordinate) + 1e-6 boxsize, per axis (one block of
+// three warps, one axis each).
+__global__ void __launch_bounds__(96)
+tree_root_box_kernel(const float *__restrict__ block_lo, const float *__restrict__ block_hi, int nblocks,
+                     double boxsize, TreeRec R, int root) {
+    const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
+    double lo = boxsize, hi = 0.0;
+    for (int b = lane; b < nblocks; b += 32) {
+        const double l = (double)block_lo[3 * b + d], h = (double)block_hi[3 * b + d];
+        if (lo > l) lo = l;
+        if (hi < h) hi = h;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
         const double margin = __dmul_rn(0.000001, boxsize);
         R.box[6 * (size_t)root + d] = __dsub_rn(lo, margin);
         R.box[6 * (size_t)root + 3 + d] = __dadd_rn(hi, margin);
@@ -151,71 +235,166 @@ struct TreeSeg {
     int nsmall, nbig;
 };
 
-// One block per segment: the split value. The samples are gathered into
-// shared memory by the whole block, a chunk at a time, and summed in slot
-// order by one thread (the reference's rounding sequence, tree_mean).
-constexpr int kTreeMeanChunk = 4096;
-__global__ void __launch_bounds__(kTreeThreads) tree_seg_mean_kernel(TreeSeg *segs, TreeParts P, TreeRec R) {
-    __shared__ double buf[kTreeMeanChunk];
-    const TreeSeg g = segs[blockIdx.x];
+// Segments whose chain of additions is made as it is, one warp per segment:
+// short ones, and all of a level that has so many that they fill the GPU side
+// by side (at 256^3 the levels of 512 and more segments took 4.4 ms with a block
+// each).
+constexpr int kMeanChainMax = 8192;
+constexpr int kMeanChainSegs = 512;
+__host__ __device__ __forceinline__ bool tree_takes_chain(int length, int nseg) {
+    return length <= kMeanChainMax || (nseg >= kMeanChainSegs && length <= 100000);
+}
+
+__global__ void __launch_bounds__(128) tree_seg_chain_kernel(TreeSeg *segs, int nseg, TreeParts P, TreeRec R) {
+    constexpr int kBatch = 256;
+    __shared__ double batch[4][kBatch];
+    const int lane = threadIdx.x & 31;
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (q >= nseg) return;
+    const TreeSeg g = segs[q];
+    if (!tree_takes_chain(g.length, nseg)) return;
     const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
+    double *s = batch[threadIdx.x >> 5];
+    double S = 0.0, next[kBatch / 32];
+#pragma unroll
+    for (int i = 0; i < kBatch / 32; ++i) next[i] = 32 * i + lane < g.length ? c[32 * i + lane] : 0.0;
+    for (int b = 0; b < g.length; b += kBatch) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kBatch / 32; ++i) s[32 * i + lane] = next[i];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kBatch / 32; ++i) {  // in flight during the additions
+            const int k = b + kBatch + 32 * i + lane;
+            next[i] = k < g.length ? c[k] : 0.0;
+        }
+        S = mean_chain(s, min(kBatch, g.length - b), S);
+    }
+    if (lane == 0) {
+        const double mean = __ddiv_rn(S, (double)g.length);
+        segs[q].mean = mean;
+        R.split[g.node] = mean;
+    }
+}
+
+// One block per longer segment: the split value, in windows of 8 groups of 512
+// samples, a warp to a group (any lane may hold any of its samples: the loads
+// are coalesced where the samples are contiguous). Groups that fit S's binade
+// are applied by every thread; the owner of one that does not puts it in order
+// in shared memory, works it out (mean_warp) and hands S on. The other groups'
+// moves stay good while S stays in the binade they were found in.
+constexpr int kMeanPerLane = 16;
+constexpr int kMeanGroup = 32 * kMeanPerLane;
+__global__ void __launch_bounds__(kTreeThreads, 3) tree_seg_mean_kernel(TreeSeg *segs, int nseg, TreeParts P, TreeRec R) {
+    constexpr int kWarps = kTreeThreads / 32;
+    __shared__ MeanMoves groups[kWarps];
+    __shared__ double s_sum;
+    __shared__ double order[kMeanGroup];  // the group that is worked out
+    const TreeSeg g = segs[blockIdx.x];
+    if (tree_takes_chain(g.length, nseg)) return;
+    const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int mul = 1;
     if (g.length > 100000) mul = g.length / 100000;
     const int nsamp = (g.length + mul - 1) / mul;  // slots 0, mul, 2 mul, ... < length
-    double mean = 0.0;
-    for (int s0 = 0; s0 < nsamp; s0 += kTreeMeanChunk) {
-        const int ns = min(kTreeMeanChunk, nsamp - s0);
-        for (int i = threadIdx.x; i < ns; i += blockDim.x) buf[i] = c[(size_t)(s0 + i) * mul];
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int i = 0; i < ns; ++i) mean = __dadd_rn(mean, buf[i]);
-        __syncthreads();
+    double S = 0.0;  // the same in every thread
+    for (int s0 = 0; s0 < nsamp; s0 += kWarps * kMeanGroup) {
+        double x[kMeanPerLane];
+        const int first = s0 + w * kMeanGroup, last = min(nsamp, first + kMeanGroup);
+#pragma unroll
+        for (int i = 0; i < kMeanPerLane; ++i)
+            x[i] = first + 32 * i + lane < last ? c[(size_t)(first + 32 * i + lane) * mul] : 0.0;
+        const int ngroup = min(kWarps, (nsamp - s0 + kMeanGroup - 1) / kMeanGroup);
+        int cur = 0;          // groups of the window already in S
+        double found = -1.0;  // the binade that the window's moves belong to
+        while (cur < ngroup) {
+            double lo, half_u;
+            if (mean_binade(S, lo, half_u)) {
+                if (lo != found) {
+                    if (w >= cur && w < ngroup) {
+                        MeanMoves m = {0.0, 0.0, false};
+#pragma unroll
+                        for (int i = 0; i < kMeanPerLane; ++i)
+                            if (first + 32 * i + lane < last) mean_add(m, x[i], S, half_u);
+                        // moves found at this S hold at every S of the binade that they keep within it
+                        m = mean_gather(m, S, lo);
+                        if (lane == 0) groups[w] = m;
+                    }
+                    found = lo;
+                    __syncthreads();
+                }
+                while (cur < ngroup && !groups[cur].half && mean_fits(S, lo, groups[cur].sum, groups[cur].size))
+                    S = __dadd_rn(S, groups[cur++].sum);
+            }
+            if (cur < ngroup) {
+                if (w == cur) {
+#pragma unroll
+                    for (int i = 0; i < kMeanPerLane; ++i) order[32 * i + lane] = x[i];
+                    __syncwarp();
+                    S = mean_warp(order, last - first, S);
+                    if (lane == 0) s_sum = S;
+                }
+                __syncthreads();
+                S = s_sum;
+                ++cur;
+            }
+            __syncthreads();  // groups, order and s_sum are read before they are rewritten
+        }
     }
     if (threadIdx.x == 0) {
-        mean = __dmul_rn(__ddiv_rn(mean, (double)g.length), (double)mul);
+        const double mean = __dmul_rn(__ddiv_rn(S, (double)g.length), (double)mul);
         segs[blockIdx.x].mean = mean;
         R.split[g.node] = mean;
     }
 }
 
 // Tiles of kTreeTile slots: tile t covers slots [tile_off[t], +kTreeTile) of
-// segment tile_seg[t]; counts the slots not above the mean.
+// segment tile_seg[t]. A warp holds kTileRounds x 32 consecutive slots, whose
+// coordinates are all loaded before any is tested: one block barrier per tile,
+// where a loop over 256-slot rounds paid two and a load latency for each (the
+// swaps took 230 us per level at 256^3 and 28 us at any small size).
+constexpr int kTileRounds = kTreeTile / kTreeThreads;
+
+struct TileFlags {
+    unsigned small[kTileRounds];  // round r's lanes whose slot is not above the mean
+    int first;                    // this lane's slot in round 0 (relative to the segment)
+    int before, total;            // slots not above the mean: in the warps before this one; in the tile
+};
+
+__device__ __forceinline__ TileFlags tree_tile_flags(const double *c, double mean, int off, int end, int *warp_tot) {
+    TileFlags f;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    f.first = off + w * (32 * kTileRounds) + lane;
+    double v[kTileRounds];
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r) v[r] = f.first + 32 * r < end ? c[f.first + 32 * r] : 0.0;
+    int cnt = 0;
+#pragma unroll
+    for (int r = 0; r < kTileRounds; ++r) {
+        f.small[r] = __ballot_sync(0xffffffffu, f.first + 32 * r < end && !(v[r] > mean));
+        cnt += __popc(f.small[r]);
+    }
+    if (lane == 0) warp_tot[w] = cnt;
+    __syncthreads();
+    f.before = f.total = 0;
+#pragma unroll
+    for (int q = 0; q < kTreeThreads / 32; ++q) {
+        if (q < w) f.before += warp_tot[q];
+        f.total += warp_tot[q];
+    }
+    return f;
+}
+
+// Counts the tile's slots not above the mean.
 __global__ void __launch_bounds__(kTreeThreads)
 tree_tile_count_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ tile_seg,
                        const int *__restrict__ tile_off, TreeParts P, int *__restrict__ tile_small) {
-    __shared__ int red[kTreeThreads / 32];
+    __shared__ int warp_tot[kTreeThreads / 32];
     const TreeSeg g = segs[tile_seg[blockIdx.x]];
     const int off = tile_off[blockIdx.x];
-    const int end = min(g.length, off + kTreeTile);
     const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
-    int cnt = 0;
-    for (int r = off + threadIdx.x; r < end; r += blockDim.x) cnt += c[r] > g.mean ? 0 : 1;
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < kTreeThreads / 32; ++w) t += red[w];
-        tile_small[blockIdx.x] = t;
-    }
-}
-
-// Block-wide exclusive prefix of one flag per thread (kTreeThreads threads).
-__device__ __forceinline__ int tree_block_prefix(int flag, int *warp_tot, int *total) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned m = __ballot_sync(0xffffffffu, flag);
-    const int before = __popc(m & ((1u << lane) - 1u));
-    if (lane == 0) warp_tot[w] = __popc(m);
-    __syncthreads();
-    int base = 0, tot = 0;
-    for (int q = 0; q < kTreeThreads / 32; ++q) {
-        const int v = warp_tot[q];
-        if (q < w) base += v;
-        tot += v;
-    }
-    __syncthreads();
-    *total = tot;
-    return base + before;
+    const TileFlags f = tree_tile_flags(c, g.mean, off, min(g.length, off + kTreeTile), warp_tot);
+    if (threadIdx.x == 0) tile_small[blockIdx.x] = f.total;
 }
 
 // The swapped slots not above the mean: map[nsmall + q] = the slot of the
@@ -232,14 +411,16 @@ tree_tile_map_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ t
     const int end = min(g.length, off + kTreeTile);
     if (end <= g.nsmall) return;  // the whole tile lies in the left part (block-uniform)
     const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
-    int small_before = tile_pre[blockIdx.x];
-    for (int r0 = off; r0 < end; r0 += blockDim.x) {
-        const int r = r0 + threadIdx.x;
-        const bool small = r < end && !(c[r] > g.mean);
-        int tot;
-        const int rank = tree_block_prefix(small ? 1 : 0, warp_tot, &tot);
-        if (small && r >= g.nsmall) map[g.ipart + g.nsmall + (g.nsmall - (small_before + rank) - 1)] = r;
-        small_before += tot;
+    const TileFlags f = tree_tile_flags(c, g.mean, off, end, warp_tot);
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+    int before = tile_pre[blockIdx.x] + f.before;
+#pragma unroll
+    for (int k = 0; k < kTileRounds; ++k) {
+        const int r = f.first + 32 * k;
+        const bool small = f.small[k] >> (threadIdx.x & 31) & 1u;
+        if (small && r >= g.nsmall)
+            map[g.ipart + g.nsmall + (g.nsmall - (before + __popc(f.small[k] & lt)) - 1)] = r;
+        before += __popc(f.small[k]);
     }
 }
 
@@ -257,18 +438,36 @@ tree_tile_swap_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ 
     const int end = min(min(g.length, off + kTreeTile), g.nsmall);
     if (end <= off) return;  // the whole tile lies in the right part (block-uniform)
     const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
-    int small_before = tile_pre[blockIdx.x];
-    for (int r0 = off; r0 < end; r0 += blockDim.x) {
-        const int r = r0 + threadIdx.x;
-        const bool in = r < end;
-        const bool big = in && c[r] > g.mean;
-        int tot;
-        const int rank = tree_block_prefix(in && !big ? 1 : 0, warp_tot, &tot);
-        if (big) {
-            const int q = r - (small_before + rank);
-            tree_swap(P, g.ipart + r, g.ipart + map[g.ipart + g.nsmall + q]);
+    const TileFlags f = tree_tile_flags(c, g.mean, off, end, warp_tot);
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+    int before = tile_pre[blockIdx.x] + f.before;
+    int to[kTileRounds];  // the partner's slot, -1: stays
+#pragma unroll
+    for (int k = 0; k < kTileRounds; ++k) {
+        const int r = f.first + 32 * k;
+        const bool big = r < end && !(f.small[k] >> (threadIdx.x & 31) & 1u);
+        to[k] = big ? map[g.ipart + g.nsmall + (r - (before + __popc(f.small[k] & lt)))] : -1;
+        before += __popc(f.small[k]);
+    }
+    // four swaps' loads at a time, then their stores
+#pragma unroll
+    for (int k0 = 0; k0 < kTileRounds; k0 += 4) {
+        double a[4][3], b[4][3];
+        int ia[4], ib[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (to[k0 + k] < 0) continue;
+            const int i = g.ipart + f.first + 32 * (k0 + k), j = g.ipart + to[k0 + k];
+            a[k][0] = P.x[i]; a[k][1] = P.y[i]; a[k][2] = P.z[i]; ia[k] = P.id[i];
+            b[k][0] = P.x[j]; b[k][1] = P.y[j]; b[k][2] = P.z[j]; ib[k] = P.id[j];
         }
-        small_before += tot;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (to[k0 + k] < 0) continue;
+            const int i = g.ipart + f.first + 32 * (k0 + k), j = g.ipart + to[k0 + k];
+            P.x[i] = b[k][0]; P.y[i] = b[k][1]; P.z[i] = b[k][2]; P.id[i] = ib[k];
+            P.x[j] = a[k][0]; P.y[j] = a[k][1]; P.z[j] = a[k][2]; P.id[j] = ia[k];
+        }
     }
 }
 
@@ -287,45 +486,41 @@ struct SmallItem {
     char axis, side;
 };
 
+constexpr int kTreeSmallThreads = 512;
+// Nodes of one depth hold more than one particle each; they have two children.
+constexpr int kTreeLevelItems = kTreeSmall / 2;
+constexpr int kTreeLevelLeaves = kTreeSmall;
+
+// A leaf made at the current depth: its slots in the task (as SmallItem::span)
+// and its place, 2 x (index of the parent within the depth) + side.
+struct SmallLeaf {
+    int span, place;
+};
+
 // Dynamic shared memory of tree_small_kernel.
 constexpr size_t kTreeSmallSmem = (size_t)kTreeSmall * (3 * sizeof(double) + sizeof(int) + sizeof(short)) +
-                                  (size_t)kTreeMaxStack * sizeof(SmallItem);
-
-__device__ __forceinline__ int tree_new_leaf(TreeRec &R, int ip, int np) {
-    const int l = atomicAdd(&R.counters[1], 1);
-    if (l >= R.leaf_cap) {
-        atomicOr(&R.counters[2], TB_LEAF_CAP);
-        return -1;
-    }
-    R.lipart[l] = ip;
-    R.lnpart[l] = np;
-    return l;
-}
-
-__device__ __forceinline__ int tree_new_node(TreeRec &R, int depth) {
-    const int k = atomicAdd(&R.counters[0], 1);
-    if (k >= R.node_cap) {
-        atomicOr(&R.counters[2], TB_NODE_CAP);
-        return -1;
-    }
-    R.depth[k] = depth;
-    atomicMax(&R.counters[3], depth);
-    return k;
-}
+                                  2 * (size_t)kTreeLevelItems * sizeof(SmallItem) +
+                                  (size_t)kTreeLevelLeaves * sizeof(SmallLeaf);
 
 // One block builds a whole subtree of at most kTreeSmall particles in shared
-// memory, node after node from an explicit stack (left child first, as the
-// reference recursion), then writes the permuted particles back.
-__global__ void __launch_bounds__(kTreeThreads)
+// memory, depth after depth, one warp per node, then writes the permuted
+// particles back. Warps split their nodes with ballots and no block barrier,
+// and the build ids of a depth's nodes and leaves (names only: the pre-order
+// numbering is made afterwards) are taken with one atomic each. A block that
+// split one node after another waited for each one's serial sum, ten barriers
+// and three atomics on counters that all blocks share: 7.6 ms at 256^3.
+__global__ void __launch_bounds__(kTreeSmallThreads)
 tree_small_kernel(const TreeTask *__restrict__ tasks, TreeParts P, TreeRec R, int maxleaf) {
     extern __shared__ double tsm[];
     double *sx = tsm, *sy = sx + kTreeSmall, *sz = sy + kTreeSmall;
     int *sid = reinterpret_cast<int *>(sz + kTreeSmall);
-    short *smap = reinterpret_cast<short *>(sid + kTreeSmall);
-    SmallItem *stack = reinterpret_cast<SmallItem *>(smap + kTreeSmall);
-    __shared__ int warp_tot[kTreeThreads / 32];
-    __shared__ int s_top, s_node, s_kpairs;
-    __shared__ double s_mean;
+    SmallItem *items = reinterpret_cast<SmallItem *>(sid + kTreeSmall);  // this depth's, then the next one's
+    SmallLeaf *leaves = reinterpret_cast<SmallLeaf *>(items + 2 * kTreeLevelItems);
+    short *smap = reinterpret_cast<short *>(leaves + kTreeLevelLeaves);
+    __shared__ int s_count[2];  // items of each half
+    __shared__ int s_nleaf, s_node0, s_leaf0;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
     const TreeTask T = tasks[blockIdx.x];
     for (int i = threadIdx.x; i < T.length; i += blockDim.x) {
         sx[i] = P.x[T.ipart + i];
@@ -340,110 +535,110 @@ tree_small_kernel(const TreeTask *__restrict__ tasks, TreeParts P, TreeRec R, in
         it.depth = (short)T.depth;
         it.axis = (char)T.axis;
         it.side = (char)T.side;
-        stack[0] = it;
-        s_top = 1;
+        items[0] = it;
+        s_count[0] = 1;
+        s_count[1] = 0;
+        s_nleaf = 0;
+        s_node0 = atomicAdd(&R.counters[0], 1);
     }
     __syncthreads();
-    while (s_top > 0) {
-        const SmallItem it = stack[s_top - 1];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            s_top -= 1;
-            const int k = tree_new_node(R, it.depth);
-            s_node = k;
-            if (k >= 0 && it.parent >= 0) R.son[2 * it.parent + it.side] = 2 * k + 1;
+    int depth = T.depth;
+    for (int half = 0;; half ^= 1, ++depth) {
+        const int count = s_count[half], node0 = s_node0;
+        if (node0 + count > R.node_cap) {  // block-uniform
+            if (threadIdx.x == 0) atomicOr(&R.counters[2], TB_NODE_CAP);
+            break;
         }
-        __syncthreads();
-        const int node = s_node;
-        if (node < 0) break;  // node capacity exceeded (status set)
-        const int base = it.span & 0xffff, len = it.span >> 16, axis = it.axis;
-        double *c = axis == 0 ? sx : (axis == 1 ? sy : sz);
-        int nleft;
-        if (len < 2) {
-            nleft = 0;
-            if (threadIdx.x == 0) R.split[node] = 0.0;
-        } else if (len == 2) {
-            nleft = 1;
-            if (threadIdx.x == 0) {
-                R.split[node] = __dmul_rn(0.5, __dadd_rn(c[base], c[base + 1]));
-                if (c[base] > c[base + 1]) {
-                    double t;
-                    t = sx[base]; sx[base] = sx[base + 1]; sx[base + 1] = t;
-                    t = sy[base]; sy[base] = sy[base + 1]; sy[base + 1] = t;
-                    t = sz[base]; sz[base] = sz[base + 1]; sz[base + 1] = t;
-                    const int ti = sid[base]; sid[base] = sid[base + 1]; sid[base + 1] = ti;
+        for (int q = w; q < count; q += kTreeSmallThreads / 32) {
+            const SmallItem it = items[half * kTreeLevelItems + q];
+            const int node = node0 + q;
+            const int base = it.span & 0xffff, len = it.span >> 16, axis = it.axis;
+            double *c = sx + axis * kTreeSmall + base;
+            double split = 0.0;
+            int nleft = 0;
+            if (len == 2) {
+                nleft = 1;
+                split = __dmul_rn(0.5, __dadd_rn(c[0], c[1]));
+                const bool swap = c[0] > c[1];
+                __syncwarp();
+                if (lane == 0 && swap) {
+                    TreeParts Q{sx, sy, sz, sid};
+                    tree_swap(Q, base, base + 1);
                 }
-            }
-        } else {
-            if (threadIdx.x == 0) {
-                s_mean = tree_mean(c + base, len);
-                R.split[node] = s_mean;
-            }
-            __syncthreads();
-            const double mean = s_mean;
-            // nsmall: slots not above the mean
-            int nsmall = 0;
-            for (int r0 = 0; r0 < len; r0 += blockDim.x) {
-                const int r = r0 + threadIdx.x;
-                int tot;
-                tree_block_prefix((r < len && !(c[base + r] > mean)) ? 1 : 0, warp_tot, &tot);
-                nsmall += tot;
-            }
-            // positions of the swapped slots by rank; the pairs are the particles
-            // above the mean among the first nsmall slots: nsmall minus the
-            // slots not above it there (read at slot nsmall)
-            if (threadIdx.x == 0) s_kpairs = 0;
-            int small_before = 0;
-            for (int r0 = 0; r0 < len; r0 += blockDim.x) {
-                const int r = r0 + threadIdx.x;
-                const bool in = r < len;
-                const bool small = in && !(c[base + r] > mean);
-                int tot;
-                const int rank = tree_block_prefix(small ? 1 : 0, warp_tot, &tot);
-                if (in) {
-                    const int sb = small_before + rank;
-                    if (!small && r < nsmall) smap[r - sb] = (short)r;
-                    else if (small && r >= nsmall) smap[nsmall + (nsmall - sb - 1)] = (short)r;
-                    if (r == nsmall) s_kpairs = nsmall - sb;
+            } else if (len > 2) {
+                const double S = len <= 512 ? mean_chain(c, len, 0.0) : mean_warp(c, len, 0.0);
+                const double mean = __ddiv_rn(S, (double)len);
+                split = mean;
+                int nsmall = 0;  // slots not above the mean
+                for (int r0 = 0; r0 < len; r0 += 32)
+                    nsmall += __popc(__ballot_sync(0xffffffffu, r0 + lane < len && !(c[r0 + lane] > mean)));
+                // the swapped slots by rank: particles above the mean among the
+                // first nsmall slots from the left, the others' from the right
+                short *map = smap + base;
+                int before = 0, kpairs = 0;
+                for (int r0 = 0; r0 < len; r0 += 32) {
+                    const int r = r0 + lane;
+                    const bool in = r < len;
+                    const bool small = in && !(c[r] > mean);
+                    const unsigned m = __ballot_sync(0xffffffffu, small);
+                    const int sb = before + __popc(m & lt);
+                    if (in && !small && r < nsmall) map[r - sb] = (short)r;
+                    else if (small && r >= nsmall) map[nsmall + (nsmall - sb - 1)] = (short)r;
+                    const unsigned left = nsmall - r0 >= 32 ? 0xffffffffu : (nsmall > r0 ? (1u << (nsmall - r0)) - 1u : 0u);
+                    kpairs += __popc(left & ~m);  // nsmall <= len: these lanes hold particles
+                    before += __popc(m);
                 }
-                small_before += tot;
+                __syncwarp();
+                TreeParts Q{sx, sy, sz, sid};
+                for (int k = lane; k < kpairs; k += 32) tree_swap(Q, base + map[k], base + map[nsmall + k]);
+                nleft = (len - nsmall) == 0 ? len - 1 : nsmall;
             }
-            __syncthreads();
-            const int kpairs = s_kpairs;
-            __syncthreads();
-            for (int q = threadIdx.x; q < kpairs; q += blockDim.x) {
-                const int a = base + smap[q], b = base + smap[nsmall + q];
-                double t;
-                t = sx[a]; sx[a] = sx[b]; sx[b] = t;
-                t = sy[a]; sy[a] = sy[b]; sy[b] = t;
-                t = sz[a]; sz[a] = sz[b]; sz[b] = t;
-                const int ti = sid[a]; sid[a] = sid[b]; sid[b] = ti;
+            if (lane == 0) {
+                R.split[node] = split;
+                R.depth[node] = it.depth;
+                if (it.parent >= 0) R.son[2 * it.parent + it.side] = 2 * node + 1;
             }
-            nleft = (len - nsmall) == 0 ? len - 1 : nsmall;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const int np[2] = {nleft, len - nleft};
-            const int ip[2] = {base, base + nleft};
-            const char naxis = (char)((axis + 1) % 3);
-            // the right child is pushed first so the left one is split next
-            for (int n = 1; n >= 0; --n) {
-                if (np[n] <= maxleaf) {
-                    const int l = tree_new_leaf(R, T.ipart + ip[n], np[n]);
-                    if (l >= 0) R.son[2 * node + n] = 2 * l;
+            if (lane < 2) {  // this lane's child
+                const int np = lane ? len - nleft : nleft, ip = lane ? base + nleft : base;
+                if (np <= maxleaf) {
+                    SmallLeaf lf;
+                    lf.span = ip | (np << 16);
+                    lf.place = 2 * q + lane;
+                    leaves[atomicAdd(&s_nleaf, 1)] = lf;
                 } else {
                     SmallItem ch;
-                    ch.span = ip[n] | (np[n] << 16);
+                    ch.span = ip | (np << 16);
                     ch.parent = node;
                     ch.depth = (short)(it.depth + 1);
-                    ch.axis = naxis;
-                    ch.side = (char)n;
-                    stack[s_top++] = ch;
+                    ch.axis = (char)((axis + 1) % 3);
+                    ch.side = (char)lane;
+                    items[(half ^ 1) * kTreeLevelItems + atomicAdd(&s_count[half ^ 1], 1)] = ch;
                 }
             }
         }
+        __syncthreads();  // this depth is split; its leaves and the next depth's items are written
+        const int nleaf = s_nleaf, more = s_count[half ^ 1];
+        if (threadIdx.x == 0) {
+            if (nleaf) s_leaf0 = atomicAdd(&R.counters[1], nleaf);
+            if (more) s_node0 = atomicAdd(&R.counters[0], more);
+        }
         __syncthreads();
+        if (threadIdx.x == 0) s_nleaf = s_count[half] = 0;
+        if (nleaf && s_leaf0 + nleaf > R.leaf_cap) {  // block-uniform
+            if (threadIdx.x == 0) atomicOr(&R.counters[2], TB_LEAF_CAP);
+            break;
+        }
+        for (int i = threadIdx.x; i < nleaf; i += blockDim.x) {
+            const SmallLeaf lf = leaves[i];
+            const int l = s_leaf0 + i;
+            R.lipart[l] = T.ipart + (lf.span & 0xffff);
+            R.lnpart[l] = lf.span >> 16;
+            R.son[2 * (node0 + (lf.place >> 1)) + (lf.place & 1)] = 2 * l;
+        }
+        if (!more) break;
+        __syncthreads();  // the leaves are read, the counts are reset
     }
+    if (threadIdx.x == 0) atomicMax(&R.counters[3], depth);
     __syncthreads();
     for (int i = threadIdx.x; i < T.length; i += blockDim.x) {
         P.x[T.ipart + i] = sx[i];
