@@ -200,16 +200,18 @@ typedef struct p2p_walk_tree {
 } p2p_walk_tree;
 /* Replaces the caller's walk_task_p2p (src/fmm.c:656-792, acceptance
  * src/fmm.c:409-479, called from fmm_task src/fmm.c:1221-1300) plus the
- * list submit: the P2P lists are walked on the GPU, one warp per sink leaf,
- * straight into CSR rows equal entry for entry to those p2p_pass_submit
+ * list submit: the P2P lists are walked on the GPU, depth by depth of the sink
+ * side, straight into CSR rows equal entry for entry to those p2p_pass_submit
  * builds from the serial walk's list, then the pair kernel runs on them.
  * Within an open pass (its leaves are the tree's leaves). Waits for the row
- * count (one device-to-host read); *ntask (nullable) = list entries. The
- * leaves are walked once: rows of up to 2048 entries are kept in a slab the
- * session holds between passes (2048 ids per leaf, halved while it would
- * exceed 8 GB) and gathered, longer rows walked a second time.
- * P2P_ERR_ARG for a child code outside the tree, P2P_ERR_CAPACITY when a
- * sink's pending pairs exceed the walk's fixed stack. */
+ * count (device-to-host reads); *ntask (nullable) = list entries. The session
+ * keeps the walk's memory between passes: about 100 bytes a node and 150 a leaf,
+ * the lists of one depth (about 1 KB a node at first) and the rows (4 bytes an entry and
+ * some; pools that turn out too small are doubled and the walk repeated). Rows of
+ * more than 8 GB are counted first and written in place by a second walk.
+ * P2P_ERR_ARG for a child code outside the tree or leaves that are not in
+ * pre-order, P2P_ERR_CAPACITY when a box's pending boxes exceed the walk's fixed
+ * stack. */
 int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *tree, double cutoff, double open_angle,
                          int64_t *ntask);
 /* ---- Device kd-tree (no counterpart in the reference's GPU code) --------
@@ -299,8 +301,8 @@ int p2p_pm_download(p2p_pm *pm, double *mass_mesh, double *potential);
  * nothing. The reference's m2l tests abs(r2) <= 1e-15 with the integer abs()
  * (src/operator.c:340-344), which skips every task with r2 < 1 in its length
  * unit: min_r2 = 1 reproduces it, 1e-15 what the test evidently means.
- * Queued on the session's stream; the M2L walk reads one count per tree
- * level back to the host, so the call returns when the pass is done. */
+ * Queued on the session's stream; the M2L walk reads its counts back to the
+ * host, so the call returns when the pass is done. */
 typedef struct p2p_fmm p2p_fmm;
 int p2p_fmm_create(p2p_session *s, p2p_fmm **out);
 int p2p_fmm_destroy(p2p_fmm *f);
@@ -309,7 +311,7 @@ int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const double *d_p
                 double min_r2, double *d_acc);
 /* Counts and device times (ms: upward, walk, M2L, downward, total; nullable
  * outputs) of the last p2p_fmm_far: M2L tasks, tasks applied (r2 >= min_r2),
- * walk levels. */
+ * depths of sink boxes walked. */
 int p2p_fmm_stats(p2p_fmm *f, int64_t *n_m2l, int64_t *n_applied, int *levels, float ms[5]);
 /* Host copies (nullable) of the leaves' multipoles after P2M and their locals
  * after L2L, 20 doubles per leaf in the reference's coefficient order. */

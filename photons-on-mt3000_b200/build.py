@@ -25,7 +25,8 @@ CUDA_SOURCES = ["p2p_core.cu", "p2p_noalloc.cu", "p2p_pair_sink_lanes.cu", "p2p_
 CUDA_HEADERS = ["p2p_kernels.cuh", "p2p_pass_kernels.cuh", "p2p_pair_kernels.cuh",
                 "p2p_device_common.cuh", "p2p_launch.h", "p2p_internal.h", "p2p_fit.h",
                 "p2p_pair_x2_impl.h", "p2p_csr.h", "p2p_args.h", "p2p_host_shared.h", "p2p_walk_kernels.cuh",
-                "p2p_pair_sreg.cuh", "p2p_tree_kernels.cuh", "p2p_fit64.h", "p2p_pair_fp64.cuh"]
+                "p2p_pair_sreg.cuh", "p2p_tree_kernels.cuh", "p2p_fit64.h", "p2p_pair_fp64.cuh",
+                "p2p_walk_test.h"]
 HOST_SOURCES = ["p2p_lists.cpp"]
 
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]

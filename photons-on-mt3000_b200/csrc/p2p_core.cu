@@ -92,7 +92,10 @@ struct p2p_session {
         row_src, tile_sums, acc, status, queue, pairs, skipped, evaluated, probe;
     DevBuf keys_a, keys_b, vals_b, hist, hoffs, hsums;  // radix sort of the list
     std::vector<DevBuf> scratch;  // grow-only temporaries of p2p_dtree_build, by request order
-    DevBuf walk_slab;             // the walk's first pass keeps short rows here (p2p_pass_submit_walk)
+    // device walk (p2p_pass_submit_walk): box records, active prefix, boxes of
+    // two depths, their undecided lists, the rows, counters
+    DevBuf walk_box, walk_active, walk_items, walk_lists[2], walk_rows, walk_ctrl;
+    int64_t walk_list_cap = 0, walk_row_cap = 0;  // chunks of the pools
     // pass state
     bool in_pass = false;
     int npart = 0, nleaf = 0;
@@ -139,11 +142,9 @@ int ensure(p2p_session *s, DevBuf &b, size_t bytes) {
 
 bool is_fp32_form(int form) { return form != P2P_FORM_PLAIN_FP64; }
 
-// The device walk's slab of short rows: up to kWalkSlabMax ids per leaf (a
-// power of two, halved down to kWalkSlabMin while it exceeds kWalkSlabBytes).
-constexpr int kWalkSlabMax = 2048;
-constexpr int kWalkSlabMin = 64;
-constexpr size_t kWalkSlabBytes = (size_t)8 << 30;
+// The device walk keeps its rows in a pool of at most this size; longer ones
+// take a second walk.
+constexpr size_t kWalkPoolBytes = (size_t)8 << 30;
 
 // Host list submits longer than 2 * kPipePieceMin entries are uploaded and
 // computed in about kPipePieces pieces of at least kPipePieceMin entries.
@@ -537,7 +538,8 @@ P2P_API int p2p_session_destroy(p2p_session *s) {
                       &s->meta, &s->pos4, &s->counts, &s->fill, &s->row_off, &s->row_src,
                       &s->tile_sums, &s->acc, &s->status, &s->queue, &s->pairs, &s->skipped, &s->evaluated, &s->probe,
                       &s->keys_a, &s->keys_b, &s->vals_b, &s->hist, &s->hoffs, &s->hsums,
-                      &s->task_t2, &s->task_s2, &s->walk_slab};
+                      &s->task_t2, &s->task_s2, &s->walk_box, &s->walk_active, &s->walk_items, &s->walk_lists[0],
+                      &s->walk_lists[1], &s->walk_rows, &s->walk_ctrl};
     if (s->copy_stream) cudaStreamSynchronize(s->copy_stream);
     for (DevBuf *b : bufs)
         if (b->p) cudaFree(b->p);
@@ -783,10 +785,10 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
         return fail(P2P_ERR_ARG, "null tree array");
     if (!(cutoff >= 0.0) || !(open_angle >= 0.0)) return fail(P2P_ERR_ARG, "bad cutoff or open angle");
     if (ntask) *ntask = 0;
-    const int nleaf = s->nleaf;
-    if (nleaf == 0 || t->nnode == 0) return P2P_OK;
+    const int nleaf = s->nleaf, nnode = t->nnode;
+    if (nleaf == 0 || nnode == 0) return P2P_OK;
     WalkArgs w;
-    w.nnode = t->nnode;
+    w.nnode = nnode;
     w.nleaf = nleaf;
     w.son = t->son;
     w.node_first = t->node_first;
@@ -797,67 +799,119 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     w.leaf_width = t->leaf_width;
     w.cutoff = cutoff;
     w.open_angle = open_angle;
-    const int threads = kWalkWarps * 32;
-    const int grid = grid_for(nleaf, kWalkWarps, s->sm_count * 32);
-    int *status = (int *)s->status.p;
-    // The first pass keeps each row's first slab_cap entries in a slab of
-    // slab_cap ids per leaf (at most kWalkSlabBytes), from which the rows are
-    // gathered; only rows longer than that are walked a second time.
-    int slab_cap = kWalkSlabMax;
-    while (slab_cap > kWalkSlabMin && (size_t)nleaf * slab_cap * sizeof(int) > kWalkSlabBytes) slab_cap >>= 1;
-    if ((size_t)nleaf * slab_cap * sizeof(int) > kWalkSlabBytes) slab_cap = 0;  // two walks
-    int *slab = nullptr;
-    if (slab_cap > 0) {
-        P2P_TRY(ensure(s, s->walk_slab, sizeof(int) * (size_t)nleaf * slab_cap));
-        slab = (int *)s->walk_slab.p;
-    }
-    // pass 1: row lengths (and the slab), then the row offsets
-    walk_rows_kernel<false><<<grid, threads, 0, s->stream>>>(w, (int *)s->counts.p, nullptr, nullptr, nullptr,
-                                                               nullptr, 0.0, 0.f, nullptr, nullptr, status, slab,
-                                                               slab_cap);
+    const size_t nbox = 2 * ((size_t)std::max(nleaf, nnode) + 1);
+    P2P_TRY(ensure(s, s->walk_box, (sizeof(WalkBox) + sizeof(WalkBox32)) * nbox));
+    P2P_TRY(ensure(s, s->walk_active, sizeof(int64_t) * ((size_t)nleaf + 1)));
+    P2P_TRY(ensure(s, s->walk_items, sizeof(WalkItem) * 2 * (size_t)nleaf));
+    P2P_TRY(ensure(s, s->walk_ctrl, sizeof(WalkCtrl)));
+    // Pools of chunks: the undecided lists of one depth (two pools in turn)
+    // and the rows. Sizes are first guesses; a walk that runs out of one is
+    // repeated with twice the size, which the session keeps. Rows beyond
+    // kWalkPoolBytes are counted first and then written to their places by a
+    // second walk.
+    const int64_t slack = walk_pool_slack(s->sm_count);
+    s->walk_list_cap = std::max(s->walk_list_cap, 2 * (int64_t)nnode + slack);
+    s->walk_row_cap = std::max(s->walk_row_cap, 10 * (int64_t)nleaf + slack);
     const int ntiles = (int)((nleaf + (int64_t)kScanTile - 1) / kScanTile);
-    int64_t *row_off = (int64_t *)s->row_off.p;
-    scan_tiles_kernel<<<ntiles, kScanThreads, 0, s->stream>>>((const int *)s->counts.p, nleaf, row_off,
-                                                               (int64_t *)s->tile_sums.p);
-    scan_sums_kernel<<<1, kScanThreads, 0, s->stream>>>((int64_t *)s->tile_sums.p, ntiles, row_off + nleaf);
-    scan_add_kernel<<<grid_for(nleaf, 256, 1 << 30), 256, 0, s->stream>>>(row_off, nleaf, (int64_t *)s->tile_sums.p);
-    CUDA_TRY(cudaGetLastError());
-    launch_count(4);
+    int64_t *row_off = (int64_t *)s->row_off.p, *tile_sums = (int64_t *)s->tile_sums.p;
+    int *counts = (int *)s->counts.p, *heads = (int *)s->fill.p;
+    auto scan = [&](const int *in, int64_t *out) {
+        scan_tiles_kernel<<<ntiles, kScanThreads, 0, s->stream>>>(in, nleaf, out, tile_sums);
+        scan_sums_kernel<<<1, kScanThreads, 0, s->stream>>>(tile_sums, ntiles, out + nleaf);
+        scan_add_kernel<<<grid_for(nleaf, 256, 1 << 30), 256, 0, s->stream>>>(out, nleaf, tile_sums);
+        launch_count(3);
+    };
+    WalkRun g;
+    std::memset(&g, 0, sizeof(g));
+    g.nnode = nnode;
+    g.nleaf = nleaf;
+    g.node_first = t->node_first;
+    g.cutoff = cutoff;
+    g.open_angle = open_angle;
+    g.cut2 = (float)(cutoff * cutoff);
+    g.th2 = (float)(open_angle * open_angle);
+    g.out_head = heads;
+    g.out_len = counts;
+    g.row_off = row_off;
     int64_t total = 0;
-    int st = 0;
-    CUDA_TRY(cudaMemcpyAsync(&total, row_off + nleaf, sizeof(total), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(&st, status, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
-    if (st & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
-    if (st & ST_WALK_STACK) return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
+    bool pooled = false;
+    // one walk (rows into the pool, counted, or written): the row offsets and
+    // the total, or an error
+    auto walk = [&](bool fill) -> int {
+        for (;;) {
+            pooled = !fill && walk_pool_bytes(s->walk_row_cap, kWalkChunk) <= kWalkPoolBytes;
+            P2P_TRY(ensure(s, s->walk_lists[0], walk_pool_bytes(s->walk_list_cap, kWalkChunk)));
+            P2P_TRY(ensure(s, s->walk_lists[1], walk_pool_bytes(s->walk_list_cap, kWalkChunk)));
+            if (pooled) P2P_TRY(ensure(s, s->walk_rows, walk_pool_bytes(s->walk_row_cap, kWalkChunk)));
+            g.box = (const WalkBox *)s->walk_box.p;
+            g.box32 = (const WalkBox32 *)(g.box + nbox);
+            g.active = (const int64_t *)s->walk_active.p;
+            g.items[0] = (WalkItem *)s->walk_items.p;
+            g.items[1] = g.items[0] + nleaf;
+            for (int k = 0; k < 2; ++k) g.lists[k] = walk_pool(s->walk_lists[k].p, s->walk_list_cap, kWalkChunk);
+            if (pooled) g.out = walk_pool(s->walk_rows.p, s->walk_row_cap, kWalkChunk);
+            g.row_src = (int *)s->row_src.p;
+            g.ctrl = (WalkCtrl *)s->walk_ctrl.p;
+            CUDA_TRY(cudaMemsetAsync(g.ctrl, 0, sizeof(WalkCtrl), s->stream));
+            if (!fill) CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nleaf, s->stream));
+            walk_pack_kernel<false><<<grid_for((int64_t)nnode + nleaf, 256, s->sm_count * 16), 256, 0, s->stream>>>(
+                w, (WalkBox *)s->walk_box.p, (WalkBox32 *)((WalkBox *)s->walk_box.p + nbox), heads, g.items[0], g.lists[0].ids, g.ctrl);
+            launch_count(1);
+            scan(heads, (int64_t *)s->walk_active.p);  // (the flags, before the heads take their place)
+            int st = 0, left = 0;
+            for (int lv = 0, n = walk_first_depths(nleaf);; n = 4) {
+                n = std::min(n, kWalkLevels - lv);
+                if (n <= 0) return fail(P2P_ERR_CAPACITY, "walk: more than %d depths", kWalkLevels);
+                CUDA_TRY(fill ? walk_depths<WALK_FILL>(s->stream, g, s->sm_count, lv, n)
+                         : pooled ? walk_depths<WALK_ROWS>(s->stream, g, s->sm_count, lv, n)
+                                  : walk_depths<WALK_COUNT>(s->stream, g, s->sm_count, lv, n));
+                launch_count(n);
+                lv += n;
+                if (!fill) scan(counts, row_off);
+                CUDA_TRY(cudaGetLastError());
+                CUDA_TRY(cudaMemcpyAsync(&total, row_off + nleaf, sizeof(total), cudaMemcpyDeviceToHost, s->stream));
+                CUDA_TRY(cudaMemcpyAsync(&left, &g.ctrl->items[lv], sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+                CUDA_TRY(cudaMemcpyAsync(&st, &g.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+                CUDA_TRY(cudaStreamSynchronize(s->stream));
+                if (st || left == 0) break;
+            }
+            const int bad = st & (ST_WALK_TREE | ST_WALK_STACK | ST_WALK_ROW);
+            if (bad) {  // closing the pass reports it too
+                int main_status = 0;
+                CUDA_TRY(cudaMemcpy(&main_status, s->status.p, sizeof(int), cudaMemcpyDeviceToHost));
+                main_status |= bad;
+                CUDA_TRY(cudaMemcpy(s->status.p, &main_status, sizeof(int), cudaMemcpyHostToDevice));
+                if (bad & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
+                return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
+            }
+            if (!st) return P2P_OK;
+            if (st & ST_WALK_LISTS) s->walk_list_cap *= 2;
+            if (st & ST_WALK_OUT) s->walk_row_cap *= 2;
+            if (std::max(s->walk_list_cap, s->walk_row_cap) > INT32_MAX)
+                return fail(P2P_ERR_CAPACITY, "walk: more lists than a pool can hold");
+        }
+    };
+    P2P_TRY(walk(false));
     if (ntask) *ntask = total;
     if (total == 0) return P2P_OK;
-    // pass 2: the rows' source ids, pair counts (short rows from the slab,
-    // long rows walked again); then the pair kernel
     P2P_TRY(ensure(s, s->row_src, sizeof(int) * (size_t)total));
-    const bool skip = skips_outside(s);
+    const bool skip = skips_outside(s), chains = pooled;
+    if (!chains) P2P_TRY(walk(true));
     const double cscale = 0.5 / s->params.split_radius;
     const float uout = (float)(s->fit.umax * (1.0 + kCutBand) * (1.0 + kOutsideMargin));
     unsigned long long *d_skipped = skip ? (unsigned long long *)s->skipped.p : nullptr;
-    if (slab)
-        walk_gather_kernel<<<grid_for(nleaf, 8, s->sm_count * 16), 256, 0, s->stream>>>(
-            (const int *)s->counts.p, row_off, nleaf, slab, slab_cap, (int *)s->row_src.p, s->d_np,
-            (const LeafMeta *)s->meta.p, cscale, uout, (unsigned long long *)s->pairs.p, d_skipped, status);
-    walk_rows_kernel<true><<<grid, threads, 0, s->stream>>>(
-        w, (int *)s->counts.p, row_off, (int *)s->row_src.p, s->d_np, (const LeafMeta *)s->meta.p, cscale, uout,
-        (unsigned long long *)s->pairs.p, d_skipped, status, nullptr, slab_cap);
-    // each row ascending by source leaf id: the serial walk's order for that sink
-    int *rs = (int *)s->row_src.p;
-    csr_sort_rows_warp_kernel<1, kSortWarpMax><<<grid_for(nleaf, 4, s->sm_count * 8), 128, 0, s->stream>>>(
-        row_off, nleaf, rs);
-    csr_sort_rows_warp_kernel<kSortWarpMax, kSortWarpMax2><<<grid_for(nleaf, 4, s->sm_count * 8), 128, 0, s->stream>>>(
-        row_off, nleaf, rs);
-    csr_sort_rows_block_kernel<<<grid_for(nleaf, 1, s->sm_count * 4), kSortBlockThreads, 0, s->stream>>>(
-        row_off, nleaf, rs);
-    csr_sort_rows_global_kernel<<<grid_for(nleaf, 1, s->sm_count), kSortBlockThreads, 0, s->stream>>>(
-        row_off, nleaf, rs);
+    // the rows into their places, and their pair counts
+    const int gather = grid_for(nleaf, 8, s->sm_count * 16);
+    if (chains)
+        walk_gather_kernel<true><<<gather, 256, 0, s->stream>>>(counts, heads, row_off, nleaf, g.out, (int *)s->row_src.p,
+                                                               s->d_np, (const LeafMeta *)s->meta.p, cscale, uout,
+                                                               (unsigned long long *)s->pairs.p, d_skipped);
+    else
+        walk_gather_kernel<false><<<gather, 256, 0, s->stream>>>(counts, heads, row_off, nleaf, g.out, (int *)s->row_src.p,
+                                                                s->d_np, (const LeafMeta *)s->meta.p, cscale, uout,
+                                                                (unsigned long long *)s->pairs.p, d_skipped);
     CUDA_TRY(cudaGetLastError());
-    launch_count(slab ? 6 : 5);
+    launch_count(1);
     return enqueue_pairs(s, true);
 }
 

@@ -9,11 +9,10 @@
 //              node's children to finish
 //   M2L walk   the reference's dual-tree recursion from (root, root)
 //              (walk_task_m2l, src/fmm.c:812-957, with the acceptance test
-//              of :409-479) expanded breadth first on the GPU, a level of
-//              pending pairs per launch: a pair is accepted as an M2L task,
-//              opened into its child pairs, or dropped
-//   M2L        each sink (leaf or node), one warp, sums over its tasks in
-//              increasing source order the source multipole's contribution
+//              of :409-479) depth by depth of the sink side on the GPU
+//              (walk_level_kernel), each sink's accepted sources in a list
+//   M2L        each sink (leaf or node), half a warp, sums over its list, in the
+//              order the walk leaves it, the source multipole's contribution
 //              to its local expansion with the erfc-truncated kernel's derivatives
 //              (m2l with LONGSHORT, src/operator.c:331-475)
 //   l2l + l2p  each leaf takes its ancestors' locals down its path from the
@@ -38,23 +37,17 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "photons_p2p.h"
 #include "p2p_host_shared.h"
 #include "p2p_internal.h"
 
-// This file's own instances of the scan and walk helpers (private namespace,
-// so their non-template kernels do not collide with the session's).
-namespace p2p_fmm_kernels {
-using namespace ::p2p;
-#include "p2p_pass_kernels.cuh"
 #include "p2p_walk_kernels.cuh"
-}  // namespace p2p_fmm_kernels
 
 #define P2P_API extern "C" __attribute__((visibility("default")))
 
 using namespace p2p;
-using namespace p2p_fmm_kernels::p2p;
 
 namespace {
 
@@ -242,185 +235,38 @@ __global__ void fmm_upward_kernel(FmmArgs f) {
     }
 }
 
-// Whether an opened pair's child can lead to a task: two leaves (a P2P pair)
-// and a pair beyond the cutoff (acceptance -1) end the recursion with none,
-// so they are not written to the next level. Codes outside the tree are
-// kept, for the next level to report.
-__device__ __forceinline__ bool walk_child_live(const WalkArgs &w, int A, int B) {
-    if (A < 0 || B < 0) return false;
-    if (!walk_valid(w, A) || !walk_valid(w, B)) return true;
-    if (A == B) return (A & 1) != 0;
-    if (!(A & 1) && !(B & 1)) return false;
-    return walk_acceptance(walk_width(w, A), walk_width(w, B), walk_center(w, A), walk_center(w, B), w.cutoff,
-                           w.open_angle) != -1;
-}
+// M2L: half a warp per sink (a sink has about 10 tasks at open angle 0.4),
+// lane j takes tasks j, j + 16, ... of its list, in the order the walk left
+// them (pre-order of the sources within a depth of the sink's path), and the
+// lanes' partial locals are summed by a fixed shuffle tree: the same sum on
+// every run. The walk keeps a sink's tasks together, so nothing is sorted.
+constexpr int kM2LThreads = 128;
 
-// One level of the M2L walk: each pending pair is accepted (a task), opened
-// into its child pairs, or dropped, as walk_task_m2l decides; children that
-// cannot lead to a task are not kept (walk_child_live). Output slots come
-// from warp-aggregated atomics; a level whose outputs exceed the buffers
-// only counts them (the host grows the buffers and repeats it).
-__global__ void fmm_walk_kernel(WalkArgs w, const int2 *__restrict__ in, int nin, int2 *__restrict__ out,
-                                long long out_cap, unsigned long long *nout, int2 *__restrict__ tasks,
-                                long long task_cap, unsigned long long *ntask, int *status) {
-    const int lane = threadIdx.x & 31;
-    const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < nin; base += stride) {
-        const int i = base + lane;
-        int2 kids[4];
-        int nk = 0, nt = 0;
-        int2 task = make_int2(0, 0);
-        if (i < nin) {
-            const int A = in[i].x, B = in[i].y;
-            const bool okA = A >= 0 && walk_valid(w, A), okB = B >= 0 && walk_valid(w, B);
-            if ((A >= 0 && !okA) || (B >= 0 && !okB)) atomicOr(status, ST_WALK_TREE);
-            if (okA && okB) {
-                if (A == B) {
-                    if (A & 1) {
-                        const int s0 = w.son[2 * (A >> 1)], s1 = w.son[2 * (A >> 1) + 1];
-                        kids[0] = make_int2(s0, s0);
-                        kids[1] = make_int2(s0, s1);
-                        kids[2] = make_int2(s1, s0);
-                        kids[3] = make_int2(s1, s1);
-                        nk = 4;
-                    }
-                } else if ((A & 1) || (B & 1)) {
-                    const double *wa = walk_width(w, A), *wb = walk_width(w, B);
-                    const int flag = walk_acceptance(wa, wb, walk_center(w, A), walk_center(w, B), w.cutoff,
-                                                     w.open_angle);
-                    if (flag == 1) {
-                        task = make_int2(A, B);
-                        nt = 1;
-                    } else if (flag == 0) {
-                        bool openA;
-                        if (!(A & 1))
-                            openA = false;
-                        else if (!(B & 1))
-                            openA = true;
-                        else  // both nodes: open the one with the larger summed width
-                            openA = __dadd_rn(__dadd_rn(wa[0], wa[1]), wa[2]) >
-                                    __dadd_rn(__dadd_rn(wb[0], wb[1]), wb[2]);
-                        if (openA) {
-                            kids[0] = make_int2(w.son[2 * (A >> 1)], B);
-                            kids[1] = make_int2(w.son[2 * (A >> 1) + 1], B);
-                        } else {
-                            kids[0] = make_int2(A, w.son[2 * (B >> 1)]);
-                            kids[1] = make_int2(A, w.son[2 * (B >> 1) + 1]);
-                        }
-                        nk = 2;
-                    }
-                }
-            }
-        }
-        {  // keep the live children only
-            int m = 0;
-            for (int c = 0; c < nk; ++c)
-                if (walk_child_live(w, kids[c].x, kids[c].y)) kids[m++] = kids[c];
-            nk = m;
-        }
-        // warp-aggregated output slots
-        int kin = nk, tin = nt;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int a = __shfl_up_sync(kFull, kin, off), b = __shfl_up_sync(kFull, tin, off);
-            if (lane >= off) {
-                kin += a;
-                tin += b;
-            }
-        }
-        unsigned long long kbase = 0, tbase = 0;
-        if (lane == 31) {
-            kbase = kin ? atomicAdd(nout, (unsigned long long)kin) : 0ull;
-            tbase = tin ? atomicAdd(ntask, (unsigned long long)tin) : 0ull;
-        }
-        kbase = __shfl_sync(kFull, kbase, 31);
-        tbase = __shfl_sync(kFull, tbase, 31);
-        const long long ko = (long long)kbase + kin - nk, to = (long long)tbase + tin - nt;
-        for (int k = 0; k < nk; ++k)
-            if (ko + k < out_cap) out[ko + k] = kids[k];
-        if (nt && to < task_cap) tasks[to] = task;
-    }
-}
-
-__global__ void fmm_task_count_kernel(WalkArgs w, const int2 *__restrict__ tasks, long long nt, int *count) {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += (long long)gridDim.x * blockDim.x)
-        atomicAdd(&count[sink_index(w, tasks[t].x)], 1);
-}
-
-__global__ void fmm_task_fill_kernel(WalkArgs w, const int2 *__restrict__ tasks, long long nt,
-                                     const int64_t *__restrict__ off, int *fill, int *seg) {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += (long long)gridDim.x * blockDim.x) {
-        const int s = sink_index(w, tasks[t].x);
-        seg[off[s] + atomicAdd(&fill[s], 1)] = tasks[t].y;
-    }
-}
-
-// M2L: one warp per sink. The sink's source codes are put in increasing
-// order (a bitonic sort in shared memory up to kM2LSort codes; above that a
-// rank sort from seg into seg2), lane j takes the sorted tasks j, j + 32, ...
-// and the lanes' partial locals are summed by a fixed shuffle tree: the same
-// order on every run, whatever order the walk emitted the tasks in.
-constexpr int kM2LWarps = 4;
-constexpr int kM2LSort = 2048;
-
-__global__ void __launch_bounds__(32 * kM2LWarps)
-fmm_m2l_kernel(FmmArgs f, const int64_t *__restrict__ off, const int *__restrict__ seg, int *__restrict__ seg2,
+__global__ void __launch_bounds__(kM2LThreads)
+fmm_m2l_kernel(FmmArgs f, const int *__restrict__ head, const int *__restrict__ len, const WalkPool pool,
                unsigned long long *applied) {
-    __shared__ int sbuf[kM2LWarps][kM2LSort];
     const WalkArgs &w = f.w;
-    const int lane = threadIdx.x & 31;
-    int *buf = sbuf[threadIdx.x >> 5];
+    constexpr int H = kWalkTaskChunk;  // lanes per sink, tasks per chunk
+    static_assert(H == 16, "a chunk of tasks is one per lane of a half warp");
+    const int lane = threadIdx.x & (H - 1);
     const int nsink = w.nleaf + w.nnode;
-    const int nwarp = (gridDim.x * blockDim.x) >> 5;
-    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nsink; s += nwarp) {
-        const int64_t a = off[s], e = off[s + 1];
-        if (a < 0 || e < a || e > off[nsink]) {  // offsets out of order: record it, skip the sink
-            if (lane == 0) atomicOr(f.status, ST_WALK_ROW);
-            continue;
-        }
-        const int k = (int)(e - a);
-        const int *src = buf;
-        if (k <= kM2LSort) {
-            int p = 1;
-            while (p < k) p <<= 1;
-            for (int i = lane; i < p; i += 32) buf[i] = i < k ? seg[a + i] : INT_MAX;
-            __syncwarp();
-            for (int size = 2; size <= p; size <<= 1) {
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (int i = lane; i < p; i += 32) {
-                        const int j = i ^ stride;
-                        if (j > i) {
-                            const int x = buf[i], y = buf[j];
-                            if ((x > y) == ((i & size) == 0)) {
-                                buf[i] = y;
-                                buf[j] = x;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-        } else {
-            for (int i = lane; i < k; i += 32) {
-                const int v = seg[a + i];
-                int r = 0;
-                for (int j = 0; j < k; ++j) {
-                    const int x = seg[a + j];
-                    r += (x < v) || (x == v && j < i);
-                }
-                seg2[a + r] = v;
-            }
-            __syncwarp();
-            src = seg2 + a;
-        }
+    const int nhalf = gridDim.x * (blockDim.x / H);
+    unsigned used = 0;
+    // whole warps stay in the loop (the shuffles below)
+    for (int s0 = (blockIdx.x * blockDim.x + threadIdx.x) / H; (s0 & ~1) < nsink; s0 += nhalf) {
+        const int s = min(s0, nsink - 1);
+        const int k = s0 < nsink ? len[s] : 0;
         double L[kNC];
 #pragma unroll
         for (int c = 0; c < kNC; ++c) L[c] = 0.0;
         const int code = s < w.nleaf ? 2 * s : 2 * (s - w.nleaf) + 1;
         const double *cs = box_center(w, code);
-        unsigned used = 0;
-        for (int t = lane; t < k; t += 32) {
-            const int sc = src[t];
+        int chunk = k ? head[s] : 0;
+        for (int b = 0; b < k; b += H) {
+            const int t = chunk;
+            if (b + H < k) chunk = pool.next[t];
+            if (b + lane >= k) continue;
+            const int sc = pool.ids[(size_t)t * H + lane];
             const double *cb = box_center(w, sc);
             const double x = cs[0] - cb[0], y = cs[1] - cb[1], z = cs[2] - cb[2];
             const double r2 = x * x + y * y + z * z;
@@ -440,19 +286,18 @@ fmm_m2l_kernel(FmmArgs f, const int64_t *__restrict__ off, const int *__restrict
                 L[c] += acc;
             }
         }
+        __syncwarp();
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = H / 2; o > 0; o >>= 1)
 #pragma unroll
-            for (int c = 0; c < kNC; ++c) L[c] += __shfl_down_sync(kFull, L[c], o);
-            used += __shfl_down_sync(kFull, used, o);
-        }
-        if (lane == 0) {
+            for (int c = 0; c < kNC; ++c) L[c] += __shfl_down_sync(kFull, L[c], o, H);
+        if (lane == 0 && s0 < nsink) {
 #pragma unroll
             for (int c = 0; c < kNC; ++c) f.sinkL[(size_t)kNC * s + c] = L[c];
-            if (used) atomicAdd(applied, (unsigned long long)used);
         }
-        __syncwarp();  // the shared buffer is rewritten by the next sink
     }
+    used = __reduce_add_sync(kFull, used);
+    if ((threadIdx.x & 31) == 0 && used) atomicAdd(applied, (unsigned long long)used);
 }
 
 // Locals down each leaf's path from the root, then the gradient at the
@@ -554,7 +399,9 @@ int blocks_for(long long n, int threads) {
 struct p2p_fmm {
     int device = 0;
     cudaStream_t stream = nullptr;
-    DevBufF parents, leafM, nodeM, sinkL, leafL, front[2], tasks, counts, off, tiles, seg, seg2, ctrl;
+    DevBufF parents, leafM, nodeM, sinkL, leafL, counts, ctrl;
+    DevBufF box, items, lists[2], tasks, walk_ctrl;  // the M2L walk
+    int64_t list_cap = 0, task_cap = 0;              // chunks of its pools
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     long long n_m2l = 0, n_applied = 0;
     int levels = 0, nleaf = 0, nnode = 0;
@@ -593,8 +440,8 @@ P2P_API int p2p_fmm_destroy(p2p_fmm *f) {
     if (!f) return P2P_OK;
     cudaSetDevice(f->device);
     cudaStreamSynchronize(f->stream);
-    DevBufF *bufs[] = {&f->parents, &f->leafM, &f->nodeM, &f->sinkL, &f->leafL, &f->front[0], &f->front[1],
-                       &f->tasks, &f->counts, &f->off, &f->tiles, &f->seg, &f->seg2, &f->ctrl};
+    DevBufF *bufs[] = {&f->parents, &f->leafM, &f->nodeM, &f->sinkL, &f->leafL, &f->counts, &f->ctrl, &f->box,
+                       &f->items, &f->lists[0], &f->lists[1], &f->tasks, &f->walk_ctrl};
     for (DevBufF *b : bufs)
         if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : f->ev)
@@ -636,8 +483,6 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     FMM_TRY(grow(f->sinkL, sizeof(double) * kNC * (size_t)nsink));
     FMM_TRY(grow(f->leafL, sizeof(double) * kNC * (size_t)nleaf));
     FMM_TRY(grow(f->counts, sizeof(int) * 2 * (size_t)nsink));
-    FMM_TRY(grow(f->off, sizeof(int64_t) * ((size_t)nsink + 1)));
-    FMM_TRY(grow(f->tiles, sizeof(int64_t) * (((size_t)nsink + kScanTile - 1) / kScanTile + 1)));
     FMM_TRY(grow(f->ctrl, 64));
     FmmArgs a;
     a.w.nnode = nnode;
@@ -675,84 +520,86 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     fmm_upward_kernel<<<blocks_for(nleaf, threads), threads, 0, st>>>(a);
     FMM_CUDA(cudaEventRecord(f->ev[1], st), "FMM upward");
 
-    // M2L walk, one level per launch
-    long long nin = 0, ntask = 0;
+    // M2L walk, one depth of sinks per launch: every sink's tasks into a pool
+    // of chunks (sizes are first guesses: a walk that runs out of one is
+    // repeated with twice the size)
+    int *head = (int *)f->counts.p, *len = head + nsink;
+    FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
+    WalkRun g;
+    std::memset(&g, 0, sizeof(g));
+    unsigned long long ntask = 0;
     if (nnode) {
-        long long fcap = std::max<long long>(4LL * nsink, 1024), tcap = std::max<long long>(4LL * nsink, 1024);
-        FMM_TRY(grow(f->front[0], sizeof(int2) * (size_t)fcap));
-        FMM_TRY(grow(f->front[1], sizeof(int2) * (size_t)fcap));
-        FMM_TRY(grow(f->tasks, sizeof(int2) * (size_t)tcap));
-        const int2 root = make_int2(1, 1);
-        FMM_CUDA(cudaMemcpyAsync(f->front[0].p, &root, sizeof(int2), cudaMemcpyHostToDevice, st), "FMM walk");
-        nin = 1;
-        int cur = 0;
-        unsigned long long h[2];
-        while (nin > 0) {
-            if (++f->levels > 4096) return report_error(P2P_ERR_CAPACITY, "FMM walk: too many levels");
-            const unsigned long long t0 = (unsigned long long)ntask;
-            FMM_CUDA(cudaMemsetAsync(ctrl, 0, sizeof(unsigned long long), st), "FMM walk");
-            FMM_CUDA(cudaMemcpyAsync(ctrl + 1, &t0, sizeof(t0), cudaMemcpyHostToDevice, st), "FMM walk");
-            fmm_walk_kernel<<<blocks_for(nin, threads), threads, 0, st>>>(
-                a.w, (const int2 *)f->front[cur].p, (int)nin, (int2 *)f->front[cur ^ 1].p, fcap, ctrl,
-                (int2 *)f->tasks.p, tcap, ctrl + 1, a.status);
-            FMM_CUDA(cudaMemcpyAsync(h, ctrl, sizeof(h), cudaMemcpyDeviceToHost, st), "FMM walk");
-            FMM_CUDA(cudaStreamSynchronize(st), "FMM walk");
-            const long long nout = (long long)h[0], nt = (long long)h[1];
-            if (nout > fcap || nt > tcap) {
-                // grow and repeat the level (the input frontier is kept)
-                if (nout > fcap) {
-                    fcap = nout + nout / 2;
-                    DevBufF keep = f->front[cur];
-                    f->front[cur] = DevBufF();
-                    FMM_TRY(grow(f->front[cur], sizeof(int2) * (size_t)fcap));
-                    FMM_CUDA(cudaMemcpyAsync(f->front[cur].p, keep.p, sizeof(int2) * (size_t)nin,
-                                             cudaMemcpyDeviceToDevice, st), "FMM walk");
-                    FMM_CUDA(cudaStreamSynchronize(st), "FMM walk");
-                    cudaFree(keep.p);
-                    FMM_TRY(grow(f->front[cur ^ 1], sizeof(int2) * (size_t)fcap));
-                }
-                if (nt > tcap) {
-                    tcap = nt + nt / 2;
-                    DevBufF keep = f->tasks;
-                    f->tasks = DevBufF();
-                    FMM_TRY(grow(f->tasks, sizeof(int2) * (size_t)tcap));
-                    if (ntask)
-                        FMM_CUDA(cudaMemcpyAsync(f->tasks.p, keep.p, sizeof(int2) * (size_t)ntask,
-                                                 cudaMemcpyDeviceToDevice, st), "FMM walk");
-                    FMM_CUDA(cudaStreamSynchronize(st), "FMM walk");
-                    cudaFree(keep.p);
-                }
-                --f->levels;
-                continue;
+        int sms = 0;
+        FMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device), "FMM walk");
+        const int64_t slack = walk_pool_slack(sms);
+        f->list_cap = std::max(f->list_cap, 2 * (int64_t)nnode + slack);
+        f->task_cap = std::max(f->task_cap, 3 * (int64_t)nsink / 2 + slack);
+        g.nnode = nnode;
+        g.nleaf = nleaf;
+        g.node_first = t->node_first;
+        g.cutoff = cutoff;
+        g.open_angle = open_angle;
+        g.cut2 = (float)(cutoff * cutoff);
+        g.th2 = (float)(open_angle * open_angle);
+        g.out_head = head;
+        g.out_len = len;
+        const size_t nbox = 2 * ((size_t)std::max(nleaf, nnode) + 1);
+        FMM_TRY(grow(f->box, (sizeof(WalkBox) + sizeof(WalkBox32)) * nbox));
+        FMM_TRY(grow(f->items, sizeof(WalkItem) * 2 * (size_t)nleaf));
+        FMM_TRY(grow(f->walk_ctrl, sizeof(WalkCtrl)));
+        g.box = (const WalkBox *)f->box.p;
+        g.box32 = (const WalkBox32 *)(g.box + nbox);
+        g.items[0] = (WalkItem *)f->items.p;
+        g.items[1] = g.items[0] + nleaf;
+        g.ctrl = (WalkCtrl *)f->walk_ctrl.p;
+        for (bool again = true; again;) {
+            again = false;
+            for (int k = 0; k < 2; ++k) {
+                FMM_TRY(grow(f->lists[k], walk_pool_bytes(f->list_cap, kWalkChunk)));
+                g.lists[k] = walk_pool(f->lists[k].p, f->list_cap, kWalkChunk);
             }
-            ntask = nt;
-            nin = nout;
-            cur ^= 1;
+            FMM_TRY(grow(f->tasks, walk_pool_bytes(f->task_cap, kWalkTaskChunk)));
+            g.out = walk_pool(f->tasks.p, f->task_cap, kWalkTaskChunk);
+            FMM_CUDA(cudaMemsetAsync(g.ctrl, 0, sizeof(WalkCtrl), st), "FMM walk");
+            walk_pack_kernel<true><<<blocks_for((long long)nnode + nleaf, threads), threads, 0, st>>>(
+                a.w, (WalkBox *)f->box.p, (WalkBox32 *)((WalkBox *)f->box.p + nbox), nullptr, g.items[0], g.lists[0].ids, g.ctrl);
+            for (int lv = 0, n = walk_first_depths(nleaf);; n = 4) {
+                n = std::min(n, kWalkLevels - lv);
+                if (n <= 0) return report_error(P2P_ERR_CAPACITY, "FMM walk: too many levels");
+                FMM_CUDA(walk_depths<WALK_M2L>(st, g, sms, lv, n), "FMM walk");
+                count_launches(n);
+                lv += n;
+                std::vector<int> boxes(lv + 1);
+                int status = 0;
+                FMM_CUDA(cudaMemcpyAsync(boxes.data(), g.ctrl->items, sizeof(int) * (lv + 1), cudaMemcpyDeviceToHost, st),
+                         "FMM walk");
+                FMM_CUDA(cudaMemcpyAsync(&status, &g.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st), "FMM walk");
+                FMM_CUDA(cudaMemcpyAsync(&ntask, &g.ctrl->ntask, sizeof(ntask), cudaMemcpyDeviceToHost, st), "FMM walk");
+                FMM_CUDA(cudaStreamSynchronize(st), "FMM walk");
+                if (status & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
+                if (status & ST_WALK_STACK) return report_error(P2P_ERR_CAPACITY, "FMM walk: stack exceeded");
+                if (status) {
+                    if (status & ST_WALK_LISTS) f->list_cap *= 2;
+                    if (status & ST_WALK_OUT) f->task_cap *= 2;
+                    if (std::max(f->list_cap, f->task_cap) > INT32_MAX)
+                        return report_error(P2P_ERR_CAPACITY, "FMM walk: more lists than a pool can hold");
+                    FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
+                    again = true;
+                    break;
+                }
+                if (boxes[lv] == 0) {
+                    f->levels = lv - (int)std::count(boxes.begin(), boxes.begin() + lv, 0);
+                    break;
+                }
+            }
         }
     }
-    f->n_m2l = ntask;
+    f->n_m2l = (long long)ntask;
     FMM_CUDA(cudaEventRecord(f->ev[2], st), "FMM walk");
 
-    // M2L: tasks grouped by sink, each sink's sum in increasing source order
-    int *count = (int *)f->counts.p, *fill = count + nsink;
-    int64_t *off = (int64_t *)f->off.p;
-    FMM_TRY(grow(f->seg, sizeof(int) * (size_t)std::max<long long>(ntask, 1)));
-    FMM_TRY(grow(f->seg2, sizeof(int) * (size_t)std::max<long long>(ntask, 1)));
-    FMM_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * 2 * (size_t)nsink, st), "FMM m2l");
-    if (ntask)
-        fmm_task_count_kernel<<<blocks_for(ntask, threads), threads, 0, st>>>(a.w, (const int2 *)f->tasks.p, ntask,
-                                                                               count);
-    const int ntiles = (int)(((int64_t)nsink + kScanTile - 1) / kScanTile);
-    int64_t *tiles = (int64_t *)f->tiles.p;
-    scan_tiles_kernel<<<ntiles, kScanThreads, 0, st>>>(count, nsink, off, tiles);
-    scan_sums_kernel<<<1, kScanThreads, 0, st>>>(tiles, ntiles, off + nsink);
-    // one thread per element (the kernel has no grid-stride loop)
-    scan_add_kernel<<<(nsink + threads - 1) / threads, threads, 0, st>>>(off, nsink, tiles);
-    if (ntask)
-        fmm_task_fill_kernel<<<blocks_for(ntask, threads), threads, 0, st>>>(a.w, (const int2 *)f->tasks.p, ntask,
-                                                                              off, fill, (int *)f->seg.p);
-    fmm_m2l_kernel<<<(int)std::min<long long>(((long long)nsink + kM2LWarps - 1) / kM2LWarps, 148LL * 16),
-                     32 * kM2LWarps, 0, st>>>(a, off, (const int *)f->seg.p, (int *)f->seg2.p, ctrl + 2);
+    // M2L: each sink's sum over its tasks
+    fmm_m2l_kernel<<<(int)std::min<long long>(((long long)nsink * kWalkTaskChunk + kM2LThreads - 1) / kM2LThreads, 148LL * 16),
+                     kM2LThreads, 0, st>>>(a, head, len, g.out, ctrl + 2);
     FMM_CUDA(cudaEventRecord(f->ev[3], st), "FMM m2l");
     fmm_downward_kernel<<<blocks_for(nleaf, 128), 128, 0, st>>>(a, d_acc);
     FMM_CUDA(cudaEventRecord(f->ev[4], st), "FMM downward");
@@ -761,9 +608,8 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     FMM_CUDA(cudaMemcpyAsync(h2, ctrl + 2, sizeof(h2), cudaMemcpyDeviceToHost, st), "FMM");
     FMM_CUDA(cudaStreamSynchronize(st), "FMM");
     f->n_applied = (long long)h2[0];
-    count_launches(4 + f->levels + (ntask ? 5 : 3));
+    count_launches(nnode ? 5 : 3);
     if ((int)h2[1] & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
-    if ((int)h2[1] & ST_WALK_ROW) return report_error(P2P_ERR_STATE, "FMM: M2L task offsets out of order");
     return P2P_OK;
 }
 

@@ -1,28 +1,43 @@
-// Device interaction-list walk: the P2P lists of PhotoNs' dual-tree walk
-// (walk_task_p2p, src/fmm.c:656-792, with the LONGSHORT acceptance test of
-// src/fmm.c:409-479) computed per sink leaf on the GPU, straight into CSR rows.
+// Device interaction-list walks on the kd-tree: the P2P lists of PhotoNs'
+// dual-tree walk (walk_task_p2p, src/fmm.c:656-792) straight into CSR rows, and
+// the M2L tasks of its walk_task_m2l (src/fmm.c:812-957), both with the
+// LONGSHORT acceptance test of src/fmm.c:409-479.
 //
-// The serial walk recurses over leaf/node pairs (A, B) from (root, root). An
-// entry (L, S) is emitted when the recursion reaches two leaves. For a fixed
-// sink leaf L the pairs it visits on the way to L's entries have A on L's
-// ancestor path, and which child of A the recursion takes is fixed by L (the
-// child whose subtree holds L); how a pair expands depends on the pair alone.
-// So one warp per sink leaf expands that part of the recursion, its lanes
-// taking up to 32 pending pairs at a time from a shared-memory stack. The
-// serial walk emits a sink's sources in pre-order of the source side, i.e. in
-// increasing leaf id (leaves are numbered in pre-order and son[0]'s subtree is
-// walked before son[1]'s); sorting each row ascending afterwards therefore
-// gives the serial order, the row a stable sort of the serial list by sink
-// gives: the rows equal those the list path builds, entry for entry.
+// The serial walks recurse over box pairs (A, B) from (root, root): a pair of
+// boxes is dropped or accepted, or the larger box is opened; (A, A) opens on
+// both sides. How a pair goes on depends on the pair alone. So the sink side
+// is taken depth by depth (walk_level_kernel, one launch per depth, one warp
+// per box A): A receives its parent's list of undecided boxes B, in leaf
+// order; opens those B that are to be opened until each is dropped, accepted,
+// kept (A is to be opened: both children of A receive the kept list) or, for
+// two leaves, emitted. A pair is tested once for all the leaves below A, where
+// a walk per sink leaf tests it again for each of them (51 ms at 256^3), and A's
+// box is in registers, so a test reads one 32-byte record: the test is bounded
+// in FP32 (p2p_walk_test.h) and repeated in FP64 only where the bound does not
+// decide. A dependent FP64 operation takes about 16 cycles and a test has some
+// 25 in a row, so in FP64 the warps mostly waited for it.
 //
-// The acceptance arithmetic is written with explicitly rounded FP64
-// operations (no contraction), the ISO C evaluation of the reference's code.
+// Order: the serial walk emits a sink's sources in pre-order of the source
+// side, i.e. in increasing leaf id (leaves are numbered in pre-order and
+// son[0]'s subtree is walked before son[1]'s). A warp keeps the boxes in that
+// order: it takes up to 32 of the first ones (from a stack of opened boxes with
+// the first on top, then from the input list), writes out the decided ones
+// that precede every box still to be opened, and puts the rest back with
+// opened boxes replaced by their children. Rows come out sorted and equal those
+// the list path builds, entry for entry, with no sort (20 ms at 256^3).
+//
+// Lists are chains of chunks of a pool, as their lengths are not known before
+// they are made. The acceptance arithmetic is written with explicitly rounded
+// FP64 operations (no contraction), the ISO C evaluation of the reference's
+// code.
 #pragma once
 
 #include "p2p_device_common.cuh"
+#include "p2p_walk_test.h"
 
 namespace p2p {
 
+// The tree as the walks' other users see it.
 struct WalkArgs {
     int nnode, nleaf;
     const int *son;           // 2 * nnode encoded children: leaf l -> 2l, node k -> 2k + 1
@@ -34,9 +49,11 @@ struct WalkArgs {
 };
 
 enum : int {
-    ST_WALK_STACK = 4,    // a sink's pending pairs exceeded the walk's stack (its row is cut short)
-    ST_WALK_ROW = 8,      // the fill pass found more entries than the count pass
-    ST_WALK_TREE = 16,    // a child code outside the tree, or a walk longer than any tree allows
+    ST_WALK_STACK = 4,    // a box's opened boxes exceeded the walk's stack
+    ST_WALK_ROW = 8,      // a row came out longer than it was counted (or, in the FMM, offsets out of order)
+    ST_WALK_TREE = 16,    // a child code outside the tree, leaves not in pre-order, or a walk longer than any tree allows
+    ST_WALK_LISTS = 32,   // the pool of undecided lists is full (the host enlarges it and repeats the walk)
+    ST_WALK_OUT = 64,     // the pool of rows (or M2L tasks) is full
 };
 
 __device__ __forceinline__ const double *walk_center(const WalkArgs &w, int c) {
@@ -46,14 +63,27 @@ __device__ __forceinline__ const double *walk_width(const WalkArgs &w, int c) {
     return (c & 1) ? w.node_width + 3 * (size_t)(c >> 1) : w.leaf_width + 3 * (size_t)(c >> 1);
 }
 
+__device__ __forceinline__ bool walk_valid(const WalkArgs &w, int c) {
+    return c >= 0 && ((c & 1) ? (c >> 1) < w.nnode : (c >> 1) < w.nleaf);
+}
+
+// The child of node code A whose subtree holds leaf L (pre-order leaf ids:
+// son[0]'s leaves precede son[1]'s); -1 for a child code outside the tree.
+__device__ __forceinline__ int walk_child_toward(const WalkArgs &w, int A, int L) {
+    const int k = A >> 1;
+    const int s1 = w.son[2 * k + 1];
+    if (!walk_valid(w, s1)) return -1;
+    const int f1 = (s1 & 1) ? w.node_first[s1 >> 1] : (s1 >> 1);
+    return L < f1 ? w.son[2 * k] : s1;
+}
+
 // acceptance (LONGSHORT), src/fmm.c:409-479: 0 open, 1 accept (M2L), -1 drop.
-__device__ __forceinline__ int walk_acceptance(const double *wi, const double *wj, const double *ci,
-                                               const double *cj, double cutoff, double open_angle) {
+__device__ __forceinline__ int walk_acceptance(const WalkBox &i, const WalkBox &j, double cutoff, double open_angle) {
     double dist[3], w[3], mn[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        dist[d] = __dsub_rn(ci[d], cj[d]);
-        w[d] = __dmul_rn(__dadd_rn(wi[d], wj[d]), 0.5);
+        dist[d] = __dsub_rn(i.c[d], j.c[d]);
+        w[d] = __dmul_rn(__dadd_rn(i.w[d], j.w[d]), 0.5);
     }
     const double dd2 = __dadd_rn(__dadd_rn(__dmul_rn(dist[0], dist[0]), __dmul_rn(dist[1], dist[1])),
                                  __dmul_rn(dist[2], dist[2]));
@@ -76,212 +106,387 @@ __device__ __forceinline__ int walk_acceptance(const double *wi, const double *w
     return 0;
 }
 
-__device__ __forceinline__ bool walk_valid(const WalkArgs &w, int c) {
-    return c >= 0 && ((c & 1) ? (c >> 1) < w.nnode : (c >> 1) < w.nleaf);
+constexpr int kWalkWarps = 4;      // boxes in flight per block
+constexpr int kWalkStack = 1024;   // opened boxes per warp (shared memory)
+constexpr int kWalkChunk = 64;     // ids per chunk of a list of undecided boxes or of a row
+constexpr int kWalkTaskChunk = 16; // ids per chunk of a sink's M2L tasks (about 10 at open angle 0.4)
+constexpr int kWalkGrab = 16;      // chunks a warp takes from a pool at a time
+constexpr int kWalkLevels = 4096;  // most depths of a walk
+
+// A sink-side box to be walked at a depth.
+struct WalkItem {
+    int code, parent;  // the box, and the node it is a child of (-1: the root)
+    int lo, hi;        // leaf ids of its subtree [lo, hi) (P2P walk)
+    int head, len;     // its parent's undecided boxes
+};
+
+struct WalkPool {
+    int *ids;   // cap chunks
+    int *next;  // cap: the chunk after this one in its list
+    int cap;
+};
+
+// Device counters of one walk.
+struct WalkCtrl {
+    int items[kWalkLevels + 1];   // boxes of each depth
+    int lists[kWalkLevels + 1];   // chunks taken by each depth's undecided lists
+    int taken[kWalkLevels + 1];   // boxes of each depth taken by warps beyond their first
+    int out;                      // chunks taken by rows or tasks
+    int status;                   // ST_WALK_* bits of this walk
+    unsigned long long ntask;     // M2L tasks
+};
+
+enum WalkMode {
+    WALK_ROWS = 0,   // P2P rows into the pool of chunks
+    WALK_COUNT = 1,  // P2P row lengths only
+    WALK_FILL = 2,   // P2P rows into row_src[row_off[L] ...]
+    WALK_M2L = 3,    // M2L tasks of every box into the pool of chunks
+};
+
+struct WalkRun {
+    int nnode, nleaf;
+    const WalkBox *box;        // box code c at index c
+    const WalkBox32 *box32;
+    float cut2, th2;           // squares of cutoff and open angle
+    const int64_t *active;     // nleaf + 1: active leaves before each leaf (P2P)
+    const int *node_first;
+    double cutoff, open_angle;
+    WalkItem *items[2];        // this depth's boxes, the next one's
+    WalkPool lists[2];         // the lists they receive, those they leave
+    WalkPool out;
+    int *out_head, *out_len;   // per leaf (P2P) or per sink, leaves then nodes (M2L)
+    const int64_t *row_off;    // WALK_FILL
+    int *row_src;
+    WalkCtrl *ctrl;
+};
+
+// The boxes' records, the leaves' active flags and the first depth (the root
+// with itself as its one undecided box).
+template <bool M2L>
+__global__ void __launch_bounds__(256)
+walk_pack_kernel(const WalkArgs w, WalkBox *__restrict__ box, WalkBox32 *__restrict__ box32,
+                 int *__restrict__ flag, WalkItem *items,
+                 int *lists, WalkCtrl *ctrl) {
+    const int n = w.nnode + w.nleaf;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const bool leaf = i < w.nleaf;
+        const int k = leaf ? i : i - w.nleaf;
+        const double *c = leaf ? w.leaf_center + 3 * (size_t)k : w.node_center + 3 * (size_t)k;
+        const double *v = leaf ? w.leaf_width + 3 * (size_t)k : w.node_width + 3 * (size_t)k;
+        WalkBox b;
+        WalkBox32 f;
+        for (int d = 0; d < 3; ++d) {
+            b.c[d] = c[d];
+            b.w[d] = v[d];
+            f.c[d] = (float)c[d];
+            f.w[d] = (float)v[d];
+        }
+        b.sum = __dadd_rn(__dadd_rn(v[0], v[1]), v[2]);
+        b.pad = 0.0;
+        f.son[0] = leaf ? -1 : w.son[2 * k];
+        f.son[1] = leaf ? -1 : w.son[2 * k + 1];
+        const int code = leaf ? 2 * k : 2 * k + 1;
+        box[code] = b;
+        box32[code] = f;
+        if (!M2L && leaf) flag[k] = w.leaf_active[k] >= 0 ? 1 : 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        items[0] = WalkItem{1, -1, 0, w.nleaf, 0, 1};
+        lists[0] = 1;  // the root's code
+        ctrl->items[0] = 1;
+    }
 }
 
-// The child of node code A whose subtree holds leaf L (pre-order leaf ids:
-// son[0]'s leaves precede son[1]'s); -1 for a child code outside the tree.
-__device__ __forceinline__ int walk_child_toward(const WalkArgs &w, int A, int L) {
-    const int k = A >> 1;
-    const int s1 = w.son[2 * k + 1];
-    if (!walk_valid(w, s1)) return -1;
-    const int f1 = (s1 & 1) ? w.node_first[s1 >> 1] : (s1 >> 1);
-    return L < f1 ? w.son[2 * k] : s1;
+__device__ __forceinline__ WalkBox32 walk_load(const WalkBox32 *p) {
+    WalkBox32 b;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(b.c[0]), "=f"(b.c[1]), "=f"(b.c[2]), "=f"(b.w[0]), "=f"(b.w[1]), "=f"(b.w[2]),
+          "=f"(reinterpret_cast<float &>(b.son[0])), "=f"(reinterpret_cast<float &>(b.son[1]))
+        : "l"(__cvta_generic_to_global(p)));
+    return b;
 }
 
-constexpr int kWalkWarps = 4;         // warps (sink leaves in flight) per block
-constexpr int kWalkWarpStack = 1024;  // pending pairs per warp (shared memory)
+// The exact test where the bound does not decide: the same outcomes.
+static __device__ __noinline__ int walk_exact(const WalkBox *box, int A, int B, double cutoff, double open_angle) {
+    const WalkBox a = box[A], b = box[B];
+    const int t = walk_acceptance(a, b, cutoff, open_angle);
+    if (t != 0) return t == 1 ? WALK_ACCEPT : WALK_DROP;
+    return (A & 1) && (!(B & 1) || a.sum > b.sum) ? WALK_OPEN_A : WALK_OPEN_B;
+}
 
-// One warp per sink leaf. FILL = false: row lengths into counts[L]; with a
-// slab, also the row's first slab_cap source ids into slab[L * slab_cap ...]
-// (walk_gather_kernel moves them into the rows). FILL = true: the row's
-// source ids into row_src[row_off[L] ...] (in the order the warp finds them;
-// the rows are sorted afterwards), the row's pair count (and, with skipped,
-// the pairs of entries wholly beyond the FP32 forms' cutoff) added into
-// *pairs / *skipped; with slab_cap > 0 only for the rows longer than
-// slab_cap (counts[L] from the first pass), the others having been gathered.
-template <bool FILL>
-__global__ void __launch_bounds__(kWalkWarps * 32)
-walk_rows_kernel(const WalkArgs w, int *__restrict__ counts, const int64_t *__restrict__ row_off,
-                 int *__restrict__ row_src, const int *__restrict__ leaf_npart,
-                 const LeafMeta *__restrict__ meta, double cscale, float uout,
-                 unsigned long long *__restrict__ pairs, unsigned long long *__restrict__ skipped,
-                 int *__restrict__ status, int *__restrict__ slab, int slab_cap) {
-    __shared__ int2 stacks[kWalkWarps][kWalkWarpStack];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    int2 *stk = stacks[wid];
-    unsigned long long my_pairs = 0, my_skip = 0;
-    for (int L = blockIdx.x * kWalkWarps + wid; L < w.nleaf; L += gridDim.x * kWalkWarps) {
-        if (w.leaf_active[L] < 0 || w.nnode <= 0) {  // warp-uniform
-            if (!FILL && lane == 0) counts[L] = 0;
-            continue;
-        }
-        if (FILL && slab_cap > 0 && counts[L] <= slab_cap) continue;  // gathered from the slab (warp-uniform)
-        if (lane == 0) stk[0] = make_int2(1, 1);  // (root, root): node 0
-        __syncwarp();
-        int sp = 1, n = 0, bad = 0;
-        int64_t base = 0, cap = 0;
-        LeafMeta mt{};
-        long long np_t = 0;
-        if (FILL) {
-            base = row_off[L];
-            cap = row_off[L + 1] - base;
-            np_t = leaf_npart[L];
-            if (skipped) mt = meta[L];
-        }
-        // every pair is visited at most once per sink: a longer walk means a
-        // malformed tree
-        long long budget = 64LL * ((long long)w.nnode + w.nleaf) + 16;
-        while (sp > 0) {
-            const int take = min(32, sp);
-            sp -= take;
-            budget -= take;
-            int2 p = make_int2(0, 0);
-            if (lane < take) p = stk[sp + lane];
-            __syncwarp();  // the batch is read before children overwrite it
-            const int A = p.x, B = p.y;
-            int nchild = 0, c0 = 0, c1 = 0, fault = 0;
-            bool emit = false;
-            if (lane < take) {
-                const bool a_node = A & 1, b_node = B & 1;
-                if ((A == B && !a_node) || (!a_node && !b_node)) {
-                    emit = true;
-                } else if (A == B) {
-                    const int c = walk_child_toward(w, A, L);
-                    const int k = A >> 1;
-                    c0 = c;  // the pairs (c, son[0]) and (c, son[1]): second codes below
-                    nchild = 2;
-                    p = make_int2(w.son[2 * k], w.son[2 * k + 1]);
-                } else {
-                    const double *wa = walk_width(w, A), *wb = walk_width(w, B);
-                    if (walk_acceptance(wa, wb, walk_center(w, A), walk_center(w, B), w.cutoff,
-                                        w.open_angle) == 0) {
-                        bool split_a = a_node && !b_node;
-                        if (a_node && b_node)
-                            split_a = __dadd_rn(__dadd_rn(wa[0], wa[1]), wa[2]) >
-                                      __dadd_rn(__dadd_rn(wb[0], wb[1]), wb[2]);
-                        if (split_a) {
-                            c0 = walk_child_toward(w, A, L);
-                            c1 = B;
-                            nchild = 1;
-                        } else {
-                            const int k = B >> 1;
-                            c0 = A;
-                            nchild = 2;
-                            p = make_int2(w.son[2 * k], w.son[2 * k + 1]);
-                        }
-                    }
+// One warp's list being written: ids appended in order, CHUNK per chunk.
+template <int CHUNK>
+struct WalkWriter {
+    int head, cur, n;  // first and current chunk, ids so far
+    int base, left;    // chunks taken from the pool and not yet used (kept between lists)
+    __device__ __forceinline__ void start() { n = 0; head = cur = -1; }
+    // Appends the ids of the lanes in mask, in lane order; false when the pool is full.
+    __device__ __forceinline__ bool append(unsigned mask, int id, const WalkPool &p, int *taken) {
+        const int k = __popc(mask);
+        if (k == 0) return true;
+        const int lane = threadIdx.x & 31;
+        const int off = n % CHUNK;
+        int room = off ? CHUNK - off : 0;  // left in the current chunk
+        const int rank = __popc(mask & ((1u << lane) - 1u));
+        const bool mine = mask >> lane & 1u;
+        if (mine && rank < room) p.ids[(size_t)cur * CHUNK + off + rank] = id;
+        while (k > room) {  // at most once where CHUNK >= 32
+            if (left == 0) {
+                if (lane == 0) base = atomicAdd(taken, kWalkGrab);
+                base = __shfl_sync(kFull, base, 0);
+                left = kWalkGrab;
+                if (base < 0 || base > p.cap - kWalkGrab) {
+                    left = 0;
+                    return false;
                 }
             }
-            // children as (first, second) codes: nchild 1 -> (c0, c1);
-            // nchild 2 -> (c0, p.x), (c0, p.y)
-            int2 ch0 = nchild == 1 ? make_int2(c0, c1) : make_int2(c0, p.x);
-            int2 ch1 = make_int2(c0, p.y);
-            if (nchild >= 1 && (!walk_valid(w, ch0.x) || !walk_valid(w, ch0.y))) fault = ST_WALK_TREE;
-            if (nchild == 2 && !walk_valid(w, ch1.y)) fault = ST_WALK_TREE;
-            if (fault) nchild = 0;
-            int incl = nchild;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int v = __shfl_up_sync(kFull, incl, off);
-                if (lane >= off) incl += v;
+            const int c = base++;
+            --left;
+            if (cur < 0) head = c;
+            else if (lane == 0) p.next[cur] = c;
+            cur = c;
+            if (mine && rank >= room && rank < room + CHUNK) p.ids[(size_t)c * CHUNK + rank - room] = id;
+            room += CHUNK;
+        }
+        n += k;
+        return true;
+    }
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kWalkWarps * 32, 8) walk_level_kernel(const WalkRun g, int level) {
+    constexpr bool M2L = MODE == WALK_M2L;
+    constexpr int OUT = M2L ? kWalkTaskChunk : kWalkChunk;
+    __shared__ int stacks[kWalkWarps][kWalkStack];
+    __shared__ WalkItem pushed[kWalkWarps][32];  // children for the next depth, written 31 or more at a time
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u, above = ~(lt | (1u << lane));
+    const int count = g.ctrl->items[level];
+    int i = blockIdx.x * kWalkWarps + wid;
+    if (i >= count || g.ctrl->status) return;  // (a walk that failed is not continued)
+    int *stk = stacks[wid];
+    const WalkItem *in = g.items[level & 1];
+    WalkItem *next_items = g.items[(level & 1) ^ 1];
+    const WalkPool from = g.lists[level & 1], to = g.lists[(level & 1) ^ 1];
+    WalkWriter<kWalkChunk> kept;
+    WalkWriter<OUT> out;
+    kept.base = kept.left = out.base = out.left = 0;
+    int npushed = 0, fault = 0;
+    unsigned long long ntask = 0;
+    auto flush = [&]() {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&g.ctrl->items[level + 1], npushed);
+        at = __shfl_sync(kFull, at, 0);
+        // disjoint subtrees: at most nleaf boxes a depth in a well-formed tree
+        if (at < 0 || at + npushed > g.nleaf) fault |= ST_WALK_TREE;
+        else if (lane < npushed) next_items[at + lane] = pushed[wid][lane];
+        npushed = 0;
+        __syncwarp();
+    };
+    // lists differ by a factor of a hundred between voids and halos, so warps
+    // take boxes as they get free, each one's next asked for before it is needed
+    int after = 0;
+    for (; i < count && !fault; i = gridDim.x * kWalkWarps + __shfl_sync(kFull, after, 0)) {
+        if (lane == 0) after = atomicAdd(&g.ctrl->taken[level], 1);
+        const WalkItem it = in[i];
+        const int A = it.code;
+        const bool a_leaf = !(A & 1);
+        const WalkBox32 a = walk_load(g.box32 + A);
+        const bool fill = MODE == WALK_FILL && a_leaf;
+        const int64_t row = fill ? g.row_off[A >> 1] : 0;
+        const int cap = fill ? (int)(g.row_off[(A >> 1) + 1] - row) : 0;
+        int chunk = it.head, chunk_next = it.len > kWalkChunk ? from.next[it.head] : 0;
+        int sp = 0, pos = 0, emitted = 0;
+        kept.start();
+        out.start();
+        // a pair is met at most once: a longer walk means a malformed tree
+        long long budget = 2LL * ((long long)g.nnode + g.nleaf) + 64;
+        while (sp > 0 || pos < it.len) {
+            // the first boxes: from the stack, then from the input
+            const int ns = min(32, sp), ni = min(32 - ns, it.len - pos);
+            int v = 0;
+            if (lane < ns) {
+                v = stk[sp - 1 - lane];
+            } else if (lane < ns + ni) {
+                const int o = (pos & (kWalkChunk - 1)) + lane - ns;
+                v = o < kWalkChunk ? from.ids[(size_t)chunk * kWalkChunk + o]
+                                   : from.ids[(size_t)chunk_next * kWalkChunk + o - kWalkChunk];
             }
-            const int total = __shfl_sync(kFull, incl, 31);
-            bad |= __reduce_or_sync(kFull, fault);
-            if (sp + total > kWalkWarpStack) {
-                bad |= ST_WALK_STACK;
+            __syncwarp();  // the boxes are read before others are put in their places
+            sp -= ns;
+            if ((pos & (kWalkChunk - 1)) + ni >= kWalkChunk) {
+                chunk = chunk_next;
+                if (it.len - (pos + ni) > kWalkChunk - ((pos + ni) & (kWalkChunk - 1))) chunk_next = from.next[chunk];
+            }
+            pos += ni;
+            budget -= ni;
+            // 0 dropped, 1 decided (emitted or kept), 2 opened
+            int cls = 0, c0 = -1, c1 = -1, B = v;
+            bool task = false;
+            if (lane < ns + ni) {
+                if (v < 0) {  // decided before
+                    B = ~v;
+                    cls = 1;
+                } else if (a_leaf && !(B & 1)) {
+                    cls = M2L ? 0 : 1;
+                } else if (A == B) {
+                    cls = 1;
+                } else {
+                    const WalkBox32 b = walk_load(g.box32 + B);
+                    if (B == it.parent) {  // (parent, parent) opened on both sides
+                        cls = 2;
+                    } else {
+                        int t = walk_bound(a, b, !a_leaf, B & 1, g.cut2, g.th2);
+                        if (t == WALK_UNDECIDED) t = walk_exact(g.box, A, B, g.cutoff, g.open_angle);
+                        cls = t == WALK_OPEN_A ? 1 : (t == WALK_OPEN_B ? 2 : 0);
+                        task = M2L && t == WALK_ACCEPT;
+                    }
+                    c0 = b.son[0];
+                    c1 = b.son[1];
+                }
+            }
+            int nc = 0;
+            if (cls == 2) {
+                const bool v0 = c0 >= 0 && ((c0 & 1) ? (c0 >> 1) < g.nnode : (c0 >> 1) < g.nleaf);
+                const bool v1 = c1 >= 0 && ((c1 & 1) ? (c1 >> 1) < g.nnode : (c1 >> 1) < g.nleaf);
+                // the M2L walk passes over absent children
+                if ((!v0 && (!M2L || c0 >= 0)) || (!v1 && (!M2L || c1 >= 0))) fault = ST_WALK_TREE;
+                if (!v0) c0 = c1;
+                nc = (v0 ? 1 : 0) + (v1 ? 1 : 0);
+            }
+            const unsigned open = __ballot_sync(kFull, cls == 2);
+            const unsigned ready = open ? (open & (0u - open)) - 1u : kFull;  // lanes before the first opened box
+            const unsigned done = __ballot_sync(kFull, cls == 1);
+            if (M2L) {
+                const unsigned tm = __ballot_sync(kFull, task);
+                if (!out.append(tm, B, g.out, &g.ctrl->out)) fault |= ST_WALK_OUT;
+                if (!a_leaf && !kept.append(done & ready, B, to, &g.ctrl->lists[level])) fault |= ST_WALK_LISTS;
+            } else if (!a_leaf) {
+                if (!kept.append(done & ready, B, to, &g.ctrl->lists[level])) fault |= ST_WALK_LISTS;
             } else {
-                const int at = sp + incl - nchild;
-                if (nchild >= 1) stk[at] = ch0;
-                if (nchild == 2) stk[at + 1] = ch1;
+                const unsigned m = done & ready;
+                if (MODE == WALK_ROWS) {
+                    if (!out.append(m, B >> 1, g.out, &g.ctrl->out)) fault |= ST_WALK_OUT;
+                } else if (MODE == WALK_FILL && (m >> lane & 1u)) {
+                    const int slot = emitted + __popc(m & lt);
+                    if (slot < cap) g.row_src[row + slot] = B >> 1;
+                    else fault |= ST_WALK_ROW;
+                }
+                emitted += __popc(m);
+            }
+            // the others back on the stack, the first on top
+            const unsigned back = done & ~ready;
+            const unsigned one = __ballot_sync(kFull, nc >= 1), two = __ballot_sync(kFull, nc == 2);
+            const int total = __popc(back) + __popc(one) + __popc(two);
+            if (sp + total > kWalkStack) {
+                fault |= ST_WALK_STACK;
+            } else {
+                const int at = sp + __popc(back & above) + __popc(one & above) + __popc(two & above);
+                if (back >> lane & 1u) stk[at] = ~B;
+                if (nc == 1) stk[at] = c0;
+                if (nc == 2) {
+                    stk[at] = c1;
+                    stk[at + 1] = c0;
+                }
                 sp += total;
             }
-            const unsigned em = __ballot_sync(kFull, emit);
-            if (emit) {
-                const int slot = n + __popc(em & lt);
-                const int S = B >> 1;
-                if (!FILL && slab && slot < slab_cap) slab[(int64_t)L * slab_cap + slot] = S;
-                if (FILL) {
-                    if (slot < cap) {
-                        row_src[base + slot] = S;
-                        const unsigned long long np = (unsigned long long)(np_t * (long long)leaf_npart[S]);
-                        my_pairs += np;
-                        if (skipped) {
-                            const LeafMeta ms = meta[S];
-                            float ox, oy, oz;
-                            entry_offset(ms, mt, cscale, ox, oy, oz);
-                            if (entry_u_min(ms, mt, ox, oy, oz) > uout) my_skip += np;
-                        }
-                    }
+            budget -= __popc(one) + __popc(two);
+            if (budget < 0) fault |= ST_WALK_TREE;
+            fault = __reduce_or_sync(kFull, fault);
+            __syncwarp();
+            if (fault) break;  // warp-uniform
+        }
+        if (fault) break;
+        if (M2L) {
+            if (lane == 0) {
+                const int s = a_leaf ? A >> 1 : g.nleaf + (A >> 1);
+                g.out_head[s] = out.head;
+                g.out_len[s] = out.n;
+            }
+            ntask += (unsigned)out.n;
+        } else if (a_leaf) {
+            if (MODE != WALK_FILL && lane == 0) {
+                if (MODE == WALK_ROWS) g.out_head[A >> 1] = out.head;
+                g.out_len[A >> 1] = emitted;
+            }
+            if (fill && emitted != cap) fault |= ST_WALK_ROW;
+        }
+        if (!a_leaf && kept.n > 0) {  // A's children receive its undecided boxes
+            const int s0 = a.son[0], s1 = a.son[1];
+            int mid = it.lo;
+            bool go0 = s0 >= 0, go1 = s1 >= 0;
+            const bool v0 = s0 >= 0 && ((s0 & 1) ? (s0 >> 1) < g.nnode : (s0 >> 1) < g.nleaf);
+            const bool v1 = s1 >= 0 && ((s1 & 1) ? (s1 >> 1) < g.nnode : (s1 >> 1) < g.nleaf);
+            if ((!v0 && (!M2L || s0 >= 0)) || (!v1 && (!M2L || s1 >= 0))) fault |= ST_WALK_TREE;
+            if (!M2L && !fault) {
+                mid = (s1 & 1) ? g.node_first[s1 >> 1] : s1 >> 1;
+                // pre-order leaves: both subtrees hold some, a leaf holds itself
+                if (mid <= it.lo || mid >= it.hi) fault |= ST_WALK_TREE;
+                else if ((!(s0 & 1) && (s0 >> 1 != it.lo || mid != it.lo + 1)) || (!(s1 & 1) && it.hi != mid + 1))
+                    fault |= ST_WALK_TREE;
+                if (!fault) {  // subtrees without a sink need no walk
+                    go0 = g.active[mid] > g.active[it.lo];
+                    go1 = g.active[it.hi] > g.active[mid];
                 }
             }
-            n += __popc(em);
-            if (FILL && n > cap) bad |= ST_WALK_ROW;
-            if (budget < 0) bad |= ST_WALK_TREE;
-            __syncwarp();
-            if (bad) break;  // warp-uniform
-        }
-        if (lane == 0) {
-            if (!FILL) counts[L] = n;
-            if (bad) atomicOr(status, bad);
+            if (!fault) {
+                if (lane == 0) {
+                    if (go0) pushed[wid][npushed] = WalkItem{s0, A, it.lo, mid, kept.head, kept.n};
+                    if (go1) pushed[wid][npushed + (go0 ? 1 : 0)] = WalkItem{s1, A, mid, it.hi, kept.head, kept.n};
+                }
+                npushed += (go0 ? 1 : 0) + (go1 ? 1 : 0);
+                __syncwarp();
+                if (npushed > 30) flush();
+            }
         }
     }
-    if (FILL) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            my_pairs += __shfl_xor_sync(kFull, my_pairs, off);
-            my_skip += __shfl_xor_sync(kFull, my_skip, off);
-        }
-        if (lane == 0) {
-            if (my_pairs) atomicAdd(pairs, my_pairs);
-            if (skipped && my_skip) atomicAdd(skipped, my_skip);
-        }
+    if (!fault && npushed) flush();
+    fault = __reduce_or_sync(kFull, fault);
+    if (lane == 0) {
+        if (fault) atomicOr(&g.ctrl->status, fault);
+        if (M2L && ntask) atomicAdd(&g.ctrl->ntask, ntask);
     }
 }
 
-// Rows of at most slab_cap entries, from the first pass's slab into their
-// CSR rows (in the order the walk found them; the row sort follows), with the
-// pair counts the fill pass would add. One warp per sink leaf; a row whose
-// offsets disagree with its length, or an id outside the leaves, sets
-// ST_WALK_ROW and is skipped.
+// Rows from the pool into their CSR places (CHAINS; else they are there
+// already), and their pair counts (with skipped, the pairs of entries wholly
+// beyond the FP32 forms' cutoff too). One warp per leaf.
+template <bool CHAINS>
 __global__ void __launch_bounds__(256)
-walk_gather_kernel(const int *__restrict__ counts, const int64_t *__restrict__ row_off, int nleaf,
-                   const int *__restrict__ slab, int slab_cap, int *__restrict__ row_src,
-                   const int *__restrict__ leaf_npart, const LeafMeta *__restrict__ meta, double cscale,
-                   float uout, unsigned long long *__restrict__ pairs, unsigned long long *__restrict__ skipped,
-                   int *__restrict__ status) {
+walk_gather_kernel(const int *__restrict__ len, const int *__restrict__ head, const int64_t *__restrict__ row_off,
+                   int nleaf, const WalkPool pool, int *__restrict__ row_src, const int *__restrict__ leaf_npart,
+                   const LeafMeta *__restrict__ meta, double cscale, float uout,
+                   unsigned long long *__restrict__ pairs, unsigned long long *__restrict__ skipped) {
     const int lane = threadIdx.x & 31;
     const int nw = (int)(((int64_t)gridDim.x * blockDim.x) >> 5);
     unsigned long long my_pairs = 0, my_skip = 0;
-    int bad = 0;
     for (int L = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); L < nleaf; L += nw) {
-        const int n = counts[L];
-        if (n <= 0 || n > slab_cap) continue;  // warp-uniform
+        const int n = len[L];
+        if (n <= 0) continue;  // warp-uniform
         const int64_t base = row_off[L];
-        if (row_off[L + 1] - base != n) {
-            bad = ST_WALK_ROW;
-            continue;
-        }
         const long long np_t = leaf_npart[L];
         LeafMeta mt{};
         if (skipped) mt = meta[L];
-        for (int i = lane; i < n; i += 32) {
-            const int S = slab[(int64_t)L * slab_cap + i];
-            if ((unsigned)S >= (unsigned)nleaf) {
-                bad = ST_WALK_ROW;
-                continue;
+        int chunk = CHAINS ? head[L] : 0;
+        for (int b = 0; b < n; b += kWalkChunk) {
+            const int after = CHAINS && b + kWalkChunk < n ? pool.next[chunk] : 0;
+#pragma unroll
+            for (int h = 0; h < kWalkChunk; h += 32) {
+                const int i = b + h + lane;
+                if (i >= n) continue;
+                int S;
+                if (CHAINS) row_src[base + i] = S = pool.ids[(size_t)chunk * kWalkChunk + h + lane];
+                else S = row_src[base + i];
+                const unsigned long long np = (unsigned long long)(np_t * (long long)leaf_npart[S]);
+                my_pairs += np;
+                if (skipped) {
+                    const LeafMeta ms = meta[S];
+                    float ox, oy, oz;
+                    entry_offset(ms, mt, cscale, ox, oy, oz);
+                    if (entry_u_min(ms, mt, ox, oy, oz) > uout) my_skip += np;
+                }
             }
-            row_src[base + i] = S;
-            const unsigned long long np = (unsigned long long)(np_t * (long long)leaf_npart[S]);
-            my_pairs += np;
-            if (skipped) {
-                const LeafMeta ms = meta[S];
-                float ox, oy, oz;
-                entry_offset(ms, mt, cscale, ox, oy, oz);
-                if (entry_u_min(ms, mt, ox, oy, oz) > uout) my_skip += np;
-            }
+            chunk = after;
         }
     }
 #pragma unroll
@@ -293,7 +498,32 @@ walk_gather_kernel(const int *__restrict__ counts, const int64_t *__restrict__ r
         if (my_pairs) atomicAdd(pairs, my_pairs);
         if (skipped && my_skip) atomicAdd(skipped, my_skip);
     }
-    if (bad) atomicOr(status, bad);
 }
+
+// ------------------------------------------------------------- launching ---
+
+// Enqueues depths [lv, lv + n) of a walk.
+template <int MODE>
+inline cudaError_t walk_depths(cudaStream_t st, const WalkRun &g, int sm_count, int lv, int n) {
+    const int blocks = min(sm_count * 8, (g.nleaf + kWalkWarps - 1) / kWalkWarps);
+    for (int l = lv; l < lv + n; ++l) walk_level_kernel<MODE><<<blocks, kWalkWarps * 32, 0, st>>>(g, l);
+    return cudaGetLastError();
+}
+
+// Depths enqueued before the host looks whether boxes are left: mean splits
+// of clustered particles go about six depths below a balanced tree (26 for
+// 828,182 leaves); an empty depth costs 2 us, another look 20.
+inline int walk_first_depths(int nleaf) {
+    int lg = 0;
+    while (lg < 30 && (1 << lg) < nleaf) ++lg;
+    return lg + 6;
+}
+
+inline size_t walk_pool_bytes(int64_t cap, int chunk) { return (size_t)cap * (size_t)(chunk + 1) * sizeof(int); }
+inline WalkPool walk_pool(void *p, int64_t cap, int chunk) {
+    return WalkPool{(int *)p, (int *)p + (size_t)cap * chunk, (int)cap};
+}
+// Chunks that warps hold without having used them.
+inline int64_t walk_pool_slack(int sm_count) { return (int64_t)sm_count * 8 * kWalkWarps * kWalkGrab; }
 
 }  // namespace p2p
