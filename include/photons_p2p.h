@@ -74,8 +74,9 @@ typedef struct {
     int warps_per_leaf;  /* sink-register mappings: 1, 2 or 4 warps share one sink leaf's
                             row, each taking a contiguous share of its list entries and
                             adding its partial forces with FP64 atomics (the summation
-                            order then varies between runs); 0 = 1. Ignored by the
-                            other mappings */
+                            order then varies between runs); 0: one warp, or in a session
+                            with few leaves four whose sums are kept apart and added in
+                            order (they repeat bit for bit). Ignored by the other mappings */
 } p2p_params;
 
 /* Lane mappings of the FP32 pair kernel. */

@@ -89,7 +89,7 @@ struct p2p_session {
     // device buffers
     DevBuf task_t2, task_s2;  // second buffer pair of pipelined submits
     DevBuf pos, mass, leaf_ip, leaf_np, task_t, task_s, meta, pos4, counts, fill, row_off,
-        row_src, tile_sums, acc, status, queue, pairs, skipped, evaluated, probe;
+        row_src, tile_sums, acc, parts, status, queue, pairs, skipped, evaluated, probe;
     DevBuf keys_a, keys_b, vals_b, hist, hoffs, hsums;  // radix sort of the list
     std::vector<DevBuf> scratch;  // grow-only temporaries of p2p_dtree_build, by request order
     // device walk (p2p_pass_submit_walk): box records, active prefix, boxes of
@@ -224,6 +224,23 @@ int default_stage(const p2p_params &p) {
 // 0.361 ms at four, 0.379 at eight) to 110^3 four are as good or better.
 int default_warps(const p2p_session *s, const p2p_params &p) {
     return p.form == P2P_FORM_PLAIN_FP64 && s->fit64.nfar && s->nleaf <= 16 * s->sm_count ? 8 : 4;
+}
+
+// Shares that a sink leaf's row is cut into (1: none). With few leaves the
+// longest row and not the work decides; the shares' sums lie in arrays of their
+// own and are added in order (two more launches, 24 bytes a particle and
+// share). Sink-register kernel, whole and in four shares: 0.117 and 0.052 ms at
+// 12^3 (512 leaves), 0.166 and 0.136 at 32^3 (3,992), 2.71 and 2.03 at 64^3
+// clustered (19,039), 16.9 and 14.6 at 101^3 with leaves of 64 (30,403); but 2.94
+// and 3.16 at 100^3 (65,513), and short rows lose sooner: 0.48 and 0.62 at 48^3
+// with leaves of 8 (33,048). So up to 900 leaves per particle of the mean leaf.
+// The FP64 kernel's blocks share rows among their warps already: 0.144 and 0.097
+// ms at 512 leaves, 0.379 and 0.407 at 2,046.
+constexpr int kRowParts = 4;
+int row_parts(const p2p_session *s) {
+    const p2p_params &p = s->params;
+    if (p.form == P2P_FORM_PLAIN_FP64) return s->fit64.nfar && s->nleaf <= 1000 ? kRowParts : 1;
+    return sink_regs(p) && p.warps_per_leaf == 0 && (int64_t)s->nleaf * s->nleaf <= 900 * (int64_t)s->npart ? kRowParts : 1;
 }
 
 // Dispatch to the lane mapping's launcher (p2p_pair_*.cu).
@@ -384,6 +401,13 @@ int enqueue_chunk(p2p_session *s, int64_t ntask, const int *d_t, const int *d_s,
 int enqueue_pairs(p2p_session *s, bool timed) {
     CUDA_TRY(cudaMemsetAsync(s->queue.p, 0, sizeof(int), s->stream));
     PairArgs a = make_args(s);
+    const int parts = row_parts(s);
+    const int64_t n3 = 3 * (int64_t)s->npart;
+    if (parts > 1) {
+        a.acc = (double *)s->parts.p;
+        a.leaf_warps = -parts;
+        CUDA_TRY(cudaMemsetAsync(a.acc, 0, sizeof(double) * (size_t)(parts * n3), s->stream));
+    }
     // Inside a stream capture the kernel's events become external event-record
     // nodes of the graph; outside it they are ordinary records.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -391,6 +415,12 @@ int enqueue_pairs(p2p_session *s, bool timed) {
     const unsigned evflags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     if (timed) CUDA_TRY(cudaEventRecordWithFlags(s->ev_k0, s->stream, evflags));
     P2P_TRY(launch_pair(s, a));
+    if (parts > 1 && n3 > 0) {
+        sum_parts_kernel<<<grid_for(n3, 256, s->sm_count * 16), 256, 0, s->stream>>>((const double *)s->parts.p, parts,
+                                                                                    n3, (double *)s->acc.p);
+        CUDA_TRY(cudaGetLastError());
+        launch_count(1);
+    }
     if (timed) CUDA_TRY(cudaEventRecordWithFlags(s->ev_k1, s->stream, evflags));
     s->kernel_timed = timed;
     return P2P_OK;
@@ -405,6 +435,9 @@ int size_pass_buffers(p2p_session *s, int npart, int nleaf, bool host_inputs, bo
         P2P_TRY(ensure(s, s->leaf_np, sizeof(int) * (size_t)nleaf));
     }
     P2P_TRY(ensure(s, s->acc, sizeof(double) * n3));
+    s->nleaf = nleaf;  // (row_parts)
+    s->npart = npart;
+    if (row_parts(s) > 1) P2P_TRY(ensure(s, s->parts, sizeof(double) * n3 * kRowParts));
     P2P_TRY(ensure(s, s->meta, sizeof(LeafMeta) * (size_t)nleaf));
     if (is_fp32_form(s->params.form)) P2P_TRY(ensure(s, s->pos4, sizeof(float4) * (size_t)npart));
     P2P_TRY(ensure(s, s->counts, sizeof(int) * (size_t)nleaf));
@@ -536,7 +569,7 @@ P2P_API int p2p_session_destroy(p2p_session *s) {
     if (s->gexec) cudaGraphExecDestroy(s->gexec);
     DevBuf *bufs[] = {&s->pos, &s->mass, &s->leaf_ip, &s->leaf_np, &s->task_t, &s->task_s,
                       &s->meta, &s->pos4, &s->counts, &s->fill, &s->row_off, &s->row_src,
-                      &s->tile_sums, &s->acc, &s->status, &s->queue, &s->pairs, &s->skipped, &s->evaluated, &s->probe,
+                      &s->tile_sums, &s->acc, &s->parts, &s->status, &s->queue, &s->pairs, &s->skipped, &s->evaluated, &s->probe,
                       &s->keys_a, &s->keys_b, &s->vals_b, &s->hist, &s->hoffs, &s->hsums,
                       &s->task_t2, &s->task_s2, &s->walk_box, &s->walk_active, &s->walk_items, &s->walk_lists[0],
                       &s->walk_lists[1], &s->walk_rows, &s->walk_ctrl};

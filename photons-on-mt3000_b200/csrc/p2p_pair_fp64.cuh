@@ -20,7 +20,8 @@
 //   - the warps of a block share one sink leaf's row, each a contiguous share
 //     of its entries, and their partial sums are added in warp and phase
 //     order: a row takes a quarter of the time at four warps, and the result
-//     repeats bit for bit.
+//     repeats bit for bit; with leaf_warps = -P (few leaves) P blocks share a
+//     row, their sums in P arrays that sum_parts_kernel adds in order.
 // Pairs whose r^2 has the cutoff's high word, and those with r^2 not finite, go
 // through the general arithmetic (plain_factor), so which pairs are inside, and
 // what NaN and infinity give, is decided exactly as there.
@@ -186,18 +187,21 @@ pair_fp64_kernel(const __grid_constant__ PairArgs a, const __grid_constant__ Fit
     const int chunk = cap / 2;
     double *const sums = wbase + 4 * (size_t)cap;  // [component and sink][lane]
     __shared__ int s_item;
+    const int parts = a.leaf_warps < 0 ? -a.leaf_warps : 1;  // blocks sharing a row, each with sums of its own
+    const size_t n3 = 3 * (size_t)a.npart;
     const double *X = a.pos, *Y = a.pos + a.npart, *Z = a.pos + 2 * (size_t)a.npart;
     for (;;) {
         __syncthreads();  // the previous item is read
         if (threadIdx.x == 0) s_item = atomicAdd(a.queue, 1);
         __syncthreads();
         const int item = s_item;
-        if (item >= a.nleaf) break;
-        const int li = item_leaf(a, item, lane);
-        const int64_t r0 = a.row_off[li], r1 = a.row_off[li + 1];
-        if (r0 >= r1) continue;
+        if (item >= a.nleaf * parts) break;
+        const int li = item_leaf(a, item / parts, lane), part = item % parts;
+        const int64_t r0 = a.row_off[li], len = a.row_off[li + 1] - r0;
+        if (len <= 0) continue;
         // this warp's contiguous share of the row's entries
-        const int64_t rb = r0 + (r1 - r0) * w / W, re = r0 + (r1 - r0) * (w + 1) / W;
+        const int64_t shares = (int64_t)parts * W, share = (int64_t)part * W + w;
+        const int64_t rb = r0 + len * share / shares, re = r0 + len * (share + 1) / shares;
         const LeafMeta mt = a.leaf[li];
         for (int s0 = 0; s0 < mt.npart; s0 += 8 * kFp64Sinks) {
             const int ns = min(8 * kFp64Sinks, mt.npart - s0);
@@ -301,7 +305,9 @@ pair_fp64_kernel(const __grid_constant__ PairArgs a, const __grid_constant__ Fit
                     const double *ws = smem_d + ww * wdoubles + 4 * (size_t)cap + row;
                     for (int jj = 0; jj < J; ++jj) v += ws[jj * G];
                 }
-                a.acc[(size_t)c * a.npart + first + sk] += MASSES ? v : v * a.mass_eq;
+                double *o = a.acc + n3 * part + (size_t)c * a.npart + first + sk;
+                v = MASSES ? v : v * a.mass_eq;
+                *o = parts > 1 ? v : *o + v;
             }
             __syncthreads();  // the sums are read before the next slice writes its own
         }

@@ -29,7 +29,9 @@
 //
 // With PairArgs::leaf_warps = W > 1 a sink leaf is W work items, each a
 // contiguous share of the row's list entries, whose partial forces are added
-// with FP64 atomics (a long row is spread over W warps).
+// with FP64 atomics (a long row is spread over W warps). With leaf_warps = -W the
+// shares go to W arrays of their own (acc: W times 3 npart, zero) instead, which
+// sum_parts_kernel adds in order: the same spread, sums that repeat bit for bit.
 //
 // Band pairs (FP32 u within the band around x_cut^2) are re-decided from FP64
 // positions by the lane that met them (band_pair), as in the other packed
@@ -240,7 +242,7 @@ pair_sreg_kernel(const __grid_constant__ PairArgs a, const int cap) {
     const unsigned lanes_below = (1u << lane) - 1u;
     unsigned long long evaluated = 0;  // pair interactions of staged sources with real sinks
     constexpr int SLICE = 8 * SPL;     // sinks of a slice: G <= 8 groups, J >= 4 phases
-    const int W = a.leaf_warps > 1 ? a.leaf_warps : 1;  // warps sharing a row (work items per leaf)
+    const int W = abs(a.leaf_warps) > 1 ? abs(a.leaf_warps) : 1;  // warps sharing a row (work items per leaf)
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(a.queue, 1);
@@ -428,7 +430,12 @@ pair_sreg_kernel(const __grid_constant__ PairArgs a, const int cap) {
                 const int idx = first + sk;
                 double *o = a.acc;
                 const size_t n = (size_t)a.npart;
-                if (W > 1) {  // other warps add their shares of the row to the same sinks
+                if (a.leaf_warps < 0) {  // this share's own sums
+                    o += 3 * n * (size_t)(item % W);
+                    o[idx] = (double)sx * a.out_scale;
+                    o[n + idx] = (double)sy * a.out_scale;
+                    o[2 * n + idx] = (double)sz * a.out_scale;
+                } else if (W > 1) {  // other warps add their shares of the row to the same sinks
                     atomicAdd(o + idx, (double)sx * a.out_scale);
                     atomicAdd(o + n + idx, (double)sy * a.out_scale);
                     atomicAdd(o + 2 * n + idx, (double)sz * a.out_scale);

@@ -584,6 +584,18 @@ __global__ void scan_add_kernel(int64_t *__restrict__ out, int n,
     if (i < n) out[i] += tile_sums[i / kScanTile];
 }
 
+// ---------------------------------------------------- sums of shared rows ---
+
+// acc += the `parts` arrays of n sums each, in order.
+__global__ void __launch_bounds__(256)
+sum_parts_kernel(const double *__restrict__ part, int parts, int64_t n, double *__restrict__ acc) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        double v = part[i];
+        for (int p = 1; p < parts; ++p) v += part[p * n + i];
+        acc[i] += v;
+    }
+}
+
 // --------------------------------------------------------------- probes ---
 
 // FP32 FFMA throughput: 8 independent dependent chains per thread.
