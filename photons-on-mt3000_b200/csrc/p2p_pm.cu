@@ -59,22 +59,20 @@ __device__ __forceinline__ int wrap(int i, int n) {
     return i < 0 ? i + n : i;
 }
 
+__device__ __forceinline__ int wrap_near(int i, int n) {
+    return i < 0 ? i + n : (i >= n ? i - n : i);
+}
+
 // Cell, neighbour cell and the neighbour's weight on one axis
 // (src/partmesh.c:99-143): i = (int)(x norm), w = (x - (i + 1/2) delta) norm,
-// the neighbour on the side of w, weight |w|.
+// the neighbour on the side of w, weight |w|. Positions inside the box take no
+// division to wrap.
 __device__ __forceinline__ void cic_axis(double x, double norm, double delta, int n, int &c, int &nb, double &w) {
     const int i = (int)__dmul_rn(x, norm);
-    double d = __dmul_rn(__dsub_rn(x, __dmul_rn(__dadd_rn((double)i, 0.5), delta)), norm);
-    int ii;
-    if (d > 0) {
-        ii = i + 1;
-    } else {
-        d = -d;
-        ii = i - 1;
-    }
-    c = wrap(i, n);
-    nb = wrap(ii, n);
-    w = d;
+    const double d = __dmul_rn(__dsub_rn(x, __dmul_rn(__dadd_rn((double)i, 0.5), delta)), norm);
+    c = (unsigned)i < (unsigned)n ? i : wrap(i, n);
+    nb = wrap_near(d > 0 ? c + 1 : c - 1, n);
+    w = d > 0 ? d : -d;
 }
 
 constexpr unsigned kFull = 0xffffffffu;
@@ -144,8 +142,19 @@ __global__ void pm_green_kernel(cufftDoubleComplex *__restrict__ spec, const dou
     spec[q].y *= g;
 }
 
-__device__ __forceinline__ int wrap_near(int i, int n) {
-    return i < 0 ? i + n : (i >= n ? i - n : i);
+// A cell's gradient as one 32-byte access (a sector): half the loads and tag
+// lookups of two 16-byte ones, which bound the interpolation.
+__device__ __forceinline__ double4 load_cell(const double4 *p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+        : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ void store_cell(double4 *p, double x, double y, double z) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "d"(x), "d"(y), "d"(z),
+                 "d"(0.0)
+                 : "memory");
 }
 
 // The 4-point difference along one axis: row = the cell's offset without
@@ -167,12 +176,10 @@ __global__ void __launch_bounds__(256) pm_gradient_kernel(const double *__restri
     if (t >= n * n) return;
     const int i = blockIdx.y, j = t / n, k = t - j * n;
     const size_t sx = (size_t)n * n, sy = n;
-    double2 *out = reinterpret_cast<double2 *>(grad + (size_t)i * sx + t);
     const double gx = diff4(phi, (size_t)j * sy + k, i, n, sx, f1h, f2h);
     const double gy = diff4(phi, (size_t)i * sx + k, j, n, sy, f1h, f2h);
     const double gz = diff4(phi, (size_t)i * sx + (size_t)j * sy, k, n, 1, f1h, f2h);
-    out[0] = make_double2(gx, gy);
-    out[1] = make_double2(gz, 0.0);
+    store_cell(grad + (size_t)i * sx + t, gx, gy, gz);
 }
 
 __global__ void __launch_bounds__(256) pm_interp_kernel(const double *__restrict__ pos, const int *__restrict__ tag,
@@ -191,11 +198,10 @@ __global__ void __launch_bounds__(256) pm_interp_kernel(const double *__restrict
                 const double wx = (q & 1) ? w[0] : 1.0 - w[0], wy = (q & 2) ? w[1] : 1.0 - w[1],
                              wz = (q & 4) ? w[2] : 1.0 - w[2];
                 const double wt = __dmul_rn(__dmul_rn(wx, wy), wz);
-                const double2 *g = reinterpret_cast<const double2 *>(grad + ((size_t)ix * n + iy) * n + iz);
-                const double2 gxy = __ldg(g), gz = __ldg(g + 1);
-                out[0] = __dadd_rn(out[0], __dmul_rn(wt, gxy.x));
-                out[1] = __dadd_rn(out[1], __dmul_rn(wt, gxy.y));
-                out[2] = __dadd_rn(out[2], __dmul_rn(wt, gz.x));
+                const double4 g = load_cell(grad + ((size_t)ix * n + iy) * n + iz);
+                out[0] = __dadd_rn(out[0], __dmul_rn(wt, g.x));
+                out[1] = __dadd_rn(out[1], __dmul_rn(wt, g.y));
+                out[2] = __dadd_rn(out[2], __dmul_rn(wt, g.z));
             }
         }
         acc[p] = out[0];
