@@ -862,7 +862,7 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     g.cutoff = cutoff;
     g.open_angle = open_angle;
     g.cut2 = (float)(cutoff * cutoff);
-    g.th2 = (float)(open_angle * open_angle);
+    g.th2 = walk_th2(open_angle);
     g.out_head = heads;
     g.out_len = counts;
     g.row_off = row_off;

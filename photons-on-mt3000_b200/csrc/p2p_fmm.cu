@@ -540,7 +540,7 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
         g.cutoff = cutoff;
         g.open_angle = open_angle;
         g.cut2 = (float)(cutoff * cutoff);
-        g.th2 = (float)(open_angle * open_angle);
+        g.th2 = walk_th2(open_angle);
         g.out_head = head;
         g.out_len = len;
         const size_t nbox = 2 * ((size_t)std::max(nleaf, nnode) + 1);

@@ -32,6 +32,8 @@
 // code.
 #pragma once
 
+#include <algorithm>
+
 #include "p2p_device_common.cuh"
 #include "p2p_walk_test.h"
 
@@ -355,7 +357,9 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8) walk_level_kernel(const Wa
                 nc = (v0 ? 1 : 0) + (v1 ? 1 : 0);
             }
             const unsigned open = __ballot_sync(kFull, cls == 2);
-            const unsigned ready = open ? (open & (0u - open)) - 1u : kFull;  // lanes before the first opened box
+            // written out: the lanes before the first opened box (M2L lists need no
+            // order, only the same one on every run)
+            const unsigned ready = M2L || !open ? kFull : (open & (0u - open)) - 1u;
             const unsigned done = __ballot_sync(kFull, cls == 1);
             if (M2L) {
                 const unsigned tm = __ballot_sync(kFull, task);
@@ -519,6 +523,9 @@ inline int walk_first_depths(int nleaf) {
     return lg + 6;
 }
 
+inline float walk_th2(double open_angle) {
+    return open_angle > 0.0 ? std::max((float)(open_angle * open_angle), 1.1754944e-38f) : 0.f;
+}
 inline size_t walk_pool_bytes(int64_t cap, int chunk) { return (size_t)cap * (size_t)(chunk + 1) * sizeof(int); }
 inline WalkPool walk_pool(void *p, int64_t cap, int chunk) {
     return WalkPool{(int *)p, (int *)p + (size_t)cap * chunk, (int)cap};

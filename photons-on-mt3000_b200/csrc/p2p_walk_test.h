@@ -38,38 +38,46 @@ enum { WALK_DROP = -1, WALK_OPEN_B = 0, WALK_ACCEPT = 1, WALK_OPEN_A = 2, WALK_U
 // sum and product again, so one axis's gap |dist| - width is off by less than
 // slack = 2^-21 (|ca| + |cb| + wa + wb); squares and sums of bounds, and the two
 // constants, by less than 1e-6 of themselves. A gap bounded to be at most zero
-// is zero in the exact test too. NaN decides nothing.
+// is zero in the exact test too. NaN decides nothing. An open angle whose square
+// vanishes in FP32 is not 0: th2 is then passed as the smallest normal number.
 P2P_HD int walk_bound(const WalkBox32 &a, const WalkBox32 &b, bool a_node, bool b_node, float cut2, float th2) {
     constexpr float kSlack = 4.76837158e-7f, kUp = 1.0f + 2.0e-6f, kDown = 1.0f - 2.0e-6f;
-    float lo2 = 0.f, hi2 = 0.f, lo1 = 0.f, d2lo = 0.f, d2hi = 0.f, wlo = 0.f, whi = 0.f, sa = 0.f, sb = 0.f;
+    float dist[3], w[3], slack[3], lo2 = 0.f, hi2 = 0.f, lo1 = 0.f;
 #ifdef __CUDACC__
 #pragma unroll
 #endif
     for (int d = 0; d < 3; ++d) {
-        const float dist = fabsf(a.c[d] - b.c[d]), w = (a.w[d] + b.w[d]) * 0.5f;
-        const float slack = kSlack * (fabsf(a.c[d]) + fabsf(b.c[d]) + a.w[d] + b.w[d]);
-        const float gap = dist - w;
-        const float lo = fmaxf(gap - slack, 0.f), hi = fmaxf(gap + slack, 0.f);
+        dist[d] = fabsf(a.c[d] - b.c[d]);
+        w[d] = (a.w[d] + b.w[d]) * 0.5f;
+        slack[d] = kSlack * (fabsf(a.c[d]) + fabsf(b.c[d]) + 2.0f * w[d]);
+        const float gap = dist[d] - w[d];
+        const float lo = fmaxf(gap - slack[d], 0.f), hi = fmaxf(gap + slack[d], 0.f);
         lo1 += lo;
         lo2 += lo * lo;
         hi2 += hi * hi;
-        const float dl = fmaxf(dist - slack, 0.f), dh = dist + slack;
-        d2lo += dl * dl;
-        d2hi += dh * dh;
-        wlo = fmaxf(wlo, w - slack);
-        whi = fmaxf(whi, w + slack);
-        sa += a.w[d];
-        sb += b.w[d];
     }
     if (lo2 * kDown > cut2 * kUp && lo1 > 1.0e-14f) return WALK_DROP;
     if (!(hi2 * kUp < cut2 * kDown)) return WALK_UNDECIDED;
-    // not dropped: accepted or opened
-    const float t_lo = 2.f * wlo, t_hi = 2.f * whi;
-    if (t_hi * t_hi * kUp < th2 * d2lo * kDown && lo1 > 1.0e-14f) return WALK_ACCEPT;
-    const float most = th2 * d2hi * kUp;
-    if (!(t_lo * t_lo * kDown >= most) || !(most < 3.0e38f)) return WALK_UNDECIDED;  // (an overflow decides nothing)
+    // not dropped: accepted (never at open angle 0) or opened
+    if (th2 > 0.f) {
+        float d2lo = 0.f, d2hi = 0.f, wlo = 0.f, whi = 0.f;
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+        for (int d = 0; d < 3; ++d) {
+            const float dl = fmaxf(dist[d] - slack[d], 0.f), dh = dist[d] + slack[d];
+            d2lo += dl * dl;
+            d2hi += dh * dh;
+            wlo = fmaxf(wlo, w[d] - slack[d]);
+            whi = fmaxf(whi, w[d] + slack[d]);
+        }
+        const float t_lo = 2.f * wlo, t_hi = 2.f * whi, most = th2 * d2hi * kUp;
+        if (t_hi * t_hi * kUp < th2 * d2lo * kDown && lo1 > 1.0e-14f) return WALK_ACCEPT;
+        if (!(t_lo * t_lo * kDown >= most) || !(most < 3.0e38f)) return WALK_UNDECIDED;  // (an overflow decides nothing)
+    }
     if (!a_node) return WALK_OPEN_B;
     if (!b_node) return WALK_OPEN_A;
+    const float sa = a.w[0] + a.w[1] + a.w[2], sb = b.w[0] + b.w[1] + b.w[2];
     if (sa * kDown > sb * kUp) return WALK_OPEN_A;
     if (sa * kUp < sb * kDown) return WALK_OPEN_B;
     return WALK_UNDECIDED;
