@@ -12,7 +12,6 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
-#include <vector>
 
 #include "photons_p2p.h"
 #include "p2p_host_shared.h"
@@ -192,118 +191,61 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
     tree_root_box_kernel<<<1, 96, 0, st>>>(blo, bhi, init_blocks, boxsize, R, 0);
     launches += 2;
 
-    // ---- nodes above kTreeSmall particles, level by level (host-driven) ----
-    std::vector<int> h_son, h_depth, h_lipart, h_lnpart;  // records made on the host
-    std::vector<TreeTask> tasks;
-    std::vector<TreeSeg> segs;
-    int nnode_h = 0, nleaf_h = 0, maxdepth = 0;
-    if (n <= kTreeSmall) {
-        tasks.push_back(TreeTask{0, n, 0, 0, -1, 0});  // the whole tree in one block
-    } else {
-        h_son.assign(2, -1);
-        h_depth.assign(1, 0);
-        nnode_h = 1;
-        segs.push_back(TreeSeg{0, n, 0, 0, 0.0, 0, 0});
-    }
-    TreeSeg *d_segs = nullptr;
-    int *d_tile_seg = nullptr, *d_tile_off = nullptr, *d_tile_pre = nullptr, *d_tile_small = nullptr;
-    size_t seg_cap = 0, tile_cap = 0;
-    int level = 0;
-    while (!segs.empty()) {
-        if (++level > 4096) return report_error(P2P_ERR_CAPACITY, "tree build: more than 4096 levels above 2048 particles");
-        const int nseg = (int)segs.size();
-        std::vector<int> tile_seg, tile_off;
-        for (int g = 0; g < nseg; ++g)
-            for (int o = 0; o < segs[g].length; o += kTreeTile) {
-                tile_seg.push_back(g);
-                tile_off.push_back(o);
-            }
-        const int ntile = (int)tile_seg.size();
-        if ((size_t)nseg > seg_cap) {
-            if (!S.get(&d_segs, 2 * (size_t)nseg)) return report_error(P2P_ERR_NOMEM, "tree build: allocation");
-            seg_cap = 2 * (size_t)nseg;
+    // ---- nodes above kTreeSmall particles, level by level; the host reads the
+    // counts once the levels that such a tree has are queued (an empty level
+    // costs its launches, a look at the counts about as much as two levels) ----
+    const int seg_cap = n / (kTreeSmall + 1) + 1, task_cap = (int)(n / ((int64_t)maxleaf + 1)) + 1;
+    const int tile_cap = (n + kTreeTile - 1) / kTreeTile + seg_cap;
+    TreeSeg *segs[2] = {nullptr, nullptr};
+    int *tile_seg[2] = {nullptr, nullptr}, *tile_off[2] = {nullptr, nullptr}, *tile_small = nullptr, *tile_pre = nullptr;
+    TreeTask *tasks = nullptr;
+    TreeLevels *lv = nullptr;
+    for (int k = 0; k < 2; ++k)
+        ok = ok && S.get(&segs[k], seg_cap) && S.get(&tile_seg[k], tile_cap) && S.get(&tile_off[k], tile_cap);
+    ok = ok && S.get(&tile_small, tile_cap) && S.get(&tile_pre, tile_cap) && S.get(&tasks, task_cap) && S.get(&lv, 1);
+    if (!ok) return report_error(P2P_ERR_NOMEM, "tree build: device allocation failed");
+    TREE_CUDA(cudaMemsetAsync(lv, 0, sizeof(TreeLevels), st));
+    TREE_CUDA(cudaMemsetAsync(R.counters, 0, 4 * sizeof(int), st));
+    tree_first_level_kernel<<<grid((n + kTreeTile - 1) / kTreeTile, kTreeThreads, INT32_MAX), kTreeThreads, 0, st>>>(
+        n, segs[0], tile_seg[0], tile_off[0], tasks, lv, R);
+    launches += 1;
+    int hc[4] = {0, 0, 0, 0}, ntask = 0, left = 0, level = 0;
+    int batch = 0;
+    while (n > kTreeSmall && ((int64_t)kTreeSmall << batch) < n) ++batch;
+    for (batch = n > kTreeSmall ? batch + 2 : 0;; batch = 2) {
+        for (const int end = std::min(level + batch, kTreeLevels); level < end; ++level) {
+            const int a = level & 1, b = a ^ 1;
+            const int nseg = level < 30 ? std::min(1 << level, seg_cap) : seg_cap;
+            const int ntile = std::min(n / kTreeTile + nseg, tile_cap);
+            tree_seg_mean_kernel<<<nseg, kTreeThreads, 0, st>>>(segs[a], lv, level, P, R);
+            tree_seg_chain_kernel<<<(nseg + 3) / 4, 128, 0, st>>>(segs[a], lv, level, P, R);
+            tree_tile_count_kernel<<<ntile, kTreeThreads, 0, st>>>(segs[a], lv, level, tile_seg[a], tile_off[a], P,
+                                                                   tile_small);
+            tree_level_kernel<<<1, kTreeLevelThreads, 0, st>>>(segs[a], tile_seg[a], tile_small, tile_pre, segs[b],
+                                                              tile_seg[b], tile_off[b], tasks, lv, level, maxleaf, seg_cap,
+                                                              task_cap, R);
+            tree_tile_map_kernel<<<ntile, kTreeThreads, 0, st>>>(segs[a], lv, level, tile_seg[a], tile_off[a], tile_pre, P,
+                                                                 map);
+            tree_tile_swap_kernel<<<ntile, kTreeThreads, 0, st>>>(segs[a], lv, level, tile_seg[a], tile_off[a], tile_pre,
+                                                                  P, map);
+            launches += 6;
         }
-        if ((size_t)ntile > tile_cap) {
-            if (!(S.get(&d_tile_seg, 2 * (size_t)ntile) && S.get(&d_tile_off, 2 * (size_t)ntile) &&
-                  S.get(&d_tile_pre, 2 * (size_t)ntile) && S.get(&d_tile_small, 2 * (size_t)ntile)))
-                return report_error(P2P_ERR_NOMEM, "tree build: allocation");
-            tile_cap = 2 * (size_t)ntile;
-        }
-        TREE_CUDA(cudaMemcpyAsync(d_segs, segs.data(), sizeof(TreeSeg) * nseg, cudaMemcpyHostToDevice, st));
-        TREE_CUDA(cudaMemcpyAsync(d_tile_seg, tile_seg.data(), sizeof(int) * ntile, cudaMemcpyHostToDevice, st));
-        TREE_CUDA(cudaMemcpyAsync(d_tile_off, tile_off.data(), sizeof(int) * ntile, cudaMemcpyHostToDevice, st));
-        const int64_t nchain = std::count_if(segs.begin(), segs.end(),
-                                             [&](const TreeSeg &g) { return tree_takes_chain(g.length, nseg); });
-        if (nchain < nseg) tree_seg_mean_kernel<<<nseg, kTreeThreads, 0, st>>>(d_segs, nseg, P, R);
-        if (nchain > 0) tree_seg_chain_kernel<<<(nseg + 3) / 4, 128, 0, st>>>(d_segs, nseg, P, R);
-        launches += (nchain < nseg ? 1 : 0) + (nchain > 0 ? 1 : 0) - 1;
-        tree_tile_count_kernel<<<ntile, kTreeThreads, 0, st>>>(d_segs, d_tile_seg, d_tile_off, P, d_tile_small);
-        launches += 2;
-        std::vector<int> tsmall(ntile), tpre(ntile);
-        TREE_CUDA(cudaMemcpyAsync(tsmall.data(), d_tile_small, sizeof(int) * ntile, cudaMemcpyDeviceToHost, st));
-        TREE_CUDA(cudaMemcpyAsync(segs.data(), d_segs, sizeof(TreeSeg) * nseg, cudaMemcpyDeviceToHost, st));  // means
-        TREE_CUDA(cudaStreamSynchronize(st));
-        for (auto &g : segs) g.nsmall = 0;
-        for (int t = 0; t < ntile; ++t) {
-            tpre[t] = segs[tile_seg[t]].nsmall;
-            segs[tile_seg[t]].nsmall += tsmall[t];
-        }
-        for (auto &g : segs) g.nbig = g.length - g.nsmall;
-        TREE_CUDA(cudaMemcpyAsync(d_segs, segs.data(), sizeof(TreeSeg) * nseg, cudaMemcpyHostToDevice, st));
-        TREE_CUDA(cudaMemcpyAsync(d_tile_pre, tpre.data(), sizeof(int) * ntile, cudaMemcpyHostToDevice, st));
-        tree_tile_map_kernel<<<ntile, kTreeThreads, 0, st>>>(d_segs, d_tile_seg, d_tile_off, d_tile_pre, P, map);
-        tree_tile_swap_kernel<<<ntile, kTreeThreads, 0, st>>>(d_segs, d_tile_seg, d_tile_off, d_tile_pre, P, map);
-        launches += 2;
         TREE_CUDA(cudaGetLastError());
-        // children: leaves, subtrees for one block, or next level's nodes
-        std::vector<TreeSeg> next;
-        for (const TreeSeg &g : segs) {
-            const int left = g.nbig == 0 ? g.length - 1 : g.nsmall;
-            const int np[2] = {left, g.length - left};
-            const int ip[2] = {g.ipart, g.ipart + left};
-            const int depth = h_depth[g.node] + 1;
-            const int axis = (g.axis + 1) % 3;
-            for (int c = 0; c < 2; ++c) {
-                if (np[c] <= maxleaf) {
-                    h_lipart.push_back(ip[c]);
-                    h_lnpart.push_back(np[c]);
-                    h_son[2 * g.node + c] = 2 * nleaf_h++;
-                } else if (np[c] <= kTreeSmall) {
-                    tasks.push_back(TreeTask{ip[c], np[c], axis, depth, g.node, c});
-                } else {
-                    const int k = nnode_h++;
-                    h_son.push_back(-1);
-                    h_son.push_back(-1);
-                    h_depth.push_back(depth);
-                    maxdepth = std::max(maxdepth, depth);
-                    h_son[2 * g.node + c] = 2 * k + 1;
-                    next.push_back(TreeSeg{ip[c], np[c], axis, k, 0.0, 0, 0});
-                }
-            }
-        }
-        segs.swap(next);
+        TREE_CUDA(cudaMemcpyAsync(&left, &lv->nseg[level], sizeof(int), cudaMemcpyDeviceToHost, st));
+        TREE_CUDA(cudaMemcpyAsync(&ntask, &lv->ntask, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TREE_CUDA(cudaMemcpyAsync(hc, R.counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
+        TREE_CUDA(cudaStreamSynchronize(st));
+        if (hc[2] & (TB_NODE_CAP | TB_LEAF_CAP)) return report_error(P2P_ERR_CAPACITY, "tree build: node capacity");
+        if (left == 0) break;
+        if (level == kTreeLevels)
+            return report_error(P2P_ERR_CAPACITY, "tree build: more than 4096 levels above 2048 particles");
     }
-    if (nnode_h > cap || nleaf_h > cap) return report_error(P2P_ERR_CAPACITY, "tree build: node capacity");
-    // host-made records to the device, then the counters for the blocks' atomics
-    if (nnode_h) {
-        TREE_CUDA(cudaMemcpyAsync(R.son, h_son.data(), sizeof(int) * 2 * nnode_h, cudaMemcpyHostToDevice, st));
-        TREE_CUDA(cudaMemcpyAsync(R.depth, h_depth.data(), sizeof(int) * nnode_h, cudaMemcpyHostToDevice, st));
-    }
-    if (nleaf_h) {
-        TREE_CUDA(cudaMemcpyAsync(R.lipart, h_lipart.data(), sizeof(int) * nleaf_h, cudaMemcpyHostToDevice, st));
-        TREE_CUDA(cudaMemcpyAsync(R.lnpart, h_lnpart.data(), sizeof(int) * nleaf_h, cudaMemcpyHostToDevice, st));
-    }
-    int hc[4] = {nnode_h, nleaf_h, 0, maxdepth};
-    TREE_CUDA(cudaMemcpyAsync(R.counters, hc, sizeof(hc), cudaMemcpyHostToDevice, st));
 
     // ---- subtrees of at most kTreeSmall particles, one block each ----
-    if (!tasks.empty()) {
-        TreeTask *d_tasks = nullptr;
-        if (!S.get(&d_tasks, tasks.size())) return report_error(P2P_ERR_NOMEM, "tree build: allocation");
-        TREE_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(TreeTask) * tasks.size(), cudaMemcpyHostToDevice, st));
+    if (ntask > 0) {
         TREE_CUDA(cudaFuncSetAttribute(tree_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kTreeSmallSmem));
-        tree_small_kernel<<<(int)tasks.size(), kTreeSmallThreads, kTreeSmallSmem, st>>>(d_tasks, P, R, maxleaf);
+        tree_small_kernel<<<ntask, kTreeSmallThreads, kTreeSmallSmem, st>>>(tasks, P, R, maxleaf);
         launches += 1;
         TREE_CUDA(cudaGetLastError());
     }
@@ -312,7 +254,7 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
     if (hc[2] & (TB_NODE_CAP | TB_LEAF_CAP))
         return report_error(P2P_ERR_CAPACITY, "tree build: more nodes or leaves than the build's capacity");
     const int nnode = hc[0], nleaf = hc[1];
-    maxdepth = hc[3];
+    const int maxdepth = hc[3];
 
     // ---- pre-order numbering and boxes, by depth ----
     const int gn = grid(nnode, 256, 4096);

@@ -12,8 +12,8 @@
 // nS particles, or n - 1 when none lies above the mean; a node of two
 // particles splits at their midpoint, swapping them when the first is above
 // the second. Nodes are split level by level while they hold more than
-// kTreeSmall particles (the mean by one thread, the partition by tiles of
-// the node's slots); smaller subtrees are built whole by one block each in
+// kTreeSmall particles (the partition by tiles of the node's slots, a level's
+// children by one block, with no host between); smaller subtrees are built whole by one block each in
 // shared memory. Nodes and leaves get build-order ids as they are made; the
 // pre-order ids of the reference (son[0]'s subtree first, leaves numbered
 // apart from nodes) and the node boxes follow from two passes over depths.
@@ -233,6 +233,15 @@ struct TreeSeg {
     int ipart, length, axis, node;
     double mean;
     int nsmall, nbig;
+    int tile0, before;  // its first tile; slots not above their means in the tiles before that
+};
+
+// Levels split level-wide: the counts of each, made by tree_level_kernel for the
+// next one, so the levels are queued without the host reading between them.
+constexpr int kTreeLevels = 4096;
+struct TreeLevels {
+    int nseg[kTreeLevels + 1], ntile[kTreeLevels + 1];
+    int ntask;  // subtrees for one block each
 };
 
 // Segments whose chain of additions is made as it is, one warp per segment:
@@ -245,11 +254,12 @@ __host__ __device__ __forceinline__ bool tree_takes_chain(int length, int nseg) 
     return length <= kMeanChainMax || (nseg >= kMeanChainSegs && length <= 100000);
 }
 
-__global__ void __launch_bounds__(128) tree_seg_chain_kernel(TreeSeg *segs, int nseg, TreeParts P, TreeRec R) {
+__global__ void __launch_bounds__(128) tree_seg_chain_kernel(TreeSeg *segs, const TreeLevels *lv, int level,
+                                                             TreeParts P, TreeRec R) {
     constexpr int kBatch = 256;
     __shared__ double batch[4][kBatch];
     const int lane = threadIdx.x & 31;
-    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nseg = lv->nseg[level];
     if (q >= nseg) return;
     const TreeSeg g = segs[q];
     if (!tree_takes_chain(g.length, nseg)) return;
@@ -285,11 +295,14 @@ __global__ void __launch_bounds__(128) tree_seg_chain_kernel(TreeSeg *segs, int 
 // moves stay good while S stays in the binade they were found in.
 constexpr int kMeanPerLane = 16;
 constexpr int kMeanGroup = 32 * kMeanPerLane;
-__global__ void __launch_bounds__(kTreeThreads, 3) tree_seg_mean_kernel(TreeSeg *segs, int nseg, TreeParts P, TreeRec R) {
+__global__ void __launch_bounds__(kTreeThreads, 3) tree_seg_mean_kernel(TreeSeg *segs, const TreeLevels *lv,
+                                                                         int level, TreeParts P, TreeRec R) {
     constexpr int kWarps = kTreeThreads / 32;
     __shared__ MeanMoves groups[kWarps];
     __shared__ double s_sum;
     __shared__ double order[kMeanGroup];  // the group that is worked out
+    const int nseg = lv->nseg[level];
+    if ((int)blockIdx.x >= nseg) return;
     const TreeSeg g = segs[blockIdx.x];
     if (tree_takes_chain(g.length, nseg)) return;
     const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
@@ -387,9 +400,11 @@ __device__ __forceinline__ TileFlags tree_tile_flags(const double *c, double mea
 
 // Counts the tile's slots not above the mean.
 __global__ void __launch_bounds__(kTreeThreads)
-tree_tile_count_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ tile_seg,
-                       const int *__restrict__ tile_off, TreeParts P, int *__restrict__ tile_small) {
+tree_tile_count_kernel(const TreeSeg *__restrict__ segs, const TreeLevels *__restrict__ lv, int level,
+                       const int *__restrict__ tile_seg, const int *__restrict__ tile_off, TreeParts P,
+                       int *__restrict__ tile_small) {
     __shared__ int warp_tot[kTreeThreads / 32];
+    if ((int)blockIdx.x >= lv->ntile[level]) return;
     const TreeSeg g = segs[tile_seg[blockIdx.x]];
     const int off = tile_off[blockIdx.x];
     const double *c = (g.axis == 0 ? P.x : (g.axis == 1 ? P.y : P.z)) + g.ipart;
@@ -402,10 +417,11 @@ tree_tile_count_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__
 // slots [nsmall, length) of the segment (relative slots). tile_pre[t] = slots
 // not above the mean before tile t within its segment.
 __global__ void __launch_bounds__(kTreeThreads)
-tree_tile_map_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ tile_seg,
-                     const int *__restrict__ tile_off, const int *__restrict__ tile_pre, TreeParts P,
-                     int *__restrict__ map) {
+tree_tile_map_kernel(const TreeSeg *__restrict__ segs, const TreeLevels *__restrict__ lv, int level,
+                     const int *__restrict__ tile_seg, const int *__restrict__ tile_off,
+                     const int *__restrict__ tile_pre, TreeParts P, int *__restrict__ map) {
     __shared__ int warp_tot[kTreeThreads / 32];
+    if ((int)blockIdx.x >= lv->ntile[level]) return;
     const TreeSeg g = segs[tile_seg[blockIdx.x]];
     const int off = tile_off[blockIdx.x];
     const int end = min(g.length, off + kTreeTile);
@@ -429,10 +445,11 @@ tree_tile_map_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ t
 // with the slot map[nsmall + q]. Only the thread of slot r touches r and its
 // partner; flags are read in [0, nsmall) only, which no other thread writes.
 __global__ void __launch_bounds__(kTreeThreads)
-tree_tile_swap_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ tile_seg,
-                      const int *__restrict__ tile_off, const int *__restrict__ tile_pre, TreeParts P,
-                      const int *__restrict__ map) {
+tree_tile_swap_kernel(const TreeSeg *__restrict__ segs, const TreeLevels *__restrict__ lv, int level,
+                      const int *__restrict__ tile_seg, const int *__restrict__ tile_off,
+                      const int *__restrict__ tile_pre, TreeParts P, const int *__restrict__ map) {
     __shared__ int warp_tot[kTreeThreads / 32];
+    if ((int)blockIdx.x >= lv->ntile[level]) return;
     const TreeSeg g = segs[tile_seg[blockIdx.x]];
     const int off = tile_off[blockIdx.x];
     const int end = min(min(g.length, off + kTreeTile), g.nsmall);
@@ -478,6 +495,147 @@ tree_tile_swap_kernel(const TreeSeg *__restrict__ segs, const int *__restrict__ 
 struct TreeTask {
     int ipart, length, axis, depth, parent, side;
 };
+
+// The root as the first level (one segment over all tiles), or as the one
+// subtree of a tree small enough for a block.
+__global__ void __launch_bounds__(kTreeThreads)
+tree_first_level_kernel(int n, TreeSeg *segs, int *__restrict__ tile_seg, int *__restrict__ tile_off, TreeTask *tasks,
+                        TreeLevels *lv, TreeRec R) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = (n + kTreeTile - 1) / kTreeTile;
+    if (n > kTreeSmall && t < nt) {
+        tile_seg[t] = 0;
+        tile_off[t] = t * kTreeTile;
+    }
+    if (t > 0) return;
+    if (n <= kTreeSmall) {
+        tasks[0] = TreeTask{0, n, 0, 0, -1, 0};
+        lv->ntask = 1;
+        return;
+    }
+    segs[0] = TreeSeg{0, n, 0, 0, 0.0, 0, 0, 0, 0};
+    lv->nseg[0] = 1;
+    lv->ntile[0] = nt;
+    R.depth[0] = 0;
+    R.counters[0] = 1;
+}
+
+constexpr int kTreeLevelThreads = 1024;
+
+// Exclusive prefix of v over a block of kTreeLevelThreads, and the total.
+__device__ __forceinline__ int tree_level_scan(int v, int *warp_tot, int &total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    if (lane == 31) warp_tot[w] = x;
+    __syncthreads();
+    int t = warp_tot[lane];  // 32 warps
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, t, off);
+        if (lane >= off) t += y;
+    }
+    total = __shfl_sync(0xffffffffu, t, 31);
+    const int before = w > 0 ? __shfl_sync(0xffffffffu, t, w - 1) : 0;
+    __syncthreads();  // warp_tot is rewritten by the next scan
+    return before + x - v;
+}
+
+// After a level's tile counts, one block: the counts before each tile within its
+// segment, every segment's split, its children (leaves, subtrees for one block,
+// or the next level's segments and tiles) and the next level's counts.
+__global__ void __launch_bounds__(kTreeLevelThreads)
+tree_level_kernel(TreeSeg *segs, const int *__restrict__ tile_seg, const int *__restrict__ tile_small, int *tile_pre,
+                  TreeSeg *next, int *__restrict__ next_tile_seg, int *__restrict__ next_tile_off, TreeTask *tasks,
+                  TreeLevels *lv, int level, int maxleaf, int seg_cap, int task_cap, TreeRec R) {
+    __shared__ int warp_tot[32];
+    __shared__ int s_next, s_task, s_node, s_leaf;
+    const int nseg = lv->nseg[level], ntile = lv->ntile[level];
+    if (nseg == 0) return;
+    if (threadIdx.x == 0) {
+        s_next = 0;
+        s_task = lv->ntask;
+        s_node = R.counters[0];
+        s_leaf = R.counters[1];
+    }
+    int carry = 0;
+    for (int b = 0; b < ntile; b += kTreeLevelThreads) {
+        const int t = b + threadIdx.x;
+        int total;
+        const int ex = tree_level_scan(t < ntile ? tile_small[t] : 0, warp_tot, total);
+        if (t < ntile) tile_pre[t] = carry + ex;
+        carry += total;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < nseg; q += kTreeLevelThreads) {
+        TreeSeg g = segs[q];
+        const int t1 = g.tile0 + (g.length + kTreeTile - 1) / kTreeTile;
+        g.before = tile_pre[g.tile0];
+        g.nsmall = (t1 < ntile ? tile_pre[t1] : carry) - g.before;
+        g.nbig = g.length - g.nsmall;
+        segs[q] = g;
+        const int left = g.nbig == 0 ? g.length - 1 : g.nsmall;
+        for (int c = 0; c < 2; ++c) {
+            const int np = c ? g.length - left : left, ip = c ? g.ipart + left : g.ipart, axis = (g.axis + 1) % 3;
+            int code = -1;
+            if (np <= maxleaf) {
+                const int l = atomicAdd(&s_leaf, 1);
+                if (l < R.leaf_cap) {
+                    R.lipart[l] = ip;
+                    R.lnpart[l] = np;
+                    code = 2 * l;
+                } else {
+                    atomicOr(&R.counters[2], TB_LEAF_CAP);
+                }
+            } else if (np <= kTreeSmall) {
+                const int k = atomicAdd(&s_task, 1);
+                if (k < task_cap) tasks[k] = TreeTask{ip, np, axis, level + 1, g.node, c};
+                else atomicOr(&R.counters[2], TB_NODE_CAP);
+                continue;  // the subtree's block records its root
+            } else {
+                const int k = atomicAdd(&s_node, 1), j = atomicAdd(&s_next, 1);
+                if (k < R.node_cap && j < seg_cap) {
+                    R.depth[k] = level + 1;
+                    next[j] = TreeSeg{ip, np, axis, k, 0.0, 0, 0, 0, 0};
+                    code = 2 * k + 1;
+                } else {
+                    atomicOr(&R.counters[2], TB_NODE_CAP);
+                }
+            }
+            R.son[2 * g.node + c] = code;
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ntile; t += kTreeLevelThreads) tile_pre[t] -= segs[tile_seg[t]].before;
+    const int nnext = min(s_next, seg_cap);
+    carry = 0;
+    for (int b = 0; b < nnext; b += kTreeLevelThreads) {
+        const int q = b + threadIdx.x;
+        int total;
+        const int ex = tree_level_scan(q < nnext ? (next[q].length + kTreeTile - 1) / kTreeTile : 0, warp_tot, total);
+        if (q < nnext) next[q].tile0 = carry + ex;
+        carry += total;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x >> 5; q < nnext; q += kTreeLevelThreads / 32) {
+        const int t0 = next[q].tile0, nt = (next[q].length + kTreeTile - 1) / kTreeTile;
+        for (int k = threadIdx.x & 31; k < nt; k += 32) {
+            next_tile_seg[t0 + k] = q;
+            next_tile_off[t0 + k] = k * kTreeTile;
+        }
+    }
+    if (threadIdx.x == 0) {
+        lv->nseg[level + 1] = nnext;
+        lv->ntile[level + 1] = carry;
+        lv->ntask = min(s_task, task_cap);
+        R.counters[0] = min(s_node, R.node_cap);
+        R.counters[1] = min(s_leaf, R.leaf_cap);
+        if (nnext > 0) R.counters[3] = level + 1;
+    }
+}
 
 struct SmallItem {
     int span;    // slot offset in the task (low 16 bits) and length (high 16 bits)
