@@ -174,21 +174,22 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
     TreeParts P;
     TreeRec R;
     std::memset(&R, 0, sizeof(R));
-    int *map = nullptr;
+    int *map = nullptr, *parent = nullptr, *lparent = nullptr, *arrived = nullptr;
     float *blo = nullptr, *bhi = nullptr;
     const int init_blocks = grid(n, kTreeThreads, 1024);
     bool ok = S.get(&P.x, n) && S.get(&P.y, n) && S.get(&P.z, n) && S.get(&P.id, n) && S.get(&map, n) &&
               S.get(&blo, 3 * (size_t)init_blocks) && S.get(&bhi, 3 * (size_t)init_blocks) &&
               S.get(&R.split, cap) && S.get(&R.son, 2 * (size_t)cap) && S.get(&R.depth, cap) &&
               S.get(&R.nn, cap) && S.get(&R.nl, cap) && S.get(&R.pre, cap) && S.get(&R.first, cap) &&
-              S.get(&R.box, 6 * (size_t)cap) && S.get(&R.lipart, cap) && S.get(&R.lnpart, cap) &&
-              S.get(&R.lid, cap) && S.get(&R.counters, 4);
+              S.get(&R.box, 6 * (size_t)cap) && S.get(&R.root, 6) && S.get(&R.lipart, cap) && S.get(&R.lnpart, cap) &&
+              S.get(&R.lid, cap) && S.get(&parent, cap) && S.get(&lparent, cap) && S.get(&arrived, cap) &&
+              S.get(&R.counters, 3);
     if (!ok) return report_error(P2P_ERR_NOMEM, "tree build: device allocation failed");
     R.node_cap = cap;
     R.leaf_cap = cap;
 
     tree_init_kernel<<<init_blocks, kTreeThreads, 0, st>>>(d_pos, n, P, blo, bhi);
-    tree_root_box_kernel<<<1, 96, 0, st>>>(blo, bhi, init_blocks, boxsize, R, 0);
+    tree_root_box_kernel<<<1, 96, 0, st>>>(blo, bhi, init_blocks, boxsize, R);
     launches += 2;
 
     // ---- nodes above kTreeSmall particles, level by level; the host reads the
@@ -205,11 +206,11 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
     ok = ok && S.get(&tile_small, tile_cap) && S.get(&tile_pre, tile_cap) && S.get(&tasks, task_cap) && S.get(&lv, 1);
     if (!ok) return report_error(P2P_ERR_NOMEM, "tree build: device allocation failed");
     TREE_CUDA(cudaMemsetAsync(lv, 0, sizeof(TreeLevels), st));
-    TREE_CUDA(cudaMemsetAsync(R.counters, 0, 4 * sizeof(int), st));
+    TREE_CUDA(cudaMemsetAsync(R.counters, 0, 3 * sizeof(int), st));
     tree_first_level_kernel<<<grid((n + kTreeTile - 1) / kTreeTile, kTreeThreads, INT32_MAX), kTreeThreads, 0, st>>>(
         n, segs[0], tile_seg[0], tile_off[0], tasks, lv, R);
     launches += 1;
-    int hc[4] = {0, 0, 0, 0}, ntask = 0, left = 0, level = 0;
+    int hc[3] = {0, 0, 0}, ntask = 0, left = 0, level = 0;
     int batch = 0;
     while (n > kTreeSmall && ((int64_t)kTreeSmall << batch) < n) ++batch;
     for (batch = n > kTreeSmall ? batch + 2 : 0;; batch = 2) {
@@ -254,15 +255,13 @@ int build_into(p2p_session *s, p2p_dtree *tree, int npart, const double *d_pos, 
     if (hc[2] & (TB_NODE_CAP | TB_LEAF_CAP))
         return report_error(P2P_ERR_CAPACITY, "tree build: more nodes or leaves than the build's capacity");
     const int nnode = hc[0], nleaf = hc[1];
-    const int maxdepth = hc[3];
 
-    // ---- pre-order numbering and boxes, by depth ----
+    // ---- pre-order numbering and boxes ----
     const int gn = grid(nnode, 256, 4096);
-    for (int d = maxdepth; d >= 0; --d) tree_count_kernel<<<gn, 256, 0, st>>>(R, nnode, d);
-    TREE_CUDA(cudaMemsetAsync(R.pre, 0, sizeof(int), st));    // the root (build id 0): pre-order id 0
-    TREE_CUDA(cudaMemsetAsync(R.first, 0, sizeof(int), st));  // its first leaf: 0
-    for (int d = 0; d <= maxdepth; ++d) tree_order_kernel<<<gn, 256, 0, st>>>(R, nnode, d);
-    launches += 2 * (maxdepth + 1);
+    tree_link_kernel<<<gn, 256, 0, st>>>(R, nnode, nleaf, parent, lparent, arrived);
+    tree_count_kernel<<<grid(nleaf, 256, 4096), 256, 0, st>>>(R, nnode, nleaf, parent, lparent, arrived);
+    tree_order_kernel<<<gn, 256, 0, st>>>(R, nnode, parent);
+    launches += 3;
 
     p2p_dtree *t = tree;
     t->device = session_device(s);

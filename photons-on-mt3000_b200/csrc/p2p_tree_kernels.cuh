@@ -46,11 +46,12 @@ struct TreeRec {
     int *pre;      // pre-order id
     int *first;    // pre-order id of the subtree's first leaf
     double *box;   // 6 per node: left[3], right[3]
+    double *root;  // the root's
     int node_cap;
     // leaves
     int *lipart, *lnpart, *lid;  // particle range, pre-order leaf id
     int leaf_cap;
-    int *counters;  // [0] nodes made, [1] leaves made, [2] status bits, [3] max depth
+    int *counters;  // [0] nodes made, [1] leaves made, [2] status bits
 };
 
 // Particles being partitioned: SoA coordinates and original indices.
@@ -206,7 +207,7 @@ __global__ void tree_init_kernel(const double *__restrict__ pos, int n, TreePart
 // three warps, one axis each).
 __global__ void __launch_bounds__(96)
 tree_root_box_kernel(const float *__restrict__ block_lo, const float *__restrict__ block_hi, int nblocks,
-                     double boxsize, TreeRec R, int root) {
+                     double boxsize, TreeRec R) {
     const int lane = threadIdx.x & 31, d = threadIdx.x >> 5;
     double lo = boxsize, hi = 0.0;
     for (int b = lane; b < nblocks; b += 32) {
@@ -220,8 +221,8 @@ tree_root_box_kernel(const float *__restrict__ block_lo, const float *__restrict
     }
     if (lane == 0) {
         const double margin = __dmul_rn(0.000001, boxsize);
-        R.box[6 * (size_t)root + d] = __dsub_rn(lo, margin);
-        R.box[6 * (size_t)root + 3 + d] = __dadd_rn(hi, margin);
+        R.root[d] = __dsub_rn(lo, margin);
+        R.root[3 + d] = __dadd_rn(hi, margin);
     }
 }
 
@@ -633,7 +634,6 @@ tree_level_kernel(TreeSeg *segs, const int *__restrict__ tile_seg, const int *__
         lv->ntask = min(s_task, task_cap);
         R.counters[0] = min(s_node, R.node_cap);
         R.counters[1] = min(s_leaf, R.leaf_cap);
-        if (nnext > 0) R.counters[3] = level + 1;
     }
 }
 
@@ -700,8 +700,7 @@ tree_small_kernel(const TreeTask *__restrict__ tasks, TreeParts P, TreeRec R, in
         s_node0 = atomicAdd(&R.counters[0], 1);
     }
     __syncthreads();
-    int depth = T.depth;
-    for (int half = 0;; half ^= 1, ++depth) {
+    for (int half = 0;; half ^= 1) {
         const int count = s_count[half], node0 = s_node0;
         if (node0 + count > R.node_cap) {  // block-uniform
             if (threadIdx.x == 0) atomicOr(&R.counters[2], TB_NODE_CAP);
@@ -796,7 +795,6 @@ tree_small_kernel(const TreeTask *__restrict__ tasks, TreeParts P, TreeRec R, in
         if (!more) break;
         __syncthreads();  // the leaves are read, the counts are reset
     }
-    if (threadIdx.x == 0) atomicMax(&R.counters[3], depth);
     __syncthreads();
     for (int i = threadIdx.x; i < T.length; i += blockDim.x) {
         P.x[T.ipart + i] = sx[i];
@@ -808,66 +806,90 @@ tree_small_kernel(const TreeTask *__restrict__ tasks, TreeParts P, TreeRec R, in
 
 // ------------------------------------------------- numbering and boxes ---
 
-// Bottom-up, nodes of depth d: subtree node and leaf counts.
-__global__ void tree_count_kernel(TreeRec R, int nnode, int d) {
+// Three passes whatever the tree's depth (one launch per depth, twice, took 26 to
+// 52 launches, a tenth of a small step): parents, counts by climbing, numbers and
+// boxes by climbing.
+
+// Each box's parent as 2 x node + side (-1: the root), nodes' arrival counts 0.
+__global__ void tree_link_kernel(TreeRec R, int nnode, int nleaf, int *__restrict__ parent,
+                                 int *__restrict__ lparent, int *__restrict__ arrived) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnode; k += gridDim.x * blockDim.x) {
-        if (R.depth[k] != d) continue;
-        int nn = 1, nl = 0;
+        arrived[k] = 0;
+        if (k == 0) parent[0] = -1;
         for (int n = 0; n < 2; ++n) {
             const int c = R.son[2 * k + n];
-            if (c < 0 || ((c & 1) && (c >> 1) >= nnode)) {  // a child never recorded
+            if (c < 0 || c == 1 || ((c & 1) ? (c >> 1) >= nnode : (c >> 1) >= nleaf)) {  // a child never recorded
                 atomicOr(&R.counters[2], TB_NUMBERING);
                 continue;
             }
-            if (c & 1) {
-                nn += R.nn[c >> 1];
-                nl += R.nl[c >> 1];
-            } else {
-                nl += 1;
-            }
+            if (c & 1) parent[c >> 1] = 2 * k + n;
+            else lparent[c >> 1] = 2 * k + n;
         }
-        R.nn[k] = nn;
-        R.nl[k] = nl;
     }
 }
 
-// Top-down, nodes of depth d (whose pre-order id, first leaf and box are
-// set): the children's ids, first leaves and boxes (center_kdtree,
-// src/fmm.c:273-327).
-__global__ void tree_order_kernel(TreeRec R, int nnode, int d) {
+// Subtree node and leaf counts: a thread per leaf climbs while it is the second
+// of a node's two children to arrive.
+__global__ void tree_count_kernel(TreeRec R, int nnode, int nleaf, const int *__restrict__ parent,
+                                  const int *__restrict__ lparent, int *__restrict__ arrived) {
+    if (R.counters[2] & TB_NUMBERING) return;
+    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nleaf; l += gridDim.x * blockDim.x) {
+        for (int p = lparent[l]; p >= 0;) {
+            const int k = p >> 1;
+            __threadfence();
+            if (atomicAdd(&arrived[k], 1) == 0) break;
+            __threadfence();
+            int nn = 1, nl = 0;
+            for (int n = 0; n < 2; ++n) {
+                const int c = R.son[2 * k + n];
+                nn += (c & 1) ? __ldcg(&R.nn[c >> 1]) : 0;
+                nl += (c & 1) ? __ldcg(&R.nl[c >> 1]) : 1;
+            }
+            R.nn[k] = nn;
+            R.nl[k] = nl;
+            p = parent[k];
+        }
+    }
+}
+
+// Every node's pre-order id, first leaf and box from its path to the root, and
+// the ids of its leaves (center_kdtree, src/fmm.c:273-327: an ancestor split on
+// an axis bounds the box on the side it was left by, the nearest one counts).
+__global__ void tree_order_kernel(TreeRec R, int nnode, const int *__restrict__ parent) {
+    if (R.counters[2] & TB_NUMBERING) return;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnode; k += gridDim.x * blockDim.x) {
-        if (R.depth[k] != d) continue;
-        const int axis = d % 3;
-        const double split = R.split[k];
-        const int pre = R.pre[k], first = R.first[k];
-        const double *bx = R.box + 6 * (size_t)k;
+        double box[6];
+        unsigned known = 0;
+        int pre = 0, first = 0, steps = 0;
+        for (int p = parent[k]; p >= 0; p = parent[p >> 1]) {
+            if (++steps > nnode) break;
+            const int a = p >> 1, right = p & 1;
+            const int side = R.depth[a] % 3 + (right ? 0 : 3);  // left child: right[axis] = split
+            if (!(known >> side & 1u)) {
+                known |= 1u << side;
+                const double split = R.split[a];
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    if (q == side) box[q] = split;
+            }
+            pre += 1;
+            if (right) {
+                const int c = R.son[2 * a];
+                pre += (c & 1) ? R.nn[c >> 1] : 0;
+                first += (c & 1) ? R.nl[c >> 1] : 1;
+            }
+        }
+        double root[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) root[q] = R.root[q];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) R.box[6 * (size_t)k + q] = known >> q & 1u ? box[q] : root[q];
+        R.pre[k] = pre;
+        R.first[k] = first;
         const int c0 = R.son[2 * k], c1 = R.son[2 * k + 1];
-        const int nodes0 = (c0 & 1) ? R.nn[c0 >> 1] : 0;
-        const int leaves0 = (c0 & 1) ? R.nl[c0 >> 1] : 1;
-        if ((c0 & 1) && (unsigned)(c0 >> 1) >= (unsigned)nnode) {
-            atomicOr(&R.counters[2], TB_NUMBERING);
-            continue;
-        }
-        for (int n = 0; n < 2; ++n) {
-            const int c = n == 0 ? c0 : c1;
-            if ((c & 1) ? (unsigned)(c >> 1) >= (unsigned)nnode : (unsigned)(c >> 1) >= (unsigned)R.leaf_cap) {
-                atomicOr(&R.counters[2], TB_NUMBERING);
-                continue;
-            }
-            const int cpre = n == 0 ? pre + 1 : pre + 1 + nodes0;
-            const int cfirst = n == 0 ? first : first + leaves0;
-            if (c & 1) {
-                const int j = c >> 1;
-                R.pre[j] = cpre;
-                R.first[j] = cfirst;
-                double *cb = R.box + 6 * (size_t)j;
-                for (int q = 0; q < 6; ++q) cb[q] = bx[q];
-                if (n == 0) cb[3 + axis] = split;  // right[axis] = split
-                else cb[axis] = split;             // left[axis] = split
-            } else {
-                R.lid[c >> 1] = cfirst;
-            }
-        }
+        if (!(c0 & 1)) R.lid[c0 >> 1] = first;
+        if (!(c1 & 1)) R.lid[c1 >> 1] = first + ((c0 & 1) ? R.nl[c0 >> 1] : 1);
+        if (steps > nnode) atomicOr(&R.counters[2], TB_NUMBERING);
     }
 }
 
