@@ -89,7 +89,9 @@ struct p2p_session {
     // device buffers
     DevBuf task_t2, task_s2;  // second buffer pair of pipelined submits
     DevBuf pos, mass, leaf_ip, leaf_np, task_t, task_s, meta, pos4, counts, fill, row_off,
-        row_src, tile_sums, acc, parts, status, queue, pairs, skipped, evaluated, probe;
+        row_src, tile_sums, acc, parts, ctl, probe;
+    // in ctl
+    void *status = nullptr, *queue = nullptr, *pairs = nullptr, *skipped = nullptr, *evaluated = nullptr;
     DevBuf keys_a, keys_b, vals_b, hist, hoffs, hsums;  // radix sort of the list
     std::vector<DevBuf> scratch;  // grow-only temporaries of p2p_dtree_build, by request order
     // device walk (p2p_pass_submit_walk): box records, active prefix, boxes of
@@ -145,6 +147,9 @@ bool is_fp32_form(int form) { return form != P2P_FORM_PLAIN_FP64; }
 // The device walk keeps its rows in a pool of at most this size; longer ones
 // take a second walk.
 constexpr size_t kWalkPoolBytes = (size_t)8 << 30;
+
+// Status word, work queue and pair counters, 64 bytes apart.
+constexpr size_t kCtlBytes = 5 * 64;
 
 // Host list submits longer than 2 * kPipePieceMin entries are uploaded and
 // computed in about kPipePieces pieces of at least kPipePieceMin entries.
@@ -308,18 +313,18 @@ int enqueue_prep(p2p_session *s) {
     const int threads = 256;
     if (form == P2P_FORM_PLAIN_FP64) {
         prep_plain_kernel<<<grid_for(nleaf, threads, 65535), threads, 0, s->stream>>>(
-            s->d_ip, s->d_np, npart, nleaf, meta, (int *)s->status.p);
+            s->d_ip, s->d_np, npart, nleaf, meta, (int *)s->status);
     } else {
         const int blocks = grid_for((int64_t)nleaf * 32, threads, 65535);
         const double c = 0.5 / s->params.split_radius;
         if (form == P2P_FORM_NAIVE_FP32)
             prep_split_kernel<false><<<blocks, threads, 0, s->stream>>>(
                 s->d_pos, s->d_mass, s->d_ip, s->d_np, npart, nleaf, c, meta, (float4 *)s->pos4.p,
-                (int *)s->status.p);
+                (int *)s->status);
         else
             prep_split_kernel<true><<<blocks, threads, 0, s->stream>>>(
                 s->d_pos, s->d_mass, s->d_ip, s->d_np, npart, nleaf, c, meta, (float4 *)s->pos4.p,
-                (int *)s->status.p);
+                (int *)s->status);
     }
     CUDA_TRY(cudaGetLastError());
     return launch_count(1);
@@ -336,8 +341,8 @@ PairArgs make_args(p2p_session *s) {
     a.pos = s->d_pos;
     a.mass = s->d_mass;
     a.acc = (double *)s->acc.p;
-    a.queue = (int *)s->queue.p;
-    a.evaluated = counts_evaluated(p) ? (unsigned long long *)s->evaluated.p : nullptr;
+    a.queue = (int *)s->queue;
+    a.evaluated = counts_evaluated(p) ? (unsigned long long *)s->evaluated : nullptr;
     a.npart = s->npart;
     a.nleaf = s->nleaf;
     fill_pass_scalars(a, p, s->fit, s->d_mass != nullptr);
@@ -381,14 +386,14 @@ int enqueue_chunk(p2p_session *s, int64_t ntask, const int *d_t, const int *d_s,
     b.hist = (int *)s->hist.p;
     b.hoffs = (int64_t *)s->hoffs.p;
     b.hsums = (int64_t *)s->hsums.p;
-    b.pairs = (unsigned long long *)s->pairs.p;
+    b.pairs = (unsigned long long *)s->pairs;
     if (skips_outside(s)) {
         // the packed kernels skip entries wholly beyond the cutoff; count their pairs
-        b.skipped = (unsigned long long *)s->skipped.p;
+        b.skipped = (unsigned long long *)s->skipped;
         b.cscale = 0.5 / s->params.split_radius;
         b.uout = (float)(s->fit.umax * (1.0 + kCutBand) * (1.0 + kOutsideMargin));
     }
-    b.status = (int *)s->status.p;
+    b.status = (int *)s->status;
     int launched = 0;
     CUDA_TRY(enqueue_csr_build(s->stream, ntask, d_t, d_s, s->nleaf, (const LeafMeta *)s->meta.p, b,
                                &launched));
@@ -399,7 +404,7 @@ int enqueue_chunk(p2p_session *s, int64_t ntask, const int *d_t, const int *d_s,
 
 // The pair kernel over the session's CSR rows (row_off, row_src).
 int enqueue_pairs(p2p_session *s, bool timed) {
-    CUDA_TRY(cudaMemsetAsync(s->queue.p, 0, sizeof(int), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->queue, 0, sizeof(int), s->stream));
     PairArgs a = make_args(s);
     const int parts = row_parts(s);
     const int64_t n3 = 3 * (int64_t)s->npart;
@@ -444,20 +449,17 @@ int size_pass_buffers(p2p_session *s, int npart, int nleaf, bool host_inputs, bo
     P2P_TRY(ensure(s, s->fill, sizeof(int) * (size_t)nleaf));
     P2P_TRY(ensure(s, s->row_off, sizeof(int64_t) * ((size_t)nleaf + 1)));
     P2P_TRY(ensure(s, s->tile_sums, sizeof(int64_t) * csr_tile_sums(nleaf)));
-    P2P_TRY(ensure(s, s->status, sizeof(int)));
-    P2P_TRY(ensure(s, s->queue, sizeof(int)));
-    P2P_TRY(ensure(s, s->pairs, sizeof(unsigned long long)));
-    P2P_TRY(ensure(s, s->skipped, sizeof(unsigned long long)));
-    P2P_TRY(ensure(s, s->evaluated, sizeof(unsigned long long)));
+    // the pass's counters lie together: one fill clears them
+    P2P_TRY(ensure(s, s->ctl, kCtlBytes));
+    unsigned char *c = (unsigned char *)s->ctl.p;
+    void **at[] = {&s->status, &s->queue, &s->pairs, &s->skipped, &s->evaluated};
+    for (int k = 0; k < 5; ++k) *at[k] = c + 64 * k;
     return P2P_OK;
 }
 
 int begin_common(p2p_session *s) {
     CUDA_TRY(cudaMemsetAsync(s->acc.p, 0, sizeof(double) * 3 * (size_t)s->npart, s->stream));
-    CUDA_TRY(cudaMemsetAsync(s->status.p, 0, sizeof(int), s->stream));
-    CUDA_TRY(cudaMemsetAsync(s->pairs.p, 0, sizeof(unsigned long long), s->stream));
-    CUDA_TRY(cudaMemsetAsync(s->skipped.p, 0, sizeof(unsigned long long), s->stream));
-    CUDA_TRY(cudaMemsetAsync(s->evaluated.p, 0, sizeof(unsigned long long), s->stream));
+    CUDA_TRY(cudaMemsetAsync(s->ctl.p, 0, kCtlBytes, s->stream));
     return enqueue_prep(s);
 }
 
@@ -569,7 +571,7 @@ P2P_API int p2p_session_destroy(p2p_session *s) {
     if (s->gexec) cudaGraphExecDestroy(s->gexec);
     DevBuf *bufs[] = {&s->pos, &s->mass, &s->leaf_ip, &s->leaf_np, &s->task_t, &s->task_s,
                       &s->meta, &s->pos4, &s->counts, &s->fill, &s->row_off, &s->row_src,
-                      &s->tile_sums, &s->acc, &s->parts, &s->status, &s->queue, &s->pairs, &s->skipped, &s->evaluated, &s->probe,
+                      &s->tile_sums, &s->acc, &s->parts, &s->ctl, &s->probe,
                       &s->keys_a, &s->keys_b, &s->vals_b, &s->hist, &s->hoffs, &s->hsums,
                       &s->task_t2, &s->task_s2, &s->walk_box, &s->walk_active, &s->walk_items, &s->walk_lists[0],
                       &s->walk_lists[1], &s->walk_rows, &s->walk_ctrl};
@@ -798,7 +800,7 @@ P2P_API int p2p_pass_end(p2p_session *s, double *gpu_seconds) {
     CUDA_TRY(cudaEventElapsedTime(&ms, s->ev_begin, s->ev_end));
     if (gpu_seconds) *gpu_seconds = ms * 1e-3;
     int status = 0;
-    CUDA_TRY(cudaMemcpy(&status, s->status.p, sizeof(int), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(&status, s->status, sizeof(int), cudaMemcpyDeviceToHost));
     if (status & ST_LEAF_RANGE) return fail(P2P_ERR_RANGE, "a leaf range lies outside the particles");
     if (status & ST_TASK_RANGE) return fail(P2P_ERR_RANGE, "a task entry names a leaf outside [0, nleaf)");
     if (status & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
@@ -911,9 +913,9 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
             const int bad = st & (ST_WALK_TREE | ST_WALK_STACK | ST_WALK_ROW);
             if (bad) {  // closing the pass reports it too
                 int main_status = 0;
-                CUDA_TRY(cudaMemcpy(&main_status, s->status.p, sizeof(int), cudaMemcpyDeviceToHost));
+                CUDA_TRY(cudaMemcpy(&main_status, s->status, sizeof(int), cudaMemcpyDeviceToHost));
                 main_status |= bad;
-                CUDA_TRY(cudaMemcpy(s->status.p, &main_status, sizeof(int), cudaMemcpyHostToDevice));
+                CUDA_TRY(cudaMemcpy(s->status, &main_status, sizeof(int), cudaMemcpyHostToDevice));
                 if (bad & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
                 return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
             }
@@ -932,17 +934,17 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     if (!chains) P2P_TRY(walk(true));
     const double cscale = 0.5 / s->params.split_radius;
     const float uout = (float)(s->fit.umax * (1.0 + kCutBand) * (1.0 + kOutsideMargin));
-    unsigned long long *d_skipped = skip ? (unsigned long long *)s->skipped.p : nullptr;
+    unsigned long long *d_skipped = skip ? (unsigned long long *)s->skipped : nullptr;
     // the rows into their places, and their pair counts
     const int gather = grid_for(nleaf, 8, s->sm_count * 16);
     if (chains)
         walk_gather_kernel<true><<<gather, 256, 0, s->stream>>>(counts, heads, row_off, nleaf, g.out, (int *)s->row_src.p,
                                                                s->d_np, (const LeafMeta *)s->meta.p, cscale, uout,
-                                                               (unsigned long long *)s->pairs.p, d_skipped);
+                                                               (unsigned long long *)s->pairs, d_skipped);
     else
         walk_gather_kernel<false><<<gather, 256, 0, s->stream>>>(counts, heads, row_off, nleaf, g.out, (int *)s->row_src.p,
                                                                 s->d_np, (const LeafMeta *)s->meta.p, cscale, uout,
-                                                                (unsigned long long *)s->pairs.p, d_skipped);
+                                                                (unsigned long long *)s->pairs, d_skipped);
     CUDA_TRY(cudaGetLastError());
     launch_count(1);
     return enqueue_pairs(s, true);
@@ -998,12 +1000,12 @@ P2P_API int p2p_pass_evaluated_pairs(p2p_session *s, int64_t *pairs) {
     unsigned long long v = 0, k = 0;
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (counts_evaluated(s->params)) {
-        CUDA_TRY(cudaMemcpy(&v, s->evaluated.p, sizeof(v), cudaMemcpyDeviceToHost));
+        CUDA_TRY(cudaMemcpy(&v, s->evaluated, sizeof(v), cudaMemcpyDeviceToHost));
         *pairs = (int64_t)v;
         return P2P_OK;
     }
-    CUDA_TRY(cudaMemcpy(&v, s->pairs.p, sizeof(v), cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(&k, s->skipped.p, sizeof(k), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(&v, s->pairs, sizeof(v), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(&k, s->skipped, sizeof(k), cudaMemcpyDeviceToHost));
     *pairs = (int64_t)(v - k);
     return P2P_OK;
 }
@@ -1013,7 +1015,7 @@ P2P_API int p2p_pass_pair_count(p2p_session *s, int64_t *pairs) {
     if (!pairs) return fail(P2P_ERR_ARG, "null argument");
     unsigned long long v = 0;
     CUDA_TRY(cudaStreamSynchronize(s->stream));
-    CUDA_TRY(cudaMemcpy(&v, s->pairs.p, sizeof(v), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(&v, s->pairs, sizeof(v), cudaMemcpyDeviceToHost));
     *pairs = (int64_t)v;
     return P2P_OK;
 }

@@ -60,13 +60,13 @@ inline cudaError_t enqueue_csr_build(cudaStream_t st, int64_t ntask, const int *
     scan_add_kernel<<<csr_grid(nleaf, threads, 1 << 30), threads, 0, st>>>(b.row_off, nleaf, b.tile_sums);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     *launches += 4;
-    // radix passes over keys in [0, nleaf]: 8-bit digits, or two 10-bit
-    // digits for 17-20 key bits (one pass fewer)
+    // radix passes over keys in [0, nleaf]: 8-bit digits, or 10-bit digits where
+    // that is a pass fewer (9-10 key bits: 5 launches; 17-20: a whole pass)
     int bits = 1;
     while (bits < 31 && ((int64_t)1 << bits) <= (int64_t)nleaf) ++bits;
     const int rtiles = (int)((ntask + kRadixTile - 1) / kRadixTile);
     // (10-bit digits up to 2^20 tiles: 4 GB of histogram and 8 GB of offsets there)
-    const int digit = (bits > 16 && bits <= 20 && rtiles <= (1 << 20)) ? 10 : 8;
+    const int digit = ((bits > 16 && bits <= 20) || (bits > 8 && bits <= 10)) && rtiles <= (1 << 20) ? 10 : 8;
     const int passes = (bits + digit - 1) / digit;
     const int nchunks = (rtiles + kColTiles - 1) / kColTiles;
     int *kbuf[2] = {b.keys_a, b.keys_b};
@@ -92,7 +92,12 @@ inline cudaError_t enqueue_csr_build(cudaStream_t st, int64_t ntask, const int *
                 radix_hist_kernel<8, false><<<rtiles, kRadixWarps * 32, 0, st>>>(kin, d_t, d_s, nleaf, ntask,
                                                                                  shift, b.hist, rtiles);
         }
-        if (digit == 10) {
+        if (rtiles <= kRadixFewTiles) {
+            if (digit == 10)
+                radix_offs_few_kernel<1024><<<1, 1024, 0, st>>>(b.hist, rtiles, b.hoffs);
+            else
+                radix_offs_few_kernel<256><<<1, 256, 0, st>>>(b.hist, rtiles, b.hoffs);
+        } else if (digit == 10) {
             radix_colsum_kernel<1024><<<nchunks, 1024, 0, st>>>(b.hist, rtiles, b.hsums);
             radix_colscan_kernel<1024><<<1, 1024, 0, st>>>(b.hsums, nchunks);
             radix_offs_kernel<1024><<<nchunks, 1024, 0, st>>>(b.hist, rtiles, b.hsums, b.hoffs);
@@ -117,7 +122,7 @@ inline cudaError_t enqueue_csr_build(cudaStream_t st, int64_t ntask, const int *
                     kin, vin, d_t, d_s, nleaf, ntask, shift, b.hoffs, rtiles, kout, vout);
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        *launches += 5;
+        *launches += rtiles <= kRadixFewTiles ? 3 : 5;
         kin = kout;
         vin = vout;
     }

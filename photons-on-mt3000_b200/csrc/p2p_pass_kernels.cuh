@@ -507,6 +507,39 @@ radix_offs_kernel(const int *__restrict__ hist, int ntiles, const int64_t *__res
     }
 }
 
+// The same for a short list in one launch of one block (a chain of three costs
+// as much as the scan itself: 12^3, 15 tiles). kRadixFewTiles tiles at most.
+constexpr int kRadixFewTiles = 32;
+
+template <int NB>
+__global__ void __launch_bounds__(NB)
+radix_offs_few_kernel(const int *__restrict__ hist, int ntiles, int64_t *__restrict__ offs) {
+    constexpr int NW = NB / 32;
+    __shared__ int wsum[NW];
+    const int d = threadIdx.x, lane = d & 31, w = d >> 5;
+    int h[kRadixFewTiles];  // every tile's count of this digit, loaded together
+    int tot = 0;
+#pragma unroll
+    for (int t = 0; t < kRadixFewTiles; ++t) h[t] = t < ntiles ? hist[t * NB + d] : 0;
+#pragma unroll
+    for (int t = 0; t < kRadixFewTiles; ++t) tot += h[t];
+    int x = tot;  // digit starts: exclusive scan of the totals over the digits
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(kFull, x, off);
+        if (lane >= off) x += y;
+    }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    int run = x - tot;
+    for (int q = 0; q < w; ++q) run += wsum[q];
+#pragma unroll
+    for (int t = 0; t < kRadixFewTiles; ++t) {
+        if (t < ntiles) offs[t * NB + d] = run;
+        run += h[t];
+    }
+}
+
 // Exclusive scan int32 -> int64 in three kernels. kScanTile elements per block.
 constexpr int kScanThreads = 256;
 constexpr int kScanPer = 8;
