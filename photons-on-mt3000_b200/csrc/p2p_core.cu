@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <tuple>
 #include <string>
 #include <vector>
@@ -79,6 +80,9 @@ struct p2p_session {
     // buffer pairs while the previous piece computes on stream
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t piece_ready[2] = {nullptr, nullptr}, piece_free[2] = {nullptr, nullptr};
+    // p2p_pass_accumulate's piece, one caller at a time
+    std::mutex stage_lock;
+    std::vector<double> stage;
     bool kernel_timed = false;
     bool dry_run = false;  // dispatch without launching (fills the occupancy cache)
     int last_blocks = 0;
@@ -147,6 +151,9 @@ bool is_fp32_form(int form) { return form != P2P_FORM_PLAIN_FP64; }
 // The device walk keeps its rows in a pool of at most this size; longer ones
 // take a second walk.
 constexpr size_t kWalkPoolBytes = (size_t)8 << 30;
+
+// Doubles per piece of p2p_pass_accumulate (512 KB).
+constexpr size_t kStageDoubles = 65536;
 
 // Status word, work queue and pair counters, 64 bytes apart.
 constexpr size_t kCtlBytes = 5 * 64;
@@ -966,10 +973,18 @@ P2P_API int p2p_pass_accumulate(p2p_session *s, double *acc) {
     P2P_TRY(check_session(s));
     if (s->in_pass) return fail(P2P_ERR_STATE, "pass still open; call p2p_pass_end first");
     if (!acc && s->npart) return fail(P2P_ERR_ARG, "null acc");
+    // By pieces through a kept buffer that stays in the cache: one copy of the
+    // whole into a new buffer touched its pages for the first time in every pass
+    // (a 32^3 pass from host arrays 1.35 ms, now 1.25). Page-locked pieces take
+    // 1.06 ms, but every session would pay 3 ms for them when it is created.
     const size_t n3 = 3 * (size_t)s->npart;
-    std::vector<double> buf(n3);
-    if (n3) CUDA_TRY(cudaMemcpy(buf.data(), s->acc.p, sizeof(double) * n3, cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n3; ++i) acc[i] += buf[i];
+    std::lock_guard<std::mutex> hold(s->stage_lock);
+    s->stage.resize(std::max(s->stage.size(), std::min(n3, kStageDoubles)));
+    for (size_t at = 0; at < n3; at += kStageDoubles) {
+        const size_t n = std::min(kStageDoubles, n3 - at);
+        CUDA_TRY(cudaMemcpy(s->stage.data(), (const double *)s->acc.p + at, sizeof(double) * n, cudaMemcpyDeviceToHost));
+        for (size_t i = 0; i < n; ++i) acc[at + i] += s->stage[i];
+    }
     return P2P_OK;
 }
 
