@@ -83,11 +83,6 @@ constexpr unsigned kFull = 0xffffffffu;
 // cell, next to each other in the input, as in tree or cell order): a
 // segmented scan over the lanes, as many steps as the longest run needs,
 // then one FP64 atomic per run. A warp whose lanes all differ skips the scan.
-// The scans, not the atomics, bound it (0.82 ms at 256^3 in cell order with
-// keys compared, runs measured and reduced corner by corner), so the lanes
-// compare their cells once per axis and side, six ballots in all: a corner's
-// runs, and which lanes have 1, 2, 4, ... predecessors in theirs, are bit
-// operations on those.
 __global__ void __launch_bounds__(256) pm_deposit_kernel(const double *__restrict__ pos, const int *__restrict__ tag,
                                                          int npart, double mass, int n, double norm, double delta,
                                                          double *__restrict__ mesh) {
@@ -96,42 +91,32 @@ __global__ void __launch_bounds__(256) pm_deposit_kernel(const double *__restric
     for (int base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < npart; base += stride) {
         const int p = base + lane;
         const bool on = p < npart && (!tag || tag[p] == 1);
-        int c[3][2] = {{-1, -1}, {-1, -1}, {-1, -1}};  // cell and neighbour per axis; -1 matches no particle's
+        int c[3] = {0, 0, 0}, nb[3] = {0, 0, 0};
         double w[3] = {0.0, 0.0, 0.0};
         if (on)
-            for (int a = 0; a < 3; ++a) cic_axis(pos[(size_t)a * npart + p], norm, delta, n, c[a][0], c[a][1], w[a]);
-        unsigned same[3][2];  // lanes whose cell (neighbour) on the axis is that of the lane before
+            for (int a = 0; a < 3; ++a) cic_axis(pos[(size_t)a * npart + p], norm, delta, n, c[a], nb[a], w[a]);
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                same[a][h] = __ballot_sync(kFull, __shfl_up_sync(kFull, c[a][h], 1) == c[a][h]) & ~1u;
-#pragma unroll
-        for (int qx = 0; qx < 2; ++qx) {
-            const double mx = __dmul_rn(mass, qx ? w[0] : 1.0 - w[0]);
-#pragma unroll
-            for (int qy = 0; qy < 2; ++qy) {
-                const double mxy = __dmul_rn(mx, qy ? w[1] : 1.0 - w[1]);
-                const unsigned sxy = same[0][qx] & same[1][qy];
-                const int row = (c[0][qx] * n + c[1][qy]) * n;
-#pragma unroll
-                for (int qz = 0; qz < 2; ++qz) {
-                    double v = on ? __dmul_rn(mxy, qz ? w[2] : 1.0 - w[2]) : 0.0;
-                    const unsigned s = sxy & same[2][qz];  // lanes that go on a run
-                    // sum each run into its last lane: lane - d is in lane's run
-                    // where lane has d predecessors there
-                    unsigned m = s;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        if (!m) break;  // warp-uniform
-                        const double vu = __shfl_up_sync(kFull, v, d);
-                        if (m >> lane & 1u) v = __dadd_rn(vu, v);
-                        m &= m << d;
-                    }
-                    const bool tail = lane == 31 || !(s >> (lane + 1) & 1u);
-                    if (tail && on) atomicAdd(&mesh[row + c[2][qz]], v);
+        for (int q = 0; q < 8; ++q) {
+            const int ix = (q & 1) ? nb[0] : c[0], iy = (q & 2) ? nb[1] : c[1], iz = (q & 4) ? nb[2] : c[2];
+            const double wx = (q & 1) ? w[0] : 1.0 - w[0], wy = (q & 2) ? w[1] : 1.0 - w[1],
+                         wz = (q & 4) ? w[2] : 1.0 - w[2];
+            const int key = on ? (ix * n + iy) * n + iz : -1;
+            double v = on ? __dmul_rn(__dmul_rn(__dmul_rn(mass, wx), wy), wz) : 0.0;
+            const int prev = __shfl_up_sync(kFull, key, 1), next = __shfl_down_sync(kFull, key, 1);
+            const bool head = lane == 0 || prev != key, tail = lane == 31 || next != key;
+            const unsigned heads = __ballot_sync(kFull, head);
+            if (heads != kFull) {
+                // sum each run of equal keys into its last lane: a scan over
+                // the lanes that adds lane - d only while it is in the run
+                const unsigned upto = heads & (0xffffffffu >> (31 - lane));
+                const int first = 31 - __clz(upto);
+                const int depth = __reduce_max_sync(kFull, (unsigned)(lane - first));
+                for (int d = 1; d <= depth; d <<= 1) {
+                    const double vu = __shfl_up_sync(kFull, v, d);
+                    if (lane - d >= first) v = __dadd_rn(vu, v);
                 }
             }
+            if (tail && key >= 0) atomicAdd(&mesh[key], v);
         }
     }
 }
