@@ -10,7 +10,12 @@
 //     needs half the instructions but a gathered shared-memory load for each
 //     coefficient, whose bank conflicts made it slower (65^3: 12.9 ms);
 //   - near, inside and beyond are decided on the high word of r^2, off the
-//     FP64 pipe; a warp whose pairs are all near, or all beyond, skips the rest;
+//     FP64 pipe; a warp whose pairs are all near, or all beyond, skips the rest.
+//     Half of the instructions are not FP64, and issue and the FP64 pipe are
+//     about equally busy (58% and 54%), so those count too: the decisions by
+//     minima over the lane's pairs, a clamp that runs only where a pair is near
+//     the softening and 32-bit shared addresses took a 65^3 pass from 10.5 to
+//     9.5 ms (33 ms in the general kernel);
 //   - a lane keeps four sinks in registers (the sink-register layout of the
 //     FP32 forms: G = ceil(ns / 4) groups of sinks, J = 32 / G source phases),
 //     so a source read from shared memory serves four independent chains;
@@ -66,6 +71,8 @@ __device__ __forceinline__ double fp64_rsqrt(const double v) {
     return fma(y * h, fma(h, 0.375, 0.5), y);
 }
 
+__device__ __forceinline__ unsigned fp64_hi(const double v) { return (unsigned)__double2hiint(v); }
+
 // One source against the lane's sinks.
 template <int SOFT, bool MASSES, int NF>
 __device__ __forceinline__ void fp64_eval(const double sx, const double sy, const double sz, const double sw,
@@ -73,20 +80,55 @@ __device__ __forceinline__ void fp64_eval(const double sx, const double sy, cons
     constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
     constexpr int N = kFp64Sinks;
     double dx[N], dy[N], dz[N], r2[N];
-    bool near = false, far = false, odd = false;
+    // Which kinds of pair there are, from the least and largest high words: a
+    // minimum of (high word - start of a range) below the range's length says
+    // that one lies in it. Two predicates and a combination a pair and kind, and
+    // a 64-bit maximum a pair for the clamp, were a sixth of the instructions.
+    unsigned least = 0xffffffffu, most = 0u;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         dx[k] = sx - L.px[k];
         dy[k] = sy - L.py[k];
         dz[k] = sz - L.pz[k];
         if (SOFT == SOFT_CLAMP)
-            r2[k] = fmax(fma(dz[k], dz[k], fma(dy[k], dy[k], dx[k] * dx[k])), a.eps2_box);
+            r2[k] = fma(dz[k], dz[k], fma(dy[k], dy[k], dx[k] * dx[k]));
         else
             r2[k] = fma(dz[k], dz[k], fma(dy[k], dy[k], fma(dx[k], dx[k], a.eps2_box)));
-        const unsigned hi = (unsigned)__double2hiint(r2[k]);
-        near = near || hi < F.hi_near;
-        far = far || (hi >= F.hi_near && hi < F.hi_in);
-        odd = odd || (hi >= F.hi_in && (hi <= F.hi_out || hi >= 0x7ff00000u));
+        least = min(least, fp64_hi(r2[k]));
+        most = max(most, fp64_hi(r2[k]));
+    }
+    if (SOFT == SOFT_CLAMP && (least <= fp64_hi(a.eps2_box) || most >= 0x7ff00000u)) {
+        least = 0xffffffffu;
+        most = 0u;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            r2[k] = fmax(r2[k], a.eps2_box);
+            least = min(least, fp64_hi(r2[k]));
+            most = max(most, fp64_hi(r2[k]));
+        }
+    }
+    unsigned past_near = 0xffffffffu, past_in = 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        past_near = min(past_near, fp64_hi(r2[k]) - F.hi_near);
+        past_in = min(past_in, fp64_hi(r2[k]) - F.hi_in);
+    }
+    const bool near = least < F.hi_near, far = past_near < F.hi_in - F.hi_near;
+    if (past_in <= F.hi_out - F.hi_in || most >= 0x7ff00000u) {  // rare
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const unsigned hi = fp64_hi(r2[k]);
+            if (!(hi >= F.hi_in && (hi <= F.hi_out || hi >= 0x7ff00000u))) continue;
+            bool keep;
+            double f = plain_factor<SOFT>(r2[k], a, keep);
+            if (keep) {
+                if (MASSES) f *= sw;
+                L.ax[k] = fma(dx[k], f, L.ax[k]);
+                L.ay[k] = fma(dy[k], f, L.ay[k]);
+                L.az[k] = fma(dz[k], f, L.az[k]);
+            }
+            dx[k] = dy[k] = dz[k] = 0.0;  // (an infinite one times the zero below would be NaN)
+        }
     }
     if (near || far) {
         double y[N], p[N];
@@ -105,8 +147,9 @@ __device__ __forceinline__ void fp64_eval(const double sx, const double sy, cons
                 for (int k = 0; k < N; ++k) q[k] = fma(q[k], r2[k] - F.near_mid, F.near[c]);
 #pragma unroll
             for (int k = 0; k < N; ++k) {
-                const double f = fma(y[k] * y[k], y[k], q[k]);
-                p[k] = (unsigned)__double2hiint(r2[k]) < F.hi_near ? f : 0.0;
+                double f = fma(y[k] * y[k], y[k], q[k]);
+                if (MASSES) f *= sw;
+                p[k] = fp64_hi(r2[k]) < F.hi_near ? f : 0.0;
             }
         }
         if (far) {
@@ -137,31 +180,16 @@ __device__ __forceinline__ void fp64_eval(const double sx, const double sy, cons
                 // 2^n by the exponent field: a far pair's n lies in [-24, -1], so nothing leaves
                 // the normal range; what other lanes make of it is not used
                 e[k] = __hiloint2double(__double2hiint(e[k]) + (n[k] << 20), __double2loint(e[k]));
-                const unsigned hi = (unsigned)__double2hiint(r2[k]);
-                const double v = (y[k] * y[k]) * y[k] * (e[k] * q[k]);
-                p[k] = hi >= F.hi_near && hi < F.hi_in ? v : p[k];
+                double v = (y[k] * y[k]) * y[k] * (e[k] * q[k]);
+                if (MASSES) v *= sw;
+                p[k] = fp64_hi(r2[k]) - F.hi_near < F.hi_in - F.hi_near ? v : p[k];
             }
         }
 #pragma unroll
         for (int k = 0; k < N; ++k) {
-            if (MASSES) p[k] *= sw;
             L.ax[k] = fma(dx[k], p[k], L.ax[k]);
             L.ay[k] = fma(dy[k], p[k], L.ay[k]);
             L.az[k] = fma(dz[k], p[k], L.az[k]);
-        }
-    }
-    if (odd) {  // rare
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            const unsigned hi = (unsigned)__double2hiint(r2[k]);
-            if (!(hi >= F.hi_in && (hi <= F.hi_out || hi >= 0x7ff00000u))) continue;
-            bool keep;
-            double f = plain_factor<SOFT>(r2[k], a, keep);
-            if (!keep) continue;
-            if (MASSES) f *= sw;
-            L.ax[k] = fma(dx[k], f, L.ax[k]);
-            L.ay[k] = fma(dy[k], f, L.ay[k]);
-            L.az[k] = fma(dz[k], f, L.az[k]);
         }
     }
 }
@@ -169,6 +197,12 @@ __device__ __forceinline__ void fp64_eval(const double sx, const double sy, cons
 __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
+}
+
+__device__ __forceinline__ double load_shared(const unsigned at) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+    return v;
 }
 
 // Shared memory of one warp: two chunks of cap / 2 sources (x, y, z and mass
@@ -184,6 +218,7 @@ pair_fp64_kernel(const __grid_constant__ PairArgs a, const __grid_constant__ Fit
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     const int wdoubles = (int)(fp64_warp_bytes(cap) / sizeof(double));
     double *const wbase = smem_d + w * wdoubles;
+    const unsigned wshared = (unsigned)__cvta_generic_to_shared(wbase);
     const int chunk = cap / 2;
     double *const sums = wbase + 4 * (size_t)cap;  // [component and sink][lane]
     __shared__ int s_item;
@@ -278,12 +313,13 @@ pair_fp64_kernel(const __grid_constant__ PairArgs a, const __grid_constant__ Fit
                 const int next = fill(wbase + (b ^ 1) * 4 * chunk);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");
                 __syncwarp();  // every lane's copies of this chunk have landed
-                const double *buf = wbase + b * 4 * chunk;
                 if (jl < J) {
+                    // a 32-bit shared address: a generic pointer's was made anew for every source
+                    const unsigned row = 8u * chunk, buf = wshared + 4u * row * b, end = buf + 8u * n;
 #pragma unroll 1
-                    for (int s = jl; s < n; s += J)
-                        fp64_eval<SOFT, MASSES, NF>(buf[s], buf[chunk + s], buf[2 * chunk + s],
-                                                    MASSES ? buf[3 * chunk + s] : 0.0, L, a, F);
+                    for (unsigned at = buf + 8u * jl; at < end; at += 8u * J)
+                        fp64_eval<SOFT, MASSES, NF>(load_shared(at), load_shared(at + row), load_shared(at + 2 * row),
+                                                    MASSES ? load_shared(at + 3 * row) : 0.0, L, a, F);
                 }
                 __syncwarp();  // the chunk is read before the copies after next overwrite it
                 n = next;

@@ -98,3 +98,23 @@ def test_a_position_that_is_not_finite_gives_what_the_general_kernel_gives(gpu, 
                    pos, ip, npt, tt, ts) for xc in (2.25, 1.2)]  # fitted; general kernel
         assert np.array_equal(np.isnan(out[0]), np.isnan(out[1]))
         assert np.isfinite(out[0][:, 8:]).all()
+
+
+@pytest.mark.parametrize("soft", [abi.SOFT_CLAMP, abi.SOFT_PLUMMER])
+def test_pairs_beyond_the_cutoff_add_nothing(gpu, soft):
+    """Also where the pair's offset or the source's mass is infinite and the
+    lane's other pairs are inside."""
+    pos = np.full((3, 8), 0.5) + 0.01 * np.random.default_rng(2).random((3, 8))
+    pos[2, 1] = np.inf  # a sink
+    pos[0, 6] = 9.0     # a source with an infinite mass
+    m = np.ones(8)
+    m[6] = np.inf
+    ip, npt = np.array([0, 4], np.int32), np.full(2, 4, np.int32)
+    tt, ts = np.array([0], np.int32), np.array([1], np.int32)
+    # (the clamp takes an infinite r^2 for 0 * inf = NaN, in the oracle's arithmetic too)
+    fitted, general = (run(make_params(form=abi.FORM_PLAIN_FP64, soft_mode=soft, soften=0.01, split_radius=0.2,
+                                       x_cut=xc), pos, ip, npt, tt, ts, masses=m) for xc in (2.25, 1.2))
+    assert np.array_equal(np.isnan(fitted), np.isnan(general))
+    for out in (fitted, general):
+        assert np.isfinite(out[:, [0, 2, 3]]).all() and (out[:, [0, 2, 3]] != 0).any(axis=0).all()
+        assert soft == abi.SOFT_CLAMP or (out[:, 1] == 0).all()
