@@ -11,7 +11,7 @@
 //     coefficient, whose bank conflicts made it slower (65^3: 12.9 ms);
 //   - near, inside and beyond are decided on the high word of r^2, off the
 //     FP64 pipe; a warp whose pairs are all near, or all beyond, skips the rest.
-//     Half of the instructions are not FP64, and issue and the FP64 pipe are
+//     Half of the instructions were not FP64, and issue and the FP64 pipe were
 //     about equally busy (58% and 54%), so those count too: the decisions by
 //     minima over the lane's pairs, a clamp that runs only where a pair is near
 //     the softening and 32-bit shared addresses took a 65^3 pass from 10.5 to
