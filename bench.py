@@ -164,15 +164,16 @@ def load_traffic(workload, form_name):
         return None
 
 
-def load_fp64_flops(workload):
-    """FP64 flops per listed pair of the plain form's pair kernel (DFMA x 2 +
-    DADD + DMUL per pair, CUDA's erfc/exp/rsqrt included) from the committed
-    ncu summary, or None."""
+def load_fp64_flops(workload, kernel="plain_fp64"):
+    """FP64 flops per listed pair of a pair kernel of the plain form (DFMA x 2 +
+    DADD + DMUL per pair) from the committed ncu summary, or None: "plain_fp64",
+    the general kernel (CUDA's erfc/exp/rsqrt included), or "pair_fp64", the one
+    for passes with a cutoff."""
     path = os.path.join(REPO, "profiles", "ncu_traffic.json")
     try:
         with open(path) as f:
             d = json.load(f)
-        return d.get(f"{workload}:plain_fp64:fp64_flops_per_pair")
+        return d.get(f"{workload}:{kernel}:fp64_flops_per_pair")
     except (OSError, ValueError):
         return None
 
@@ -191,12 +192,12 @@ def combine_ranks(total_s, e2e_s, pairs, dist, device):
     return float(t[0]), float(t[1]), float(pt[0])
 
 
-def plain_roofline(workload, pairs, kernel_ms, fp64_peak, fp32_peak):
+def plain_roofline(workload, pairs, kernel_ms, fp64_peak, fp32_peak, kernel="plain_fp64"):
     """The plain FP64 form's pair kernel against the measured FP64 and FP32
-    peaks: FP64 flops per pair counted by ncu (the form's own arithmetic
-    calls CUDA's FP64 erfc, exp and rsqrt, so its flops are counted where they
-    execute rather than from the source)."""
-    f64 = load_fp64_flops(workload)
+    peaks: FP64 flops per pair counted by ncu (the general kernel calls CUDA's
+    FP64 erfc, exp and rsqrt, so flops are counted where they execute rather
+    than from the source)."""
+    f64 = load_fp64_flops(workload, kernel)
     if not f64:
         return {"bound": "fp64", "peak": fp64_peak, "unit": "TFLOP/s", "flops_per_pair": None}
     achieved = pairs / (kernel_ms * 1e-3) * f64 / 1e12
@@ -568,7 +569,7 @@ def run_ours(args, rank, world, dist):
             sess.set_params(params_for(cfg, abi.FORM_PLAIN_FP64, mass))
             p_s, p_k, _ = resident_passes(sess, max(1, min(args.steps, 3)), 1)
             plain = {"value": P / float(np.mean(p_s)), "kernel_ms": float(np.mean(p_k))}
-            plain["roofline"] = plain_roofline(args.workload, P, plain["kernel_ms"], fp64_peak, fp32_peak)
+            plain["roofline"] = plain_roofline(args.workload, P, plain["kernel_ms"], fp64_peak, fp32_peak, "pair_fp64")
             loc = tl.tag == 1
             acc_plain = result(sess)
             num = np.linalg.norm(acc_form - acc_plain, axis=0)[loc]
@@ -621,7 +622,7 @@ def run_ours(args, rank, world, dist):
     kernel_pairs_per_s = P / (mean_kernel_ms * 1e-3)
     roofline = None
     if form == abi.FORM_PLAIN_FP64:
-        roofline = plain_roofline(args.workload, P, mean_kernel_ms, fp64_peak, fp32_peak)
+        roofline = plain_roofline(args.workload, P, mean_kernel_ms, fp64_peak, fp32_peak, "pair_fp64")
     if F:
         # flops of the pairs the kernel evaluates (entries wholly beyond the
         # cutoff are skipped: counted in the metric's pairs, not in the flops)
