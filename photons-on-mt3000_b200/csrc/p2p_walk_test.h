@@ -29,6 +29,17 @@ struct alignas(32) WalkBox32 {
 // What becomes of a pair of different boxes.
 enum { WALK_DROP = -1, WALK_OPEN_B = 0, WALK_ACCEPT = 1, WALK_OPEN_A = 2, WALK_UNDECIDED = 3 };
 
+// max(v, 0) that keeps NaN (fmaxf gives 0 and would leave a pair with a NaN gap to
+// its other axes); one instruction on the device.
+P2P_HD float walk_max0(float v) {
+#ifdef __CUDA_ARCH__
+    asm("max.NaN.f32 %0, %0, 0f00000000;" : "+f"(v));
+    return v;
+#else
+    return v < 0.f ? 0.f : v;
+#endif
+}
+
 // The pair (a, b) bounded in FP32: WALK_UNDECIDED unless the exact test's
 // outcome is certain. a_node, b_node: the boxes are nodes (a larger node a is
 // opened before b; a leaf is never opened). cut2, th2: the squares of cutoff
@@ -38,8 +49,10 @@ enum { WALK_DROP = -1, WALK_OPEN_B = 0, WALK_ACCEPT = 1, WALK_OPEN_A = 2, WALK_U
 // sum and product again, so one axis's gap |dist| - width is off by less than
 // slack = 2^-21 (|ca| + |cb| + wa + wb); squares and sums of bounds, and the two
 // constants, by less than 1e-6 of themselves. A gap bounded to be at most zero
-// is zero in the exact test too. NaN decides nothing. An open angle whose square
-// vanishes in FP32 is not 0: th2 is then passed as the smallest normal number.
+// is zero in the exact test too. An open angle whose square vanishes in FP32 is
+// not 0: th2 is then passed as the smallest normal number. A pair with NaN or
+// infinity in either box is undecided: its gap's bounds are NaN on that axis, which
+// walk_max0 keeps, and no comparison with their sums holds.
 P2P_HD int walk_bound(const WalkBox32 &a, const WalkBox32 &b, bool a_node, bool b_node, float cut2, float th2) {
     constexpr float kSlack = 4.76837158e-7f, kUp = 1.0f + 2.0e-6f, kDown = 1.0f - 2.0e-6f;
     float dist[3], w[3], slack[3], lo2 = 0.f, hi2 = 0.f, lo1 = 0.f;
@@ -51,7 +64,7 @@ P2P_HD int walk_bound(const WalkBox32 &a, const WalkBox32 &b, bool a_node, bool 
         w[d] = (a.w[d] + b.w[d]) * 0.5f;
         slack[d] = kSlack * (fabsf(a.c[d]) + fabsf(b.c[d]) + 2.0f * w[d]);
         const float gap = dist[d] - w[d];
-        const float lo = fmaxf(gap - slack[d], 0.f), hi = fmaxf(gap + slack[d], 0.f);
+        const float lo = walk_max0(gap - slack[d]), hi = walk_max0(gap + slack[d]);
         lo1 += lo;
         lo2 += lo * lo;
         hi2 += hi * hi;

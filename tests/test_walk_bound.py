@@ -93,3 +93,51 @@ def test_a_decided_pair_is_decided_as_in_fp64(program, box, angle, offset):
     assert wrong == 0
     if offset <= 1.0 and 1e-6 < box < 1e10:
         assert decided > 0.5 * n
+
+
+# Boxes with one centre or width NaN or infinite: the exact test opens a pair whose
+# gap is NaN (no comparison with NaN holds), so the bound may only leave it to that
+# test; where it decides another pair, it decides the same.
+NONFINITE = SOURCE.split("int main")[0] + r"""
+#include <limits>
+int main() {
+    const double bad[] = {std::numeric_limits<double>::quiet_NaN(), std::numeric_limits<double>::infinity(),
+                          -std::numeric_limits<double>::infinity()};
+    long wrong = 0, n = 0;
+    for (double value : bad)
+        for (int at = 0; at < 12; ++at)            // which number of which box
+            for (int gap = 0; gap < 8; ++gap)      // on which axes the boxes lie apart
+                for (int kinds = 0; kinds < 4; ++kinds)
+                    for (double angle : {0.0, 0.4}) {
+                        WalkBox a, b;
+                        WalkBox32 fa, fb;
+                        for (int d = 0; d < 3; ++d) {
+                            a.c[d] = 0.5;
+                            b.c[d] = 0.5 + (gap >> d & 1 ? 5.0 : 0.0);
+                            a.w[d] = b.w[d] = 0.25;
+                        }
+                        WalkBox &box = at < 6 ? a : b;
+                        (at % 6 < 3 ? box.c : box.w)[at % 3] = value;
+                        a.sum = (a.w[0] + a.w[1]) + a.w[2];
+                        b.sum = (b.w[0] + b.w[1]) + b.w[2];
+                        for (int d = 0; d < 3; ++d) {
+                            fa.c[d] = (float)a.c[d]; fa.w[d] = (float)a.w[d];
+                            fb.c[d] = (float)b.c[d]; fb.w[d] = (float)b.w[d];
+                        }
+                        const bool an = kinds & 1, bn = (kinds & 2) || !an;
+                        const int r = walk_bound(fa, fb, an, bn, 0.01f, (float)(angle * angle));
+                        if (r != WALK_UNDECIDED && (value != value || r != exact(a, b, an, bn, 0.1, angle))) ++wrong;
+                        ++n;
+                    }
+    printf("%ld %ld\n", wrong, n);
+}
+"""
+
+
+def test_a_box_that_is_not_finite_is_left_to_the_exact_test(tmp_path):
+    (tmp_path / "n.cpp").write_text(NONFINITE)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I",
+                           os.path.join(REPO, "photons-on-mt3000_b200", "csrc"), str(tmp_path / "n.cpp"), "-o",
+                           str(tmp_path / "n")])
+    wrong, n = map(int, subprocess.check_output([str(tmp_path / "n")], text=True).split())
+    assert n == 3 * 12 * 8 * 4 * 2 and wrong == 0
