@@ -249,10 +249,10 @@ int default_warps(const p2p_session *s, const p2p_params &p) {
 // The FP64 kernel's blocks share rows among their warps already: 0.144 and 0.097
 // ms at 512 leaves, 0.379 and 0.407 at 2,046.
 constexpr int kRowParts = 4;
-int row_parts(const p2p_session *s) {
+int row_parts(const p2p_session *s, int npart, int nleaf) {
     const p2p_params &p = s->params;
-    if (p.form == P2P_FORM_PLAIN_FP64) return s->fit64.nfar && s->nleaf <= 1000 ? kRowParts : 1;
-    return sink_regs(p) && p.warps_per_leaf == 0 && (int64_t)s->nleaf * s->nleaf <= 900 * (int64_t)s->npart ? kRowParts : 1;
+    if (p.form == P2P_FORM_PLAIN_FP64) return s->fit64.nfar && nleaf <= 1000 ? kRowParts : 1;
+    return sink_regs(p) && p.warps_per_leaf == 0 && (int64_t)nleaf * nleaf <= 900 * (int64_t)npart ? kRowParts : 1;
 }
 
 // Dispatch to the lane mapping's launcher (p2p_pair_*.cu).
@@ -413,7 +413,7 @@ int enqueue_chunk(p2p_session *s, int64_t ntask, const int *d_t, const int *d_s,
 int enqueue_pairs(p2p_session *s, bool timed) {
     CUDA_TRY(cudaMemsetAsync(s->queue, 0, sizeof(int), s->stream));
     PairArgs a = make_args(s);
-    const int parts = row_parts(s);
+    const int parts = row_parts(s, s->npart, s->nleaf);
     const int64_t n3 = 3 * (int64_t)s->npart;
     if (parts > 1) {
         a.acc = (double *)s->parts.p;
@@ -438,6 +438,9 @@ int enqueue_pairs(p2p_session *s, bool timed) {
     return P2P_OK;
 }
 
+// The session's own counts stay as they are: the callers set them once every
+// buffer has its size, so that after a refused begin the result calls still go
+// by the last pass's.
 int size_pass_buffers(p2p_session *s, int npart, int nleaf, bool host_inputs, bool masses) {
     const size_t n3 = 3 * (size_t)npart;
     if (host_inputs) {
@@ -447,9 +450,7 @@ int size_pass_buffers(p2p_session *s, int npart, int nleaf, bool host_inputs, bo
         P2P_TRY(ensure(s, s->leaf_np, sizeof(int) * (size_t)nleaf));
     }
     P2P_TRY(ensure(s, s->acc, sizeof(double) * n3));
-    s->nleaf = nleaf;  // (row_parts)
-    s->npart = npart;
-    if (row_parts(s) > 1) P2P_TRY(ensure(s, s->parts, sizeof(double) * n3 * kRowParts));
+    if (row_parts(s, npart, nleaf) > 1) P2P_TRY(ensure(s, s->parts, sizeof(double) * n3 * kRowParts));
     P2P_TRY(ensure(s, s->meta, sizeof(LeafMeta) * (size_t)nleaf));
     if (is_fp32_form(s->params.form)) P2P_TRY(ensure(s, s->pos4, sizeof(float4) * (size_t)npart));
     P2P_TRY(ensure(s, s->counts, sizeof(int) * (size_t)nleaf));
