@@ -118,6 +118,14 @@ int p2p_session_create(int device, p2p_session **out);
 int p2p_session_destroy(p2p_session *s);
 int p2p_session_set_params(p2p_session *s, const p2p_params *params);
 int p2p_session_get_params(const p2p_session *s, p2p_params *params);
+/* First sizes and bounds of the memory that p2p_pass_submit_walk keeps, and
+ * p2p_fmm_far of far fields created afterwards; 0: the default. list_chunks:
+ * chunks of 64 boxes for the undecided lists of a depth; out_chunks: chunks of
+ * 64 entries for the rows (of 16 for M2L tasks); both at least 16, and doubled
+ * while a walk runs out of them. row_bytes: the most bytes of rows kept while
+ * they are walked (default 8 GB); longer ones are counted first and written by a
+ * second walk. Results do not depend on any of them. */
+int p2p_session_walk_limits(p2p_session *s, int64_t list_chunks, int64_t out_chunks, int64_t row_bytes);
 /* The cudaStream_t (as void*) every launch of this session goes to. */
 void *p2p_session_stream(p2p_session *s);
 /* Degree of the fitted polynomial used by the FP32 forms (0 for FP64). */
@@ -208,8 +216,9 @@ typedef struct p2p_walk_tree {
  * count (device-to-host reads); *ntask (nullable) = list entries. The session
  * keeps the walk's memory between passes: about 100 bytes a node and 150 a leaf,
  * the lists of one depth (about 1 KB a node at first) and the rows (4 bytes an entry and
- * some; pools that turn out too small are doubled and the walk repeated). Rows of
- * more than 8 GB are counted first and written in place by a second walk.
+ * some; pools that turn out too small are doubled and the walk repeated). Rows that
+ * do not fit in 8 GB are counted first and written in place by a second walk
+ * (p2p_session_walk_limits).
  * P2P_ERR_ARG for a child code outside the tree or leaves that are not in
  * pre-order, P2P_ERR_CAPACITY when a box's pending boxes exceed the walk's fixed
  * stack. */

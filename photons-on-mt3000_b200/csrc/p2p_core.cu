@@ -71,6 +71,9 @@ struct DevBuf {
 
 using namespace p2p;
 
+// Chunks a leaf's row is first taken to need in the device walk: 640 entries.
+constexpr int64_t kWalkRowChunks = 10;
+
 struct p2p_session {
     int device = 0;
     int sm_count = 0;
@@ -101,7 +104,8 @@ struct p2p_session {
     // device walk (p2p_pass_submit_walk): box records, active prefix, boxes of
     // two depths, their undecided lists, the rows, counters
     DevBuf walk_box, walk_active, walk_items, walk_lists[2], walk_rows, walk_ctrl;
-    int64_t walk_list_cap = 0, walk_row_cap = 0;  // chunks of the pools
+    int64_t walk_row_chunks = kWalkRowChunks;  // chunks a leaf's row took in the last walk, on average
+    WalkLimits walk_limits;
     // pass state
     bool in_pass = false;
     int npart = 0, nleaf = 0;
@@ -490,6 +494,7 @@ int check_params(const p2p_params *p) { return validate_params(p); }
 void count_launches(int n) { g_launches += n; }
 cudaError_t allow_large_smem() { return allow_smem_all(); }
 int session_device(const p2p_session *s) { return s ? s->device : 0; }
+WalkLimits session_walk_limits(const p2p_session *s) { return s ? s->walk_limits : WalkLimits(); }
 
 void *session_scratch(p2p_session *s, int slot, size_t bytes) {
     if (!s || slot < 0) return nullptr;
@@ -621,6 +626,16 @@ P2P_API int p2p_session_set_params(p2p_session *s, const p2p_params *params) {
 P2P_API int p2p_session_get_params(const p2p_session *s, p2p_params *params) {
     if (!s || !params) return fail(P2P_ERR_ARG, "null argument");
     *params = s->params;
+    return P2P_OK;
+}
+
+P2P_API int p2p_session_walk_limits(p2p_session *s, int64_t list_chunks, int64_t out_chunks, int64_t row_bytes) {
+    if (!s) return fail(P2P_ERR_ARG, "null session");
+    // (a warp takes kWalkGrab chunks of a pool at a time)
+    if ((list_chunks && list_chunks < kWalkGrab) || (out_chunks && out_chunks < kWalkGrab) || row_bytes < 0 ||
+        std::max(list_chunks, out_chunks) > INT32_MAX)
+        return fail(P2P_ERR_ARG, "walk limits: a pool holds at least %d chunks", kWalkGrab);
+    s->walk_limits = WalkLimits{list_chunks, out_chunks, row_bytes};
     return P2P_OK;
 }
 
@@ -847,14 +862,23 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     P2P_TRY(ensure(s, s->walk_active, sizeof(int64_t) * ((size_t)nleaf + 1)));
     P2P_TRY(ensure(s, s->walk_items, sizeof(WalkItem) * 2 * (size_t)nleaf));
     P2P_TRY(ensure(s, s->walk_ctrl, sizeof(WalkCtrl)));
-    // Pools of chunks: the undecided lists of one depth (two pools in turn)
-    // and the rows. Sizes are first guesses; a walk that runs out of one is
-    // repeated with twice the size, which the session keeps. Rows beyond
-    // kWalkPoolBytes are counted first and then written to their places by a
-    // second walk.
+    // Pools of chunks: the undecided lists of one depth (two pools in turn) and
+    // the rows. Sizes are first guesses, or what the session's buffers hold from
+    // earlier walks; a walk that runs out of a pool is repeated with twice the size.
+    // Only the buffers outlive the pass: a size that could not be allocated is
+    // forgotten with it. Rows that the last walk's mean length puts above the
+    // limit, or that grow beyond it, are counted and then written to their places
+    // by a second walk.
+    const WalkLimits &lim = s->walk_limits;
+    const size_t chunk_bytes = walk_pool_bytes(1, kWalkChunk);
     const int64_t slack = walk_pool_slack(s->sm_count);
-    s->walk_list_cap = std::max(s->walk_list_cap, 2 * (int64_t)nnode + slack);
-    s->walk_row_cap = std::max(s->walk_row_cap, 10 * (int64_t)nleaf + slack);
+    const int64_t row_limit = std::min<int64_t>(
+        (int64_t)((lim.row_bytes ? (size_t)lim.row_bytes : kWalkPoolBytes) / chunk_bytes), INT32_MAX);
+    int64_t list_cap = std::max(lim.list_chunks ? lim.list_chunks : 2 * (int64_t)nnode + slack,
+                                (int64_t)(std::min(s->walk_lists[0].cap, s->walk_lists[1].cap) / chunk_bytes));
+    int64_t row_cap = lim.out_chunks ? lim.out_chunks : s->walk_row_chunks * nleaf + slack;
+    bool pooled = row_cap <= row_limit;
+    if (pooled) row_cap = std::max(row_cap, std::min(row_limit, (int64_t)(s->walk_rows.cap / chunk_bytes)));
     const int ntiles = (int)((nleaf + (int64_t)kScanTile - 1) / kScanTile);
     int64_t *row_off = (int64_t *)s->row_off.p, *tile_sums = (int64_t *)s->tile_sums.p;
     int *counts = (int *)s->counts.p, *heads = (int *)s->fill.p;
@@ -877,22 +901,20 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     g.out_len = counts;
     g.row_off = row_off;
     int64_t total = 0;
-    bool pooled = false;
     // one walk (rows into the pool, counted, or written): the row offsets and
     // the total, or an error
     auto walk = [&](bool fill) -> int {
         for (;;) {
-            pooled = !fill && walk_pool_bytes(s->walk_row_cap, kWalkChunk) <= kWalkPoolBytes;
-            P2P_TRY(ensure(s, s->walk_lists[0], walk_pool_bytes(s->walk_list_cap, kWalkChunk)));
-            P2P_TRY(ensure(s, s->walk_lists[1], walk_pool_bytes(s->walk_list_cap, kWalkChunk)));
-            if (pooled) P2P_TRY(ensure(s, s->walk_rows, walk_pool_bytes(s->walk_row_cap, kWalkChunk)));
+            P2P_TRY(ensure(s, s->walk_lists[0], walk_pool_bytes(list_cap, kWalkChunk)));
+            P2P_TRY(ensure(s, s->walk_lists[1], walk_pool_bytes(list_cap, kWalkChunk)));
+            if (pooled && ensure(s, s->walk_rows, walk_pool_bytes(row_cap, kWalkChunk)) != P2P_OK) pooled = false;
             g.box = (const WalkBox *)s->walk_box.p;
             g.box32 = (const WalkBox32 *)(g.box + nbox);
             g.active = (const int64_t *)s->walk_active.p;
             g.items[0] = (WalkItem *)s->walk_items.p;
             g.items[1] = g.items[0] + nleaf;
-            for (int k = 0; k < 2; ++k) g.lists[k] = walk_pool(s->walk_lists[k].p, s->walk_list_cap, kWalkChunk);
-            if (pooled) g.out = walk_pool(s->walk_rows.p, s->walk_row_cap, kWalkChunk);
+            for (int k = 0; k < 2; ++k) g.lists[k] = walk_pool(s->walk_lists[k].p, list_cap, kWalkChunk);
+            if (pooled) g.out = walk_pool(s->walk_rows.p, row_cap, kWalkChunk);
             g.row_src = (int *)s->row_src.p;
             g.ctrl = (WalkCtrl *)s->walk_ctrl.p;
             CUDA_TRY(cudaMemsetAsync(g.ctrl, 0, sizeof(WalkCtrl), s->stream));
@@ -928,17 +950,21 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
                 return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
             }
             if (!st) return P2P_OK;
-            if (st & ST_WALK_LISTS) s->walk_list_cap *= 2;
-            if (st & ST_WALK_OUT) s->walk_row_cap *= 2;
-            if (std::max(s->walk_list_cap, s->walk_row_cap) > INT32_MAX)
-                return fail(P2P_ERR_CAPACITY, "walk: more lists than a pool can hold");
+            if (st & ST_WALK_LISTS) list_cap *= 2;
+            if (list_cap > INT32_MAX) return fail(P2P_ERR_CAPACITY, "walk: more lists than a pool can hold");
+            if (st & ST_WALK_OUT) {
+                pooled = row_cap < row_limit;
+                row_cap = std::min(2 * row_cap, row_limit);
+            }
         }
     };
     P2P_TRY(walk(false));
+    const bool chains = pooled;
+    s->walk_row_chunks = std::max<int64_t>(kWalkRowChunks, total / kWalkChunk / nleaf + 2);
     if (ntask) *ntask = total;
     if (total == 0) return P2P_OK;
     P2P_TRY(ensure(s, s->row_src, sizeof(int) * (size_t)total));
-    const bool skip = skips_outside(s), chains = pooled;
+    const bool skip = skips_outside(s);
     if (!chains) P2P_TRY(walk(true));
     const double cscale = 0.5 / s->params.split_radius;
     const float uout = (float)(s->fit.umax * (1.0 + kCutBand) * (1.0 + kOutsideMargin));

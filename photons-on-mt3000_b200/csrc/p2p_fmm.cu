@@ -401,7 +401,7 @@ struct p2p_fmm {
     cudaStream_t stream = nullptr;
     DevBufF parents, leafM, nodeM, sinkL, leafL, counts, ctrl;
     DevBufF box, items, lists[2], tasks, walk_ctrl;  // the M2L walk
-    int64_t list_cap = 0, task_cap = 0;              // chunks of its pools
+    WalkLimits limits;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     long long n_m2l = 0, n_applied = 0;
     int levels = 0, nleaf = 0, nnode = 0;
@@ -425,6 +425,7 @@ P2P_API int p2p_fmm_create(p2p_session *s, p2p_fmm **out) {
     p2p_fmm *f = new p2p_fmm();
     f->device = session_device(s);
     f->stream = (cudaStream_t)p2p_session_stream(s);
+    f->limits = session_walk_limits(s);
     for (cudaEvent_t &e : f->ev) {
         if (cudaEventCreate(&e) != cudaSuccess) {
             cudaGetLastError();
@@ -521,8 +522,9 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     FMM_CUDA(cudaEventRecord(f->ev[1], st), "FMM upward");
 
     // M2L walk, one depth of sinks per launch: every sink's tasks into a pool
-    // of chunks (sizes are first guesses: a walk that runs out of one is
-    // repeated with twice the size)
+    // of chunks (sizes are first guesses, or what the buffers hold from earlier
+    // walks: a walk that runs out of one is repeated with twice the size; only the
+    // buffers outlive the call)
     int *head = (int *)f->counts.p, *len = head + nsink;
     FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
     WalkRun g;
@@ -532,8 +534,10 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
         int sms = 0;
         FMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device), "FMM walk");
         const int64_t slack = walk_pool_slack(sms);
-        f->list_cap = std::max(f->list_cap, 2 * (int64_t)nnode + slack);
-        f->task_cap = std::max(f->task_cap, 3 * (int64_t)nsink / 2 + slack);
+        int64_t list_cap = std::max(f->limits.list_chunks ? f->limits.list_chunks : 2 * (int64_t)nnode + slack,
+                                    (int64_t)(std::min(f->lists[0].cap, f->lists[1].cap) / walk_pool_bytes(1, kWalkChunk)));
+        int64_t task_cap = std::max(f->limits.out_chunks ? f->limits.out_chunks : 3 * (int64_t)nsink / 2 + slack,
+                                    (int64_t)(f->tasks.cap / walk_pool_bytes(1, kWalkTaskChunk)));
         g.nnode = nnode;
         g.nleaf = nleaf;
         g.node_first = t->node_first;
@@ -555,11 +559,11 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
         for (bool again = true; again;) {
             again = false;
             for (int k = 0; k < 2; ++k) {
-                FMM_TRY(grow(f->lists[k], walk_pool_bytes(f->list_cap, kWalkChunk)));
-                g.lists[k] = walk_pool(f->lists[k].p, f->list_cap, kWalkChunk);
+                FMM_TRY(grow(f->lists[k], walk_pool_bytes(list_cap, kWalkChunk)));
+                g.lists[k] = walk_pool(f->lists[k].p, list_cap, kWalkChunk);
             }
-            FMM_TRY(grow(f->tasks, walk_pool_bytes(f->task_cap, kWalkTaskChunk)));
-            g.out = walk_pool(f->tasks.p, f->task_cap, kWalkTaskChunk);
+            FMM_TRY(grow(f->tasks, walk_pool_bytes(task_cap, kWalkTaskChunk)));
+            g.out = walk_pool(f->tasks.p, task_cap, kWalkTaskChunk);
             FMM_CUDA(cudaMemsetAsync(g.ctrl, 0, sizeof(WalkCtrl), st), "FMM walk");
             walk_pack_kernel<true><<<blocks_for((long long)nnode + nleaf, threads), threads, 0, st>>>(
                 a.w, (WalkBox *)f->box.p, (WalkBox32 *)((WalkBox *)f->box.p + nbox), nullptr, g.items[0], g.lists[0].ids, g.ctrl);
@@ -579,9 +583,9 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
                 if (status & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
                 if (status & ST_WALK_STACK) return report_error(P2P_ERR_CAPACITY, "FMM walk: stack exceeded");
                 if (status) {
-                    if (status & ST_WALK_LISTS) f->list_cap *= 2;
-                    if (status & ST_WALK_OUT) f->task_cap *= 2;
-                    if (std::max(f->list_cap, f->task_cap) > INT32_MAX)
+                    if (status & ST_WALK_LISTS) list_cap *= 2;
+                    if (status & ST_WALK_OUT) task_cap *= 2;
+                    if (std::max(list_cap, task_cap) > INT32_MAX)
                         return report_error(P2P_ERR_CAPACITY, "FMM walk: more lists than a pool can hold");
                     FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
                     again = true;

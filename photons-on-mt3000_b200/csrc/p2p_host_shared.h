@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 #include "photons_p2p.h"
 
 namespace p2p {
@@ -17,6 +19,12 @@ void count_launches(int n);
 cudaError_t allow_large_smem();
 // The CUDA device of a session.
 int session_device(const p2p_session *s);
+// First sizes and bounds of the device walks (p2p_session_walk_limits); 0: the default.
+struct WalkLimits {
+    int64_t list_chunks = 0, out_chunks = 0;  // of the undecided lists; of the rows or tasks
+    int64_t row_bytes = 0;                    // most bytes of rows kept while walking
+};
+WalkLimits session_walk_limits(const p2p_session *s);
 // Device scratch the session keeps between calls: slot k holds at least
 // bytes (grown when smaller, after the session's stream has drained;
 // nullptr with p2p_last_error set when allocation fails). Freed with the
