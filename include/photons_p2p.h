@@ -215,8 +215,9 @@ typedef struct p2p_walk_tree {
  * Within an open pass (its leaves are the tree's leaves). Waits for the row
  * count (device-to-host reads); *ntask (nullable) = list entries. The session
  * keeps the walk's memory between passes: about 100 bytes a node and 150 a leaf,
- * the lists of one depth (about 1 KB a node at first) and the rows (4 bytes an entry and
- * some; pools that turn out too small are doubled and the walk repeated). Rows that
+ * the lists of one depth (at first about 1 KB a node, 8 KB a leaf up to 40 MB) and the
+ * rows (at first 2.6 KB a leaf, 4 KB a leaf up to 20 MB; pools that turn out too small
+ * are doubled and the walk repeated). Rows that
  * do not fit in 8 GB are counted first and written in place by a second walk
  * (p2p_session_walk_limits).
  * P2P_ERR_ARG for a child code outside the tree or leaves that are not in

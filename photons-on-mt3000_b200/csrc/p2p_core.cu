@@ -871,7 +871,7 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     // by a second walk.
     const WalkLimits &lim = s->walk_limits;
     const size_t chunk_bytes = walk_pool_bytes(1, kWalkChunk);
-    const int64_t slack = walk_pool_slack(s->sm_count);
+    const int64_t slack = walk_pool_slack(s->sm_count, nleaf);
     const int64_t row_limit = std::min<int64_t>(
         (int64_t)((lim.row_bytes ? (size_t)lim.row_bytes : kWalkPoolBytes) / chunk_bytes), INT32_MAX);
     int64_t list_cap = std::max(lim.list_chunks ? lim.list_chunks : 2 * (int64_t)nnode + slack,

@@ -533,10 +533,9 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     if (nnode) {
         int sms = 0;
         FMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device), "FMM walk");
-        const int64_t slack = walk_pool_slack(sms);
-        int64_t list_cap = std::max(f->limits.list_chunks ? f->limits.list_chunks : 2 * (int64_t)nnode + slack,
+        int64_t list_cap = std::max(f->limits.list_chunks ? f->limits.list_chunks : 2 * (int64_t)nnode + walk_pool_slack(sms, nleaf),
                                     (int64_t)(std::min(f->lists[0].cap, f->lists[1].cap) / walk_pool_bytes(1, kWalkChunk)));
-        int64_t task_cap = std::max(f->limits.out_chunks ? f->limits.out_chunks : 3 * (int64_t)nsink / 2 + slack,
+        int64_t task_cap = std::max(f->limits.out_chunks ? f->limits.out_chunks : 3 * (int64_t)nsink / 2 + walk_pool_slack(sms, nsink),
                                     (int64_t)(f->tasks.cap / walk_pool_bytes(1, kWalkTaskChunk)));
         g.nnode = nnode;
         g.nleaf = nleaf;

@@ -506,10 +506,15 @@ walk_gather_kernel(const int *__restrict__ len, const int *__restrict__ head, co
 
 // ------------------------------------------------------------- launching ---
 
+// Blocks of a launch: a depth has at most one box per leaf.
+inline int walk_blocks(int sm_count, int boxes) {
+    return std::min(sm_count * 8, (boxes + kWalkWarps - 1) / kWalkWarps);
+}
+
 // Enqueues depths [lv, lv + n) of a walk.
 template <int MODE>
 inline cudaError_t walk_depths(cudaStream_t st, const WalkRun &g, int sm_count, int lv, int n) {
-    const int blocks = min(sm_count * 8, (g.nleaf + kWalkWarps - 1) / kWalkWarps);
+    const int blocks = walk_blocks(sm_count, g.nleaf);
     for (int l = lv; l < lv + n; ++l) walk_level_kernel<MODE><<<blocks, kWalkWarps * 32, 0, st>>>(g, l);
     return cudaGetLastError();
 }
@@ -530,7 +535,10 @@ inline size_t walk_pool_bytes(int64_t cap, int chunk) { return (size_t)cap * (si
 inline WalkPool walk_pool(void *p, int64_t cap, int chunk) {
     return WalkPool{(int *)p, (int *)p + (size_t)cap * chunk, (int)cap};
 }
-// Chunks that warps hold without having used them.
-inline int64_t walk_pool_slack(int sm_count) { return (int64_t)sm_count * 8 * kWalkWarps * kWalkGrab; }
+// Chunks that warps hold without having used them, for `boxes` boxes with lists:
+// 16 a box, 75,776 (20 MB of lists) where they fill the GPU.
+inline int64_t walk_pool_slack(int sm_count, int boxes) {
+    return (int64_t)walk_blocks(sm_count, boxes) * kWalkWarps * kWalkGrab;
+}
 
 }  // namespace p2p

@@ -89,3 +89,23 @@ def test_far_field_does_not_depend_on_the_pools(gpu):
     assert out[0][1] > 0 and np.abs(out[0][0]).max() > 0
     for o in out[1:]:
         assert o[1:] == out[0][1:] and np.array_equal(o[0], out[0][0])
+
+
+def test_a_small_trees_walk_takes_little_memory(gpu):
+    """500 leaves: the pools take some 8 MB for the lists and 5 for the rows, where
+    pools for a GPU full of warps took 74."""
+    import torch
+
+    g = np.random.default_rng(1)
+    with L.Tree(g.random((3, 4500)), np.ones(4500, np.int32), 16, 1.0) as tree:
+        assert 300 < tree.nleaf < 700
+        dev = DeviceWalkTree(tree, f"cuda:{gpu}")
+        used = []
+        for _ in range(2):  # (the first loads the kernels)
+            with Session(gpu, params_for(W.c1_config(), abi.FORM_SPLIT, 1.0)) as s:
+                s.begin(tree.pos, tree.leaf_ipart, tree.leaf_npart)
+                before = torch.cuda.mem_get_info(gpu)[0]
+                s.submit_walk(dev, 0.1, 0.0)
+                used.append(before - torch.cuda.mem_get_info(gpu)[0])
+                s.end()
+    assert used[1] < 40e6
