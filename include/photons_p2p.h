@@ -124,8 +124,11 @@ int p2p_session_get_params(const p2p_session *s, p2p_params *params);
  * 64 entries for the rows (of 16 for M2L tasks); both at least 16, and doubled
  * while a walk runs out of them. row_bytes: the most bytes of rows kept while
  * they are walked (default 8 GB); longer ones are counted first and written by a
- * second walk. Results do not depend on any of them. */
-int p2p_session_walk_limits(p2p_session *s, int64_t list_chunks, int64_t out_chunks, int64_t row_bytes);
+ * second walk. depths: of a tree that is walked by depth (default 18 more than a
+ * balanced tree of its leaves has, at most 96); a deeper one is walked by sink leaf.
+ * The rows do not depend on any of them, nor the M2L tasks; a far field by sink leaf
+ * sums a box's tasks in another order. */
+int p2p_session_walk_limits(p2p_session *s, int64_t list_chunks, int64_t out_chunks, int64_t row_bytes, int depths);
 /* The cudaStream_t (as void*) every launch of this session goes to. */
 void *p2p_session_stream(p2p_session *s);
 /* Degree of the fitted polynomial used by the FP32 forms (0 for FP64). */
@@ -220,9 +223,10 @@ typedef struct p2p_walk_tree {
  * are doubled and the walk repeated). Rows that
  * do not fit in 8 GB are counted first and written in place by a second walk
  * (p2p_session_walk_limits).
+ * Trees far deeper than a balanced one (many particles at one point) are walked by
+ * sink leaf, rows counted and then written, with stacks of 80 MB at first.
  * P2P_ERR_ARG for a child code outside the tree or leaves that are not in
- * pre-order, P2P_ERR_CAPACITY when a box's pending boxes exceed the walk's fixed
- * stack. */
+ * pre-order. */
 int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *tree, double cutoff, double open_angle,
                          int64_t *ntask);
 /* ---- Device kd-tree (no counterpart in the reference's GPU code) --------

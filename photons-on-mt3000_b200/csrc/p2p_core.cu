@@ -629,13 +629,14 @@ P2P_API int p2p_session_get_params(const p2p_session *s, p2p_params *params) {
     return P2P_OK;
 }
 
-P2P_API int p2p_session_walk_limits(p2p_session *s, int64_t list_chunks, int64_t out_chunks, int64_t row_bytes) {
+P2P_API int p2p_session_walk_limits(p2p_session *s, int64_t list_chunks, int64_t out_chunks, int64_t row_bytes,
+                                    int depths) {
     if (!s) return fail(P2P_ERR_ARG, "null session");
     // (a warp takes kWalkGrab chunks of a pool at a time)
     if ((list_chunks && list_chunks < kWalkGrab) || (out_chunks && out_chunks < kWalkGrab) || row_bytes < 0 ||
-        std::max(list_chunks, out_chunks) > INT32_MAX)
+        depths < 0 || std::max(list_chunks, out_chunks) > INT32_MAX)
         return fail(P2P_ERR_ARG, "walk limits: a pool holds at least %d chunks", kWalkGrab);
-    s->walk_limits = WalkLimits{list_chunks, out_chunks, row_bytes};
+    s->walk_limits = WalkLimits{list_chunks, out_chunks, row_bytes, depths};
     return P2P_OK;
 }
 
@@ -827,7 +828,7 @@ P2P_API int p2p_pass_end(p2p_session *s, double *gpu_seconds) {
     if (status & ST_LEAF_RANGE) return fail(P2P_ERR_RANGE, "a leaf range lies outside the particles");
     if (status & ST_TASK_RANGE) return fail(P2P_ERR_RANGE, "a task entry names a leaf outside [0, nleaf)");
     if (status & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
-    if (status & (ST_WALK_STACK | ST_WALK_ROW)) return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
+    if (status & ST_WALK_ROW) return fail(P2P_ERR_CAPACITY, "walk: a row came out otherwise than it was counted");
     return P2P_OK;
 }
 
@@ -901,12 +902,21 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
     g.out_len = counts;
     g.row_off = row_off;
     int64_t total = 0;
+    const int depths = lim.depths ? std::min(lim.depths, kWalkLevels) : walk_first_depths(nleaf) + kWalkExtraDepths;
+    bool by_sink = false;  // a deep tree (walk_sink_kernel; rows are counted, then written)
+    int stack_cap = kWalkSinkStack;
     // one walk (rows into the pool, counted, or written): the row offsets and
     // the total, or an error
     auto walk = [&](bool fill) -> int {
         for (;;) {
-            P2P_TRY(ensure(s, s->walk_lists[0], walk_pool_bytes(list_cap, kWalkChunk)));
-            P2P_TRY(ensure(s, s->walk_lists[1], walk_pool_bytes(list_cap, kWalkChunk)));
+            const int sink_blocks = walk_sink_blocks(s->sm_count, nleaf, stack_cap);
+            if (by_sink) {
+                P2P_TRY(ensure(s, s->walk_lists[0], walk_sink_bytes(sink_blocks, stack_cap)));
+                P2P_TRY(ensure(s, s->walk_lists[1], sizeof(int) * ((size_t)nnode + nleaf)));
+            } else {
+                P2P_TRY(ensure(s, s->walk_lists[0], walk_pool_bytes(list_cap, kWalkChunk)));
+                P2P_TRY(ensure(s, s->walk_lists[1], walk_pool_bytes(list_cap, kWalkChunk)));
+            }
             if (pooled && ensure(s, s->walk_rows, walk_pool_bytes(row_cap, kWalkChunk)) != P2P_OK) pooled = false;
             g.box = (const WalkBox *)s->walk_box.p;
             g.box32 = (const WalkBox32 *)(g.box + nbox);
@@ -925,12 +935,19 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
             scan(heads, (int64_t *)s->walk_active.p);  // (the flags, before the heads take their place)
             int st = 0, left = 0;
             for (int lv = 0, n = walk_first_depths(nleaf);; n = 4) {
-                n = std::min(n, kWalkLevels - lv);
-                if (n <= 0) return fail(P2P_ERR_CAPACITY, "walk: more than %d depths", kWalkLevels);
-                CUDA_TRY(fill ? walk_depths<WALK_FILL>(s->stream, g, s->sm_count, lv, n)
-                         : pooled ? walk_depths<WALK_ROWS>(s->stream, g, s->sm_count, lv, n)
-                                  : walk_depths<WALK_COUNT>(s->stream, g, s->sm_count, lv, n));
-                launch_count(n);
+                n = by_sink ? 1 : std::min(n, depths - lv);
+                if (by_sink) {
+                    int *refs = (int *)s->walk_lists[1].p;
+                    int2 *stacks = (int2 *)s->walk_lists[0].p;
+                    CUDA_TRY(fill ? walk_sinks<WALK_FILL>(s->stream, g, w.son, refs, sink_blocks, stacks, stack_cap, nullptr)
+                                  : walk_sinks<WALK_COUNT>(s->stream, g, w.son, refs, sink_blocks, stacks, stack_cap, nullptr));
+                    launch_count(2);
+                } else {
+                    CUDA_TRY(fill ? walk_depths<WALK_FILL>(s->stream, g, s->sm_count, lv, n)
+                             : pooled ? walk_depths<WALK_ROWS>(s->stream, g, s->sm_count, lv, n)
+                                      : walk_depths<WALK_COUNT>(s->stream, g, s->sm_count, lv, n));
+                    launch_count(n);
+                }
                 lv += n;
                 if (!fill) scan(counts, row_off);
                 CUDA_TRY(cudaGetLastError());
@@ -938,16 +955,27 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
                 CUDA_TRY(cudaMemcpyAsync(&left, &g.ctrl->items[lv], sizeof(int), cudaMemcpyDeviceToHost, s->stream));
                 CUDA_TRY(cudaMemcpyAsync(&st, &g.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
                 CUDA_TRY(cudaStreamSynchronize(s->stream));
-                if (st || left == 0) break;
+                if (st || by_sink || left == 0 || lv == depths) break;
             }
-            const int bad = st & (ST_WALK_TREE | ST_WALK_STACK | ST_WALK_ROW);
+            const int bad = st & (ST_WALK_TREE | ST_WALK_ROW);
             if (bad) {  // closing the pass reports it too
                 int main_status = 0;
                 CUDA_TRY(cudaMemcpy(&main_status, s->status, sizeof(int), cudaMemcpyDeviceToHost));
                 main_status |= bad;
                 CUDA_TRY(cudaMemcpy(s->status, &main_status, sizeof(int), cudaMemcpyHostToDevice));
                 if (bad & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
-                return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
+                return fail(P2P_ERR_CAPACITY, "walk: a row came out otherwise than it was counted");
+            }
+            if (by_sink) {
+                if (!st) return P2P_OK;
+                if (stack_cap > (1 << 28)) return fail(P2P_ERR_CAPACITY, "walk: a sink's walk exceeded its stack");
+                stack_cap *= 2;
+                continue;
+            }
+            if ((st & ST_WALK_STACK) || (!st && left != 0)) {
+                by_sink = true;
+                pooled = false;
+                continue;
             }
             if (!st) return P2P_OK;
             if (st & ST_WALK_LISTS) list_cap *= 2;

@@ -23,6 +23,7 @@ int session_device(const p2p_session *s);
 struct WalkLimits {
     int64_t list_chunks = 0, out_chunks = 0;  // of the undecided lists; of the rows or tasks
     int64_t row_bytes = 0;                    // most bytes of rows kept while walking
+    int depths = 0;                           // of a walk by depth
 };
 WalkLimits session_walk_limits(const p2p_session *s);
 // Device scratch the session keeps between calls: slot k holds at least

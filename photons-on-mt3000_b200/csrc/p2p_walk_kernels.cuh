@@ -26,6 +26,9 @@
 // opened boxes replaced by their children. Rows come out sorted and equal those
 // the list path builds, entry for entry, with no sort (20 ms at 256^3).
 //
+// A tree much deeper than a balanced one, or one whose opened boxes outgrow a
+// warp's stack, is walked by sink leaf instead (walk_sink_kernel).
+//
 // Lists are chains of chunks of a pool, as their lengths are not known before
 // they are made. The acceptance arithmetic is written with explicitly rounded
 // FP64 operations (no contraction), the ISO C evaluation of the reference's
@@ -51,7 +54,7 @@ struct WalkArgs {
 };
 
 enum : int {
-    ST_WALK_STACK = 4,    // a box's opened boxes exceeded the walk's stack
+    ST_WALK_STACK = 4,    // a warp's opened boxes exceeded its stack (the host walks by sink leaf, or enlarges that walk's)
     ST_WALK_ROW = 8,      // a row came out longer than it was counted (or, in the FMM, offsets out of order)
     ST_WALK_TREE = 16,    // a child code outside the tree, leaves not in pre-order, or a walk longer than any tree allows
     ST_WALK_LISTS = 32,   // the pool of undecided lists is full (the host enlarges it and repeats the walk)
@@ -113,7 +116,11 @@ constexpr int kWalkStack = 1024;   // opened boxes per warp (shared memory)
 constexpr int kWalkChunk = 64;     // ids per chunk of a list of undecided boxes or of a row
 constexpr int kWalkTaskChunk = 16; // ids per chunk of a sink's M2L tasks (about 10 at open angle 0.4)
 constexpr int kWalkGrab = 16;      // chunks a warp takes from a pool at a time
-constexpr int kWalkLevels = 4096;  // most depths of a walk
+constexpr int kWalkLevels = 96;    // most depths of a walk by depth
+// Depths beyond walk_first_depths before a tree is walked by sink leaf. Clustered
+// particles need none; 20^3 particles, 48 of them at one point, take 1.3 ms by depth
+// and 0.6 by sink leaf, 300 of them 3.5 ms by sink leaf after what this many depths took.
+constexpr int kWalkExtraDepths = 12;
 
 // A sink-side box to be walked at a depth.
 struct WalkItem {
@@ -452,6 +459,178 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8) walk_level_kernel(const Wa
     }
 }
 
+// ---------------------------------------------------------- deep trees ---
+//
+// By depth, a leaf's warp follows what it opens alone while the next depth waits,
+// and decided leaves wait on the stack for the open boxes before them. Particles at
+// one point make a chain of splits that each peel off one particle: D depths of up
+// to D - d steps each, and up to D leaves waiting. Such trees are walked by sink
+// leaf: one warp per leaf L takes the pairs (A, B) from (root, root) that lead to
+// L's entries, A on L's path, so no leaf waits for another, with a stack in global
+// memory that the host enlarges as needed. Each pair is tested again for every
+// leaf below A (7.6 ms for 128^3 clustered particles, 3.1 by depth).
+
+// Whether every box is the child of one node at most, and the root of none: what
+// the walk meets from the root then ends, whatever the codes.
+static __global__ void __launch_bounds__(256)
+walk_refs_kernel(const int *__restrict__ son, int nnode, int nleaf, int *__restrict__ refs, WalkCtrl *ctrl) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * nnode; i += gridDim.x * blockDim.x) {
+        const int c = son[i];
+        if (c < 0 || ((c & 1) ? (c >> 1) >= nnode : (c >> 1) >= nleaf)) continue;  // reported where it is met
+        if (c == 1 || atomicAdd(&refs[(c & 1) ? nleaf + (c >> 1) : c >> 1], 1) > 0)
+            atomicOr(&ctrl->status, ST_WALK_TREE);
+    }
+}
+
+// MODE: WALK_COUNT, WALK_FILL (rows in leaf order, as walk_level_kernel) or
+// WALK_M2L (a box's tasks belong to the warp of its first leaf, which appends them
+// one by one in the order of its walk; tail: per sink, its last chunk).
+// Stacks: cap pairs per warp. Pairs lie on the stack in leaf order of B, whose
+// subtrees do not overlap, the first on top.
+template <int MODE>
+__global__ void __launch_bounds__(kWalkWarps * 32)
+walk_sink_kernel(const WalkRun g, int2 *stacks, int cap, int *__restrict__ tail) {
+    constexpr bool M2L = MODE == WALK_M2L;
+    const int lane = threadIdx.x & 31, warp = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
+    const unsigned lt = (1u << lane) - 1u, above = ~(lt | (1u << lane));
+    int2 *stk = stacks + (size_t)warp * cap;
+    int fault = 0, depths = 0;
+    unsigned long long ntask = 0;
+    auto valid = [&](int c) { return c >= 0 && ((c & 1) ? (c >> 1) < g.nnode : (c >> 1) < g.nleaf); };
+    auto first_leaf = [&](int c) { return (c & 1) ? g.node_first[c >> 1] : c >> 1; };
+    for (int L = warp; L < g.nleaf && !g.ctrl->status; L += gridDim.x * kWalkWarps) {
+        if (!M2L && g.active[L + 1] == g.active[L]) continue;  // (its count is 0)
+        const int64_t row = MODE == WALK_FILL ? g.row_off[L] : 0;
+        const int room = MODE == WALK_FILL ? (int)(g.row_off[L + 1] - row) : 0;
+        // the child of a node on L's path that leads on to L (-1: none)
+        auto toward = [&](const int son[2]) {
+            const int s0 = son[0], s1 = son[1];
+            int c = s0;
+            if (s1 >= 0 || !M2L) {  // (the M2L walk passes over absent children)
+                if (!valid(s1)) return -1;
+                if (s0 < 0 || L >= first_leaf(s1)) c = s1;
+            }
+            return valid(c) && ((c & 1) || c >> 1 == L) ? c : -1;
+        };
+        if (lane == 0) stk[0] = make_int2(1, 1);
+        __syncwarp();
+        int sp = 1, emitted = 0;
+        while (sp > 0) {
+            const int ns = min(32, sp);
+            int2 v = make_int2(0, 0);
+            if (lane < ns) v = stk[sp - 1 - lane];
+            __syncwarp();  // the pairs are read before others are put in their places
+            sp -= ns;
+            const int A = v.x;
+            int B = v.y, cls = 0;  // 0 dropped, 1 decided, 2 opened
+            int nc = 0, ca = A, c0 = -1, c1 = -1;  // the opened pair's nc pairs: (ca, c0), (ca, c1)
+            bool task = false;
+            if (lane < ns) {
+                if (B < 0) {  // decided before
+                    B = ~B;
+                    cls = 1;
+                } else if (!(A & 1) && !(B & 1)) {
+                    cls = M2L ? 0 : 1;
+                } else {
+                    const WalkBox32 a = walk_load(g.box32 + A), b = walk_load(g.box32 + B);
+                    int t = WALK_OPEN_B;
+                    if (A != B) {
+                        t = walk_bound(a, b, A & 1, B & 1, g.cut2, g.th2);
+                        if (t == WALK_UNDECIDED) t = walk_exact(g.box, A, B, g.cutoff, g.open_angle);
+                    }
+                    task = M2L && t == WALK_ACCEPT && first_leaf(A) == L;
+                    if (t == WALK_OPEN_A || A == B) {
+                        ca = toward(a.son);
+                        if (ca < 0) fault = ST_WALK_TREE;
+                    }
+                    if (t == WALK_OPEN_A) {
+                        cls = 2;
+                        nc = 1;
+                        c0 = B;
+                    } else if (t == WALK_OPEN_B) {  // (A, A) is opened on both sides
+                        cls = 2;
+                        c0 = b.son[0];
+                        c1 = b.son[1];
+                        const bool v0 = valid(c0), v1 = valid(c1);
+                        if ((!v0 && (!M2L || c0 >= 0)) || (!v1 && (!M2L || c1 >= 0))) fault = ST_WALK_TREE;
+                        if (!v0) c0 = c1;
+                        nc = (v0 ? 1 : 0) + (v1 ? 1 : 0);
+                    }
+                }
+            }
+            const unsigned open = __ballot_sync(kFull, cls == 2), done = __ballot_sync(kFull, cls == 1);
+            const unsigned ready = !open ? kFull : (open & (0u - open)) - 1u;
+            if (M2L) {
+                for (unsigned m = __ballot_sync(kFull, task); m; m &= m - 1u) {
+                    const int from = __ffs(m) - 1;
+                    const int a = __shfl_sync(kFull, A, from), b = __shfl_sync(kFull, B, from);
+                    if (lane == 0 && !fault) {
+                        const int s = (a & 1) ? g.nleaf + (a >> 1) : a >> 1, n = g.out_len[s];
+                        int c;
+                        if (n % kWalkTaskChunk) {
+                            c = tail[s];
+                        } else {
+                            c = atomicAdd(&g.ctrl->out, 1);
+                            if (c < 0 || c >= g.out.cap) {
+                                fault = ST_WALK_OUT;
+                            } else {
+                                if (n == 0) g.out_head[s] = c;
+                                else g.out.next[tail[s]] = c;
+                                tail[s] = c;
+                            }
+                        }
+                        if (!fault) {
+                            g.out.ids[(size_t)c * kWalkTaskChunk + n % kWalkTaskChunk] = b;
+                            g.out_len[s] = n + 1;
+                            ++ntask;
+                        }
+                    }
+                }
+            } else {
+                const unsigned m = done & ready;
+                if (MODE == WALK_FILL && (m >> lane & 1u)) {
+                    const int slot = emitted + __popc(m & lt);
+                    if (slot < room) g.row_src[row + slot] = B >> 1;
+                    else fault = ST_WALK_ROW;
+                }
+                emitted += __popc(m);
+            }
+            // the others back on the stack, the first on top
+            const unsigned back = done & ~ready;
+            const unsigned one = __ballot_sync(kFull, nc >= 1), two = __ballot_sync(kFull, nc == 2);
+            const int total = __popc(back) + __popc(one) + __popc(two);
+            if (sp > cap - total) {
+                fault |= ST_WALK_STACK;
+            } else {
+                const int at = sp + __popc(back & above) + __popc(one & above) + __popc(two & above);
+                if (back >> lane & 1u) stk[at] = make_int2(A, ~B);
+                if (nc == 1) stk[at] = make_int2(ca, c0);
+                if (nc == 2) {
+                    stk[at] = make_int2(ca, c1);
+                    stk[at + 1] = make_int2(ca, c0);
+                }
+                sp += total;
+            }
+            fault = __reduce_or_sync(kFull, fault);
+            __syncwarp();
+            if (fault) break;  // warp-uniform
+        }
+        if (fault) break;
+        if (MODE == WALK_COUNT && lane == 0) g.out_len[L] = emitted;
+        if (MODE == WALK_FILL && emitted != room) fault = ST_WALK_ROW;
+        if (M2L) {  // L's depth: its path's nodes and itself
+            int d = 1;
+            for (int c = 1; c >= 0 && (c & 1) && d <= g.nnode + 1; ++d) c = toward(g.box32[c].son);
+            depths = max(depths, d);
+        }
+    }
+    if (lane == 0) {
+        if (fault) atomicOr(&g.ctrl->status, fault);
+        if (M2L && ntask) atomicAdd(&g.ctrl->ntask, ntask);
+        if (M2L && depths) atomicMax(&g.ctrl->items[0], depths);
+    }
+}
+
 // Rows from the pool into their CSR places (CHAINS; else they are there
 // already), and their pair counts (with skipped, the pairs of entries wholly
 // beyond the FP32 forms' cutoff too). One warp per leaf.
@@ -526,6 +705,27 @@ inline int walk_first_depths(int nleaf) {
     int lg = 0;
     while (lg < 30 && (1 << lg) < nleaf) ++lg;
     return lg + 6;
+}
+
+// Blocks of a walk by sink leaf and its stacks' memory, at most 1 GB unless a
+// single block's takes more.
+constexpr int kWalkSinkStack = 2048;  // pairs a warp at first
+inline int walk_sink_blocks(int sm_count, int nleaf, int cap) {
+    const int64_t block = (int64_t)kWalkWarps * cap * (int64_t)sizeof(int2);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(walk_blocks(sm_count, nleaf), ((int64_t)1 << 30) / block));
+}
+inline size_t walk_sink_bytes(int blocks, int cap) { return (size_t)blocks * kWalkWarps * cap * sizeof(int2); }
+
+// Enqueues a walk by sink leaf: refs (nnode + nleaf ints) is cleared here.
+template <int MODE>
+inline cudaError_t walk_sinks(cudaStream_t st, const WalkRun &g, const int *son, int *refs, int blocks, int2 *stacks,
+                              int cap, int *tail) {
+    cudaError_t e = cudaMemsetAsync(refs, 0, sizeof(int) * ((size_t)g.nnode + g.nleaf), st);
+    if (e != cudaSuccess) return e;
+    walk_refs_kernel<<<std::min((2 * (int64_t)g.nnode + 255) / 256, (int64_t)4096), 256, 0, st>>>(son, g.nnode, g.nleaf,
+                                                                                                 refs, g.ctrl);
+    walk_sink_kernel<MODE><<<blocks, kWalkWarps * 32, 0, st>>>(g, stacks, cap, tail);
+    return cudaGetLastError();
 }
 
 inline float walk_th2(double open_angle) {

@@ -114,7 +114,7 @@ SIGNATURES = {
     "p2p_session_destroy": (_i, [_vp]),
     "p2p_session_set_params": (_i, [_vp, ctypes.POINTER(Params)]),
     "p2p_session_get_params": (_i, [_vp, ctypes.POINTER(Params)]),
-    "p2p_session_walk_limits": (_i, [_vp, _i64, _i64, _i64]),
+    "p2p_session_walk_limits": (_i, [_vp, _i64, _i64, _i64, _i]),
     "p2p_session_stream": (_vp, [_vp]),
     "p2p_session_poly_degree": (_i, [_vp]),
     "p2p_session_poly_error": (_d, [_vp]),

@@ -74,9 +74,9 @@ class Session:
     def set_params(self, params):
         _check(self.lib, self.lib.p2p_session_set_params(self.h, ctypes.byref(params)))
 
-    def walk_limits(self, list_chunks=0, out_chunks=0, row_bytes=0):
+    def walk_limits(self, list_chunks=0, out_chunks=0, row_bytes=0, depths=0):
         """First sizes and bounds of the device walks' memory (0: the default)."""
-        _check(self.lib, self.lib.p2p_session_walk_limits(self.h, list_chunks, out_chunks, row_bytes))
+        _check(self.lib, self.lib.p2p_session_walk_limits(self.h, list_chunks, out_chunks, row_bytes, depths))
 
     @property
     def stream(self):
