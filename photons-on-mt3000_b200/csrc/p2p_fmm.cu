@@ -400,7 +400,7 @@ struct p2p_fmm {
     int device = 0;
     cudaStream_t stream = nullptr;
     DevBufF parents, leafM, nodeM, sinkL, leafL, counts, ctrl;
-    DevBufF box, items, lists[2], tasks, walk_ctrl;  // the M2L walk
+    DevBufF box, items, lists[2], tasks, tails, walk_ctrl;  // the M2L walk
     WalkLimits limits;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     long long n_m2l = 0, n_applied = 0;
@@ -442,7 +442,7 @@ P2P_API int p2p_fmm_destroy(p2p_fmm *f) {
     cudaSetDevice(f->device);
     cudaStreamSynchronize(f->stream);
     DevBufF *bufs[] = {&f->parents, &f->leafM, &f->nodeM, &f->sinkL, &f->leafL, &f->counts, &f->ctrl, &f->box,
-                       &f->items, &f->lists[0], &f->lists[1], &f->tasks, &f->walk_ctrl};
+                       &f->items, &f->lists[0], &f->lists[1], &f->tasks, &f->tails, &f->walk_ctrl};
     for (DevBufF *b : bufs)
         if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : f->ev)
@@ -526,7 +526,7 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     // walks: a walk that runs out of one is repeated with twice the size; only the
     // buffers outlive the call)
     int *head = (int *)f->counts.p, *len = head + nsink;
-    FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
+    if (!nnode) FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
     WalkRun g;
     std::memset(&g, 0, sizeof(g));
     unsigned long long ntask = 0;
@@ -555,45 +555,58 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
         g.items[0] = (WalkItem *)f->items.p;
         g.items[1] = g.items[0] + nleaf;
         g.ctrl = (WalkCtrl *)f->walk_ctrl.p;
-        for (bool again = true; again;) {
-            again = false;
-            for (int k = 0; k < 2; ++k) {
-                FMM_TRY(grow(f->lists[k], walk_pool_bytes(list_cap, kWalkChunk)));
-                g.lists[k] = walk_pool(f->lists[k].p, list_cap, kWalkChunk);
+        const int depths = f->limits.depths ? std::min(f->limits.depths, kWalkLevels) : walk_first_depths(nleaf) + kWalkExtraDepths;
+        bool by_sink = false;  // a deep tree (walk_sink_kernel)
+        int stack_cap = kWalkSinkStack;
+        for (;;) {
+            const int sink_blocks = walk_sink_blocks(sms, nleaf, stack_cap);
+            if (by_sink) {
+                FMM_TRY(grow(f->lists[0], walk_sink_bytes(sink_blocks, stack_cap)));
+                FMM_TRY(grow(f->lists[1], sizeof(int) * (size_t)nsink));
+                FMM_TRY(grow(f->tails, sizeof(int) * (size_t)nsink));
+            } else {
+                for (int k = 0; k < 2; ++k) FMM_TRY(grow(f->lists[k], walk_pool_bytes(list_cap, kWalkChunk)));
             }
+            for (int k = 0; k < 2; ++k) g.lists[k] = walk_pool(f->lists[k].p, list_cap, kWalkChunk);
             FMM_TRY(grow(f->tasks, walk_pool_bytes(task_cap, kWalkTaskChunk)));
             g.out = walk_pool(f->tasks.p, task_cap, kWalkTaskChunk);
+            FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
             FMM_CUDA(cudaMemsetAsync(g.ctrl, 0, sizeof(WalkCtrl), st), "FMM walk");
             walk_pack_kernel<true><<<blocks_for((long long)nnode + nleaf, threads), threads, 0, st>>>(
                 a.w, (WalkBox *)f->box.p, (WalkBox32 *)((WalkBox *)f->box.p + nbox), nullptr, g.items[0], g.lists[0].ids, g.ctrl);
-            for (int lv = 0, n = walk_first_depths(nleaf);; n = 4) {
-                n = std::min(n, kWalkLevels - lv);
-                if (n <= 0) return report_error(P2P_ERR_CAPACITY, "FMM walk: too many levels");
-                FMM_CUDA(walk_depths<WALK_M2L>(st, g, sms, lv, n), "FMM walk");
-                count_launches(n);
+            int status = 0, lv = 0;
+            std::vector<int> boxes;  // of each depth
+            for (int n = walk_first_depths(nleaf);; n = 4) {
+                n = by_sink ? 0 : std::min(n, depths - lv);
+                if (by_sink)
+                    FMM_CUDA(walk_sinks<WALK_M2L>(st, g, t->son, (int *)f->lists[1].p, sink_blocks, (int2 *)f->lists[0].p,
+                                                  stack_cap, (int *)f->tails.p), "FMM walk");
+                else
+                    FMM_CUDA(walk_depths<WALK_M2L>(st, g, sms, lv, n), "FMM walk");
+                count_launches(by_sink ? 2 : n);
                 lv += n;
-                std::vector<int> boxes(lv + 1);
-                int status = 0;
+                boxes.resize(lv + 1);
                 FMM_CUDA(cudaMemcpyAsync(boxes.data(), g.ctrl->items, sizeof(int) * (lv + 1), cudaMemcpyDeviceToHost, st),
                          "FMM walk");
                 FMM_CUDA(cudaMemcpyAsync(&status, &g.ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st), "FMM walk");
                 FMM_CUDA(cudaMemcpyAsync(&ntask, &g.ctrl->ntask, sizeof(ntask), cudaMemcpyDeviceToHost, st), "FMM walk");
                 FMM_CUDA(cudaStreamSynchronize(st), "FMM walk");
-                if (status & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
-                if (status & ST_WALK_STACK) return report_error(P2P_ERR_CAPACITY, "FMM walk: stack exceeded");
-                if (status) {
-                    if (status & ST_WALK_LISTS) list_cap *= 2;
-                    if (status & ST_WALK_OUT) task_cap *= 2;
-                    if (std::max(list_cap, task_cap) > INT32_MAX)
-                        return report_error(P2P_ERR_CAPACITY, "FMM walk: more lists than a pool can hold");
-                    FMM_CUDA(cudaMemsetAsync(len, 0, sizeof(int) * (size_t)nsink, st), "FMM walk");
-                    again = true;
-                    break;
-                }
-                if (boxes[lv] == 0) {
-                    f->levels = lv - (int)std::count(boxes.begin(), boxes.begin() + lv, 0);
-                    break;
-                }
+                if (status || by_sink || boxes[lv] == 0 || lv == depths) break;
+            }
+            if (status & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
+            if (!status && (by_sink || boxes[lv] == 0)) {
+                f->levels = by_sink ? boxes[0] : lv - (int)std::count(boxes.begin(), boxes.begin() + lv, 0);
+                break;
+            }
+            if (status & ST_WALK_LISTS) list_cap *= 2;
+            if (status & ST_WALK_OUT) task_cap *= 2;
+            if (std::max(list_cap, task_cap) > INT32_MAX)
+                return report_error(P2P_ERR_CAPACITY, "FMM walk: more lists than a pool can hold");
+            if (!by_sink) {
+                by_sink = (status & ST_WALK_STACK) || !status;  // (boxes are left below the last depth)
+            } else if (status & ST_WALK_STACK) {
+                if (stack_cap > (1 << 28)) return report_error(P2P_ERR_CAPACITY, "FMM walk: a sink's walk exceeded its stack");
+                stack_cap *= 2;
             }
         }
     }
