@@ -92,7 +92,7 @@ struct p2p_session {
     std::map<std::tuple<const void *, int, size_t>, int> occupancy;
     p2p_params params{};
     PolyFit fit;
-    Fit64 fit64{};  // FP64 form
+    Fit64For fit64;  // FP64 form
     // device buffers
     DevBuf task_t2, task_s2;  // second buffer pair of pipelined submits
     DevBuf pos, mass, leaf_ip, leaf_np, task_t, task_s, meta, pos4, counts, fill, row_off,
@@ -239,7 +239,7 @@ int default_stage(const p2p_params &p) {
 // 0.144 ms where four take 0.220 (12^3, 900 leaves); from 32^3 (3,900 leaves:
 // 0.361 ms at four, 0.379 at eight) to 110^3 four are as good or better.
 int default_warps(const p2p_session *s, const p2p_params &p) {
-    return p.form == P2P_FORM_PLAIN_FP64 && s->fit64.nfar && s->nleaf <= 16 * s->sm_count ? 8 : 4;
+    return p.form == P2P_FORM_PLAIN_FP64 && s->fit64.fit().nfar && s->nleaf <= 16 * s->sm_count ? 8 : 4;
 }
 
 // Shares that a sink leaf's row is cut into (1: none). With few leaves the
@@ -255,7 +255,7 @@ int default_warps(const p2p_session *s, const p2p_params &p) {
 constexpr int kRowParts = 4;
 int row_parts(const p2p_session *s, int npart, int nleaf) {
     const p2p_params &p = s->params;
-    if (p.form == P2P_FORM_PLAIN_FP64) return s->fit64.nfar && nleaf <= 1000 ? kRowParts : 1;
+    if (p.form == P2P_FORM_PLAIN_FP64) return s->fit64.fit().nfar && nleaf <= 1000 ? kRowParts : 1;
     return sink_regs(p) && p.warps_per_leaf == 0 && (int64_t)nleaf * nleaf <= 900 * (int64_t)npart ? kRowParts : 1;
 }
 
@@ -275,7 +275,7 @@ int launch_pair(p2p_session *s, const PairArgs &a) {
     L.dry_run = s->dry_run;
     L.occ = &s->occupancy;
     L.sink_pairs = p.kernel_variant == P2P_VARIANT_SOURCE_LANES_X2_S16 ? 8 : 16;
-    L.fit64 = &s->fit64;
+    L.fit64 = &s->fit64.fit();
     L.sreg_spl = p.kernel_variant == P2P_VARIANT_SINK_REGS8 ? 8 : 4;
     PairLaunchResult r;
     if (p.form == P2P_FORM_PLAIN_FP64)
@@ -609,7 +609,7 @@ P2P_API int p2p_session_set_params(p2p_session *s, const p2p_params *params) {
     P2P_TRY(validate_params(params));
     s->params = *params;
     if (params->form == P2P_FORM_PLAIN_FP64)
-        s->fit64 = fit64(params->x_cut, params->split_radius, params->soften);
+        s->fit64.set(params->x_cut, params->split_radius, params->soften);
     if (is_fp32_form(params->form)) {
         s->fit = fit_h(fit_umax(params->x_cut), params->poly_tol > 0.0 ? params->poly_tol : kDefaultPolyTol);
     } else {

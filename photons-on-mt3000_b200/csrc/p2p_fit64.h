@@ -137,4 +137,26 @@ inline Fit64 fit64(double x_cut, double split_radius, double soften) {
     return F;
 }
 
+// The fit with the three numbers that it was made for. A fit takes 0.1 to 0.2 ms on
+// the host, and a caller may set its parameters before every pass (PhotoNs' entry
+// points do), mostly to the same numbers.
+class Fit64For {
+  public:
+    // Makes the fit unless it is there; whether it was made.
+    bool set(double x_cut, double split_radius, double soften) {
+        if (made_ && x_cut == of_[0] && split_radius == of_[1] && soften == of_[2]) return false;
+        fit_ = fit64(x_cut, split_radius, soften);
+        of_[0] = x_cut;
+        of_[1] = split_radius;
+        of_[2] = soften;
+        return made_ = true;
+    }
+    const Fit64 &fit() const { return fit_; }
+
+  private:
+    Fit64 fit_{};
+    double of_[3] = {0.0, 0.0, 0.0};
+    bool made_ = false;
+};
+
 }  // namespace p2p

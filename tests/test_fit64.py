@@ -62,3 +62,39 @@ def test_pair_factor_is_within_ten_half_ulps(program, x_cut, coefs, rs):
 @pytest.mark.parametrize("x_cut", [0.0, -1.0, 1.0, 4.5, float("nan")])
 def test_other_cutoffs_have_no_fit(program, x_cut):
     assert subprocess.check_output([program, str(x_cut), "0.1"], text=True).split()[0] == "0"
+
+
+KEPT = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "p2p_fit64.h"
+using namespace p2p;
+static bool same(const Fit64 &a, const Fit64 &b) {
+    bool s = a.nfar == b.nfar && a.hi_near == b.hi_near && a.hi_in == b.hi_in && a.hi_out == b.hi_out &&
+             a.near_mid == b.near_mid && a.far_mid == b.far_mid && a.e_hi == b.e_hi && a.e_lo == b.e_lo;
+    for (int i = 0; i < kFit64Near; ++i) s = s && a.near[i] == b.near[i];
+    for (int i = 0; i < kFit64MaxFar; ++i) s = s && a.far[i] == b.far[i];
+    for (int i = 0; i < kFit64Exp; ++i) s = s && a.exp2[i] == b.exp2[i];
+    return s;
+}
+int main() {
+    // x_cut, split radius, softening, and whether the fit has to be made
+    const double call[][4] = {{2.8125, 0.01, 1e-4, 1}, {2.8125, 0.01, 1e-4, 0}, {2.25, 0.01, 1e-4, 1}, {2.25, 0.02, 1e-4, 1},
+                              {2.25, 0.02, 1e-70, 1}, {2.25, 0.02, 1e-70, 0}, {2.25, 0.02, 1e-4, 1}, {0.0, 0.02, 1e-4, 1},
+                              {0.0, 0.02, 1e-4, 0}, {2.8125, 0.01, 1e-4, 1}};
+    Fit64For kept;
+    int wrong = kept.fit().nfar != 0;
+    for (auto &c : call) {
+        if (kept.set(c[0], c[1], c[2]) != (c[3] != 0)) ++wrong;
+        if (!same(kept.fit(), fit64(c[0], c[1], c[2]))) ++wrong;
+    }
+    printf("%d\n", wrong);
+}
+"""
+
+
+def test_the_fit_is_made_again_only_for_other_numbers(tmp_path):
+    (tmp_path / "k.cpp").write_text(KEPT)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-I", os.path.join(REPO, "photons-on-mt3000_b200", "csrc"),
+                           str(tmp_path / "k.cpp"), "-o", str(tmp_path / "k")])
+    assert subprocess.check_output([str(tmp_path / "k")], text=True).split() == ["0"]
