@@ -4,15 +4,17 @@ The shape of a pass is (mapping and sink tile, sources staged per warp,
 warps per block, warps per sink leaf): the sink-register kernel keeps four
 sinks per lane in registers over 32-sink slices (SINK_REGS) or eight over
 64-sink slices (SINK_REGS8, so leaves of up to 64 particles stage their
-sources once), and spreads one sink leaf's row over 1, 2 or 4 warps
-(warps_per_leaf, partial forces added with atomics); the packed source-lane kernel holds a slice of a sink leaf
+sources once), and takes one sink leaf's row in the session's own way (1: one
+warp, or in a session with few leaves four whose sums are kept apart and added
+in order) or spreads it over 2 or 4 warps (partial forces added with atomics);
+the packed source-lane kernel holds a slice of a sink leaf
 in registers against one staged source per lane (32 sinks, SOURCE_LANES_X2,
 or 16 sinks with half the partial registers and more resident warps,
 SOURCE_LANES_X2_S16); the packed sink-lane kernel keeps one sink pair per
 lane and spreads the staged sources over the lanes (SINK_LANES_X2),
 stage_sources is the source chunk a warp stages in shared memory before it
-computes, and every sink leaf is one warp's work item (the persistent
-kernel's work-stealing unit). Which shape wins depends on how many particles
+computes, and a sink leaf, or its share of the row, is one warp's work item (the
+persistent kernel's work-stealing unit). Which shape wins depends on how many particles
 the leaves hold and how long the rows are, so tuned shapes are cached under
 a key built from the leaf-size histogram (quartiles of particles per leaf,
 mean list entries per sink leaf, leaf cap) plus the form and softening.
@@ -23,9 +25,9 @@ keeps the fastest. The sample holds about `sample_pairs` pairs (1e10) and
 at least 64 sink leaves per resident warp: with a few per warp the tail of
 uneven rows dominates and spreading a row over several warps wins on the
 sample but not on the pass.
-A shape that spreads rows over several warps adds their partial forces with
-FP64 atomics, so its results do not repeat bit for bit between runs; it is
-kept only when it beats the fastest one-warp shape by more than
+A shape with 2 or 4 warps per leaf adds their partial forces with FP64
+atomics, so its results do not repeat bit for bit between runs; it is kept
+only when it beats the fastest repeatable shape by more than
 `repeatable_margin` (choose()).
 """
 import json
@@ -46,7 +48,8 @@ CANDIDATES = [
 ] + [(abi.VARIANT_SINK_LANES_X2, st, w) for st in (128, 256, 512) for w in (2, 4)
 ] + [(abi.VARIANT_SINK_REGS, st, w, lw) for st in (256, 384) for w in (2, 4) for lw in (1, 2, 4)
 ] + [(abi.VARIANT_SINK_REGS8, st, w, lw) for st in (256, 384) for w in (2, 4) for lw in (1, 2)]
-# every candidate as (variant, stage, warps per block, warps per leaf)
+# every candidate as (variant, stage, warps per block, warps per leaf), the last 1 for
+# the session's own, repeatable way with rows (shape_params)
 CANDIDATES = [c if len(c) == 4 else c + (1,) for c in CANDIDATES]
 
 
@@ -96,8 +99,8 @@ def save_cache(path, cache):
 
 def choose(results, repeatable_margin=0.03):
     """The record to keep among timed candidates: the fastest, unless it
-    spreads rows over several warps (leaf_warps > 1) and is not faster than
-    the fastest one-warp candidate by more than repeatable_margin, in which
+    adds the warps of a row with atomics (leaf_warps > 1) and is not faster than
+    the fastest other candidate by more than repeatable_margin, in which
     case that one (its results repeat bit for bit)."""
     best = max(results, key=lambda r: r["pairs_per_s"])
     one = [r for r in results if r.get("leaf_warps", 1) == 1]
@@ -106,6 +109,17 @@ def choose(results, repeatable_margin=0.03):
         if best["pairs_per_s"] <= b1["pairs_per_s"] * (1.0 + repeatable_margin):
             return b1
     return best
+
+
+def shape_params(cfg, form, mass, variant, stage, warps, leaf_warps=1):
+    """Pass parameters with a candidate's launch shape. One warp per leaf is
+    asked for as 0, the default, with which a session with few leaves cuts
+    rows into shares (12^3: 0.117 ms whole, 0.052 in shares); 1 would keep
+    rows whole."""
+    p = params_for(cfg, form, mass)
+    p.kernel_variant, p.stage_sources, p.warps_per_block = variant, stage, warps
+    p.warps_per_leaf = leaf_warps if leaf_warps > 1 else 0
+    return p
 
 
 # Sample size by rows: every resident warp of the persistent pair kernel
@@ -127,10 +141,7 @@ def tune(cfg, lists, form, mass, device=0, sample_pairs=1e10, cache_path=None, r
     cache = load_cache(cache_path) if cache_path else {}
 
     def apply(rec):
-        p = params_for(cfg, form, mass)
-        p.kernel_variant, p.stage_sources, p.warps_per_block = rec["variant"], rec["stage"], rec["warps"]
-        p.warps_per_leaf = rec.get("leaf_warps", 1)
-        return p
+        return shape_params(cfg, form, mass, rec["variant"], rec["stage"], rec["warps"], rec.get("leaf_warps", 1))
 
     if key in cache:
         return apply(cache[key]), dict(cache[key], key=key, cached=True)
@@ -149,11 +160,8 @@ def tune(cfg, lists, form, mass, device=0, sample_pairs=1e10, cache_path=None, r
     with Session(device) as s:
         for cand in cands:
             variant, stage, warps, lw = cand if len(cand) == 4 else tuple(cand) + (1,)
-            p = params_for(cfg, form, mass)
-            p.kernel_variant, p.stage_sources, p.warps_per_block = variant, stage, warps
-            p.warps_per_leaf = lw
             try:
-                s.set_params(p)
+                s.set_params(shape_params(cfg, form, mass, variant, stage, warps, lw))
                 ms = []
                 for _ in range(repeats + 1):
                     s.run_device(*args)

@@ -104,3 +104,27 @@ def test_sample_rows_keeps_enough_rows():
     assert np.array_equal(st, t[(t % k) == 0]) and np.array_equal(ss, s[(t % k) == 0])
     st2, _, _ = autotune.sample_rows(n, t, s, total / 10, min_rows=1)
     assert np.unique(st2).size < np.unique(st).size  # the pair target rules when min_rows is small
+
+
+def test_a_tuned_one_warp_shape_keeps_the_sessions_way_with_rows(tmp_path):
+    """One warp per leaf, from a candidate or a cached record, is the default 0 (a
+    session with few leaves cuts rows into shares), not 1, which keeps rows whole and
+    would make a tuned small pass slower than an untuned one; 2 and 4 stay."""
+    from photons_p2p import workloads as W
+
+    cfg = W.c1_config()
+    for variant, stage, warps, lw in autotune.CANDIDATES:
+        p = autotune.shape_params(cfg, abi.FORM_SPLIT, 1.0, variant, stage, warps, lw)
+        assert (p.kernel_variant, p.stage_sources, p.warps_per_block) == (variant, stage, warps)
+        assert p.warps_per_leaf == {1: 0, 2: 2, 4: 4}[lw]
+
+    class Lists:
+        leaf_npart, task_t, task_s = lists()
+
+    path = str(tmp_path / "tune.json")
+    key = autotune.histogram_key(Lists.leaf_npart, Lists.task_t, abi.FORM_SPLIT, cfg.soft_mode)
+    for leaf_warps, want in ((1, 0), (2, 2)):
+        autotune.save_cache(path, {key: {"variant": abi.VARIANT_SINK_REGS, "stage": 256, "warps": 4,
+                                         "leaf_warps": leaf_warps, "pairs_per_s": 1.0}})
+        p, rec = autotune.tune(cfg, Lists, abi.FORM_SPLIT, 1.0, cache_path=path)
+        assert rec["cached"] and p.warps_per_leaf == want
