@@ -164,6 +164,12 @@ def load_traffic(workload, form_name):
         return None
 
 
+def fp64_kernel(x_cut):
+    """The FP64 form's pair kernel for a cutoff: "pair_fp64" where the pair factor
+    is fitted (csrc/p2p_fit64.h), else "plain_fp64"."""
+    return "pair_fp64" if 1.25 <= x_cut <= 4.0 else "plain_fp64"
+
+
 def load_fp64_flops(workload, kernel="plain_fp64"):
     """FP64 flops per listed pair of a pair kernel of the plain form (DFMA x 2 +
     DADD + DMUL per pair) from the committed ncu summary, or None: "plain_fp64",
@@ -569,7 +575,8 @@ def run_ours(args, rank, world, dist):
             sess.set_params(params_for(cfg, abi.FORM_PLAIN_FP64, mass))
             p_s, p_k, _ = resident_passes(sess, max(1, min(args.steps, 3)), 1)
             plain = {"value": P / float(np.mean(p_s)), "kernel_ms": float(np.mean(p_k))}
-            plain["roofline"] = plain_roofline(args.workload, P, plain["kernel_ms"], fp64_peak, fp32_peak, "pair_fp64")
+            plain["roofline"] = plain_roofline(args.workload, P, plain["kernel_ms"], fp64_peak, fp32_peak,
+                                               fp64_kernel(cfg.x_cut))
             loc = tl.tag == 1
             acc_plain = result(sess)
             num = np.linalg.norm(acc_form - acc_plain, axis=0)[loc]
@@ -622,7 +629,7 @@ def run_ours(args, rank, world, dist):
     kernel_pairs_per_s = P / (mean_kernel_ms * 1e-3)
     roofline = None
     if form == abi.FORM_PLAIN_FP64:
-        roofline = plain_roofline(args.workload, P, mean_kernel_ms, fp64_peak, fp32_peak, "pair_fp64")
+        roofline = plain_roofline(args.workload, P, mean_kernel_ms, fp64_peak, fp32_peak, fp64_kernel(cfg.x_cut))
     if F:
         # flops of the pairs the kernel evaluates (entries wholly beyond the
         # cutoff are skipped: counted in the metric's pairs, not in the flops)

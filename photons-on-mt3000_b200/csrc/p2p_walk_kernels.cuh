@@ -64,9 +64,6 @@ enum : int {
 __device__ __forceinline__ const double *walk_center(const WalkArgs &w, int c) {
     return (c & 1) ? w.node_center + 3 * (size_t)(c >> 1) : w.leaf_center + 3 * (size_t)(c >> 1);
 }
-__device__ __forceinline__ const double *walk_width(const WalkArgs &w, int c) {
-    return (c & 1) ? w.node_width + 3 * (size_t)(c >> 1) : w.leaf_width + 3 * (size_t)(c >> 1);
-}
 
 __device__ __forceinline__ bool walk_valid(const WalkArgs &w, int c) {
     return c >= 0 && ((c & 1) ? (c >> 1) < w.nnode : (c >> 1) < w.nleaf);
