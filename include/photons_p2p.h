@@ -317,7 +317,8 @@ int p2p_pm_download(p2p_pm *pm, double *mass_mesh, double *potential);
  * (src/operator.c:340-344), which skips every task with r2 < 1 in its length
  * unit: min_r2 = 1 reproduces it, 1e-15 what the test evidently means.
  * Queued on the session's stream; the M2L walk reads its counts back to the
- * host, so the call returns when the pass is done. */
+ * host, so the call returns when the pass is done. Its walk is that of
+ * p2p_pass_submit_walk: by depth, deep trees by sink leaf. */
 typedef struct p2p_fmm p2p_fmm;
 int p2p_fmm_create(p2p_session *s, p2p_fmm **out);
 int p2p_fmm_destroy(p2p_fmm *f);
@@ -369,8 +370,9 @@ int p2p_session_last_kernel_ms(p2p_session *s, float *ms);
  * the rest of the device are not synchronised. The numeric fields of params
  * are checked as p2p_session_set_params checks them; warps_per_block,
  * blocks_per_sm, kernel_variant and warps_per_leaf are ignored (the split
- * form always runs the packed source-lane kernel, 4 warps per block, as many
- * blocks as fit, one warp per sink leaf).
+ * form always runs the packed source-lane kernel, the FP64 form the general one
+ * that calls erfc and exp for every pair, at a third of the speed of a session with
+ * a cutoff; 4 warps per block, as many blocks as fit, one warp per sink leaf).
  *
  * Limit: the scratch needed, about 16*npart (split form only) + 48*nleaf +
  * 4*ntask bytes plus 256-byte alignment of each piece, must fit in

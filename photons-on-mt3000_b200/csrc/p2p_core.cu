@@ -235,23 +235,32 @@ int default_stage(const p2p_params &p) {
 }
 
 // Warps per block. The FP64 kernel's warps share a sink leaf's row: with so
-// few leaves that the rows' length and not their number decides, eight take
-// 0.144 ms where four take 0.220 (12^3, 900 leaves); from 32^3 (3,900 leaves:
-// 0.361 ms at four, 0.379 at eight) to 110^3 four are as good or better.
+// few leaves that the rows' length and not their number decides, eight are
+// better. Rows whole, at four and eight (lattices, leaves of 32): 0.185 and
+// 0.128 ms at 12^3 (512 leaves), 0.207 and 0.169 at 16^3 (1,003), 0.367 and
+// 0.342 at 24^3 (2,048), 0.498 and 0.480 at 28^3 (2,144), 0.564 and 0.560 at
+// 32^3 (4,010), 1.98 and 2.21 at 48^3 (8,192). With the drop-in's shorter rows
+// it is even lower: 0.315 and 0.347 at 32^3 (2,072 leaves).
 int default_warps(const p2p_session *s, const p2p_params &p) {
     return p.form == P2P_FORM_PLAIN_FP64 && s->fit64.fit().nfar && s->nleaf <= 16 * s->sm_count ? 8 : 4;
 }
 
 // Shares that a sink leaf's row is cut into (1: none). With few leaves the
 // longest row and not the work decides; the shares' sums lie in arrays of their
-// own and are added in order (two more launches, 24 bytes a particle and
-// share). Sink-register kernel, whole and in four shares: 0.117 and 0.052 ms at
-// 12^3 (512 leaves), 0.166 and 0.136 at 32^3 (3,992), 2.71 and 2.03 at 64^3
-// clustered (19,039), 16.9 and 14.6 at 101^3 with leaves of 64 (30,403); but 2.94
-// and 3.16 at 100^3 (65,513), and short rows lose sooner: 0.48 and 0.62 at 48^3
-// with leaves of 8 (33,048). So up to 900 leaves per particle of the mean leaf.
-// The FP64 kernel's blocks share rows among their warps already: 0.144 and 0.097
-// ms at 512 leaves, 0.379 and 0.407 at 2,046.
+// own and are added in order (two more launches, 216 bytes a particle for every
+// list chunk). Sink-register kernel, whole and in four shares: 0.097 and 0.045 ms
+// at 12^3 (512 leaves), 0.166 and 0.133 at 32^3 (4,010), 0.097 and 0.076 there with
+// the drop-in's settings (2,072), 18.7 and 15.4 at 101^3 clustered with leaves of
+// 64 (31,694: nleaf^2 = 712 npart). Long rows of clustered particles would gain
+// further up (64^3: 4.4 and 3.3 ms at 942 npart, 100^3: 8.6 and 8.1 at 2,780), but
+// lattices lose at 100^3 (2.94 and 3.16 ms, 65,513 leaves) and short rows at
+// 48^3 with leaves of 8 (0.48 and 0.62, 5,436 npart). So up to 900 npart: 900
+// leaves per particle of the mean leaf. Many small chunks keep the gain (101^3 in
+// 256: 254 and 131 ms) unless they hold a few dozen entries (12^3 in 256 chunks of
+// 73: 14.1 and 15.3 ms).
+// The FP64 kernel's blocks share rows among their warps already; with eight warps
+// whole and in shares: 0.128 and 0.084 ms at 512 leaves, 0.169 and 0.154 at 1,003,
+// 0.275 and 0.242 at 1,052 (20^3), but 0.342 and 0.371 at 2,048 (24^3).
 constexpr int kRowParts = 4;
 int row_parts(const p2p_session *s, int npart, int nleaf) {
     const p2p_params &p = s->params;
@@ -768,7 +777,8 @@ P2P_API int p2p_pass_submit(p2p_session *s, int64_t ntask, const int *task_t, co
         // Large lists (FP32 forms): upload in pieces on the copy stream while
         // the previous piece's CSR build and pair kernel run (each piece is a
         // list chunk, as the reference's LEN_TASK chunks are). The FP64 form
-        // keeps one chunk: its slowest rows would stretch every piece's tail.
+        // keeps one chunk: beside its kernel (841 ms at 256^3) the upload of
+        // the list (3.4 GB) is small.
         const int64_t piece = std::max<int64_t>(kPipePieceMin, (ntask + kPipePieces - 1) / kPipePieces);
         P2P_TRY(ensure(s, s->task_t, sizeof(int) * (size_t)piece));
         P2P_TRY(ensure(s, s->task_s, sizeof(int) * (size_t)piece));

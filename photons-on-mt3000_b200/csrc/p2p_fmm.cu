@@ -10,7 +10,8 @@
 //   M2L walk   the reference's dual-tree recursion from (root, root)
 //              (walk_task_m2l, src/fmm.c:812-957, with the acceptance test
 //              of :409-479) depth by depth of the sink side on the GPU
-//              (walk_level_kernel), each sink's accepted sources in a list
+//              (walk_level_kernel; deep trees by sink leaf, walk_sink_kernel),
+//              each sink's accepted sources in a list
 //   M2L        each sink (leaf or node), half a warp, sums over its list, in the
 //              order the walk leaves it, the source multipole's contribution
 //              to its local expansion with the erfc-truncated kernel's derivatives
@@ -237,9 +238,8 @@ __global__ void fmm_upward_kernel(FmmArgs f) {
 
 // M2L: half a warp per sink (a sink has about 10 tasks at open angle 0.4),
 // lane j takes tasks j, j + 16, ... of its list, in the order the walk left
-// them (pre-order of the sources within a depth of the sink's path), and the
-// lanes' partial locals are summed by a fixed shuffle tree: the same sum on
-// every run. The walk keeps a sink's tasks together, so nothing is sorted.
+// them (which does not vary between runs), and the lanes' partial locals are
+// summed by a fixed shuffle tree: the same sum on every run. The walk keeps a sink's tasks together, so nothing is sorted.
 constexpr int kM2LThreads = 128;
 
 __global__ void __launch_bounds__(kM2LThreads)

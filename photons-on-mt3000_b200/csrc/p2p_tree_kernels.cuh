@@ -13,10 +13,11 @@
 // particles splits at their midpoint, swapping them when the first is above
 // the second. Nodes are split level by level while they hold more than
 // kTreeSmall particles (the partition by tiles of the node's slots, a level's
-// children by one block, with no host between); smaller subtrees are built whole by one block each in
-// shared memory. Nodes and leaves get build-order ids as they are made; the
-// pre-order ids of the reference (son[0]'s subtree first, leaves numbered
-// apart from nodes) and the node boxes follow from two passes over depths.
+// children by one block, with no host between); smaller subtrees are built whole
+// by one block each in shared memory. Nodes and leaves get build-order ids as they
+// are made; the pre-order ids of the reference (son[0]'s subtree first, leaves
+// numbered apart from nodes) and the node boxes follow from three passes: parents,
+// counts from the leaves up, numbers and boxes from each node's path to the root.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -807,8 +808,7 @@ tree_small_kernel(const TreeTask *__restrict__ tasks, TreeParts P, TreeRec R, in
 // ------------------------------------------------- numbering and boxes ---
 
 // Three passes whatever the tree's depth (one launch per depth, twice, took 26 to
-// 52 launches, a tenth of a small step): parents, counts by climbing, numbers and
-// boxes by climbing.
+// 52 launches, a tenth of a small step).
 
 // Each box's parent as 2 x node + side (-1: the root), nodes' arrival counts 0.
 __global__ void tree_link_kernel(TreeRec R, int nnode, int nleaf, int *__restrict__ parent,

@@ -87,9 +87,8 @@ def test_lattice_no_m2l(gpu):
 def test_large_tree_is_deterministic(gpu):
     """256^3 clustered particles (1.65M sinks: more than one thread per sink
     fits in a capped grid): the far field runs to the end, every task is
-    applied with min_r2 = 1e-15, and two runs give the same bits (tasks are
-    summed per sink in increasing source order, whatever order the walk
-    found them in)."""
+    applied with min_r2 = 1e-15, and two runs give the same bits (a sink's
+    tasks are summed in the order the walk leaves them in, which does not vary)."""
     import torch
 
     cfg = W.scaled(W.c2_config(), open_angle=0.4)
