@@ -226,7 +226,8 @@ typedef struct p2p_walk_tree {
  * Trees far deeper than a balanced one (many particles at one point) are walked by
  * sink leaf, rows counted and then written, with stacks of 80 MB at first.
  * P2P_ERR_ARG for a child code outside the tree or leaves that are not in
- * pre-order. */
+ * pre-order, P2P_ERR_CAPACITY for trees with chains of more than about 11,000
+ * splits (p2p_dtree_build makes up to 6,143). */
 int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *tree, double cutoff, double open_angle,
                          int64_t *ntask);
 /* ---- Device kd-tree (no counterpart in the reference's GPU code) --------

@@ -156,6 +156,8 @@ bool is_fp32_form(int form) { return form != P2P_FORM_PLAIN_FP64; }
 // take a second walk.
 constexpr size_t kWalkPoolBytes = (size_t)8 << 30;
 
+constexpr const char *kWalkTooLong = "walk: a leaf's walk met more pairs than it may (a chain of thousands of splits)";
+
 // Doubles per piece of p2p_pass_accumulate (512 KB).
 constexpr size_t kStageDoubles = 65536;
 
@@ -838,6 +840,7 @@ P2P_API int p2p_pass_end(p2p_session *s, double *gpu_seconds) {
     if (status & ST_LEAF_RANGE) return fail(P2P_ERR_RANGE, "a leaf range lies outside the particles");
     if (status & ST_TASK_RANGE) return fail(P2P_ERR_RANGE, "a task entry names a leaf outside [0, nleaf)");
     if (status & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
+    if (status & ST_WALK_LONG) return fail(P2P_ERR_CAPACITY, kWalkTooLong);
     if (status & ST_WALK_ROW) return fail(P2P_ERR_CAPACITY, "walk: a row came out otherwise than it was counted");
     return P2P_OK;
 }
@@ -967,13 +970,14 @@ P2P_API int p2p_pass_submit_walk(p2p_session *s, const p2p_walk_tree *t, double 
                 CUDA_TRY(cudaStreamSynchronize(s->stream));
                 if (st || by_sink || left == 0 || lv == depths) break;
             }
-            const int bad = st & (ST_WALK_TREE | ST_WALK_ROW);
+            const int bad = st & (ST_WALK_TREE | ST_WALK_ROW | ST_WALK_LONG);
             if (bad) {  // closing the pass reports it too
                 int main_status = 0;
                 CUDA_TRY(cudaMemcpy(&main_status, s->status, sizeof(int), cudaMemcpyDeviceToHost));
                 main_status |= bad;
                 CUDA_TRY(cudaMemcpy(s->status, &main_status, sizeof(int), cudaMemcpyHostToDevice));
                 if (bad & ST_WALK_TREE) return fail(P2P_ERR_ARG, "walk: a child code outside the tree");
+                if (bad & ST_WALK_LONG) return fail(P2P_ERR_CAPACITY, kWalkTooLong);
                 return fail(P2P_ERR_CAPACITY, "walk: a row came out otherwise than it was counted");
             }
             if (by_sink) {

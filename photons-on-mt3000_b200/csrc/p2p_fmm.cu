@@ -594,6 +594,7 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
                 if (status || by_sink || boxes[lv] == 0 || lv == depths) break;
             }
             if (status & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
+            if (status & ST_WALK_LONG) return report_error(P2P_ERR_CAPACITY, "FMM walk: a leaf's walk met more pairs than it may");
             if (!status && (by_sink || boxes[lv] == 0)) {
                 f->levels = by_sink ? boxes[0] : lv - (int)std::count(boxes.begin(), boxes.begin() + lv, 0);
                 break;

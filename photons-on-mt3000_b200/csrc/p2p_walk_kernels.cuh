@@ -59,6 +59,7 @@ enum : int {
     ST_WALK_TREE = 16,    // a child code outside the tree, leaves not in pre-order, or a walk longer than any tree allows
     ST_WALK_LISTS = 32,   // the pool of undecided lists is full (the host enlarges it and repeats the walk)
     ST_WALK_OUT = 64,     // the pool of rows (or M2L tasks) is full
+    ST_WALK_LONG = 128,   // a walk by sink leaf met more pairs than it may
 };
 
 __device__ __forceinline__ const double *walk_center(const WalkArgs &w, int c) {
@@ -482,8 +483,12 @@ walk_refs_kernel(const int *__restrict__ son, int nnode, int nleaf, int *__restr
 // MODE: WALK_COUNT, WALK_FILL (rows in leaf order, as walk_level_kernel) or
 // WALK_M2L (a box's tasks belong to the warp of its first leaf, which appends them
 // one by one in the order of its walk; tail: per sink, its last chunk).
-// Stacks: cap pairs per warp. Pairs lie on the stack in leaf order of B, whose
-// subtrees do not overlap, the first on top.
+// A leaf's walk ends after kWalkSinkPairs pairs, or 64 a box in larger trees: some
+// seconds, three times what the deepest chain that the tree build makes takes (6,143
+// splits, 19 million pairs). Stacks: cap pairs per warp. Pairs lie on the stack in
+// leaf order of B, whose subtrees do not overlap, the first on top.
+constexpr long long kWalkSinkPairs = 1LL << 26;
+
 template <int MODE>
 __global__ void __launch_bounds__(kWalkWarps * 32)
 walk_sink_kernel(const WalkRun g, int2 *stacks, int cap, int *__restrict__ tail) {
@@ -495,7 +500,9 @@ walk_sink_kernel(const WalkRun g, int2 *stacks, int cap, int *__restrict__ tail)
     unsigned long long ntask = 0;
     auto valid = [&](int c) { return c >= 0 && ((c & 1) ? (c >> 1) < g.nnode : (c >> 1) < g.nleaf); };
     auto first_leaf = [&](int c) { return (c & 1) ? g.node_first[c >> 1] : c >> 1; };
-    for (int L = warp; L < g.nleaf && !g.ctrl->status; L += gridDim.x * kWalkWarps) {
+    const volatile int &failed = g.ctrl->status;  // (a walk that failed is not continued)
+    for (int L = warp; L < g.nleaf; L += gridDim.x * kWalkWarps) {
+        if (__any_sync(kFull, failed)) break;
         if (!M2L && g.active[L + 1] == g.active[L]) continue;  // (its count is 0)
         const int64_t row = MODE == WALK_FILL ? g.row_off[L] : 0;
         const int room = MODE == WALK_FILL ? (int)(g.row_off[L + 1] - row) : 0;
@@ -512,12 +519,14 @@ walk_sink_kernel(const WalkRun g, int2 *stacks, int cap, int *__restrict__ tail)
         if (lane == 0) stk[0] = make_int2(1, 1);
         __syncwarp();
         int sp = 1, emitted = 0;
+        long long budget = max(kWalkSinkPairs, 64LL * ((long long)g.nnode + g.nleaf));
         while (sp > 0) {
             const int ns = min(32, sp);
             int2 v = make_int2(0, 0);
             if (lane < ns) v = stk[sp - 1 - lane];
             __syncwarp();  // the pairs are read before others are put in their places
             sp -= ns;
+            budget -= ns;
             const int A = v.x;
             int B = v.y, cls = 0;  // 0 dropped, 1 decided, 2 opened
             int nc = 0, ca = A, c0 = -1, c1 = -1;  // the opened pair's nc pairs: (ca, c0), (ca, c1)
@@ -596,6 +605,7 @@ walk_sink_kernel(const WalkRun g, int2 *stacks, int cap, int *__restrict__ tail)
             const unsigned back = done & ~ready;
             const unsigned one = __ballot_sync(kFull, nc >= 1), two = __ballot_sync(kFull, nc == 2);
             const int total = __popc(back) + __popc(one) + __popc(two);
+            if (budget < 0) fault |= ST_WALK_LONG;
             if (sp > cap - total) {
                 fault |= ST_WALK_STACK;
             } else {

@@ -39,6 +39,25 @@ def test_particles_at_one_point(gpu, together, angle):
         assert check(s, tree, 0.0, angle) > 0
 
 
+def test_the_deepest_trees(gpu):
+    """About the deepest chain that the tree build makes is walked; one so long that a
+    leaf's walk would take minutes is refused, and the session goes on."""
+    with Session(gpu, params_for(W.c1_config(), abi.FORM_SPLIT, 1.0)) as s:
+        pos, tag = particles(20, 6000)
+        with L.Tree(pos, tag, 16, 1.0) as tree:
+            assert check(s, tree, 0.05, 0.0) > 6000**2 / 2
+        pos, tag = particles(25, 15000)
+        with L.Tree(pos, tag, 16, 1.0) as tree:
+            s.begin(tree.pos, tree.leaf_ipart, tree.leaf_npart)
+            with pytest.raises(P2PError) as e:
+                s.submit_walk(DeviceWalkTree(tree, f"cuda:{gpu}"), 0.05, 0.0)
+            assert e.value.status == abi.P2P_ERR_CAPACITY
+            assert s.lib.p2p_pass_end(s.h, None) == abi.P2P_ERR_CAPACITY
+        pos, tag = particles(12, 0)
+        with L.Tree(pos, tag, 16, 1.0) as tree:
+            check(s, tree, 0.1, 0.0)
+
+
 @pytest.mark.parametrize("name", ["c1", "clustered", "two_leaves"])
 @pytest.mark.parametrize("depths", [1, 3, 96])
 def test_depth_limit_changes_no_row(gpu, name, depths):
