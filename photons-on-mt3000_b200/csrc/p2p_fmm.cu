@@ -533,10 +533,12 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
     if (nnode) {
         int sms = 0;
         FMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device), "FMM walk");
-        int64_t list_cap = std::max(f->limits.list_chunks ? f->limits.list_chunks : 2 * (int64_t)nnode + walk_pool_slack(sms, nleaf),
-                                    (int64_t)(std::min(f->lists[0].cap, f->lists[1].cap) / walk_pool_bytes(1, kWalkChunk)));
-        int64_t task_cap = std::max(f->limits.out_chunks ? f->limits.out_chunks : 3 * (int64_t)nsink / 2 + walk_pool_slack(sms, nsink),
-                                    (int64_t)(f->tasks.cap / walk_pool_bytes(1, kWalkTaskChunk)));
+        const WalkLimits &lim = f->limits;
+        int64_t list_cap = lim.list_chunks ? lim.list_chunks : 2 * (int64_t)nnode + walk_pool_slack(sms, nleaf);
+        int64_t task_cap = lim.out_chunks ? lim.out_chunks : 3 * (int64_t)nsink / 2 + walk_pool_slack(sms, nsink);
+        const size_t lists_held = std::min(f->lists[0].cap, f->lists[1].cap);
+        list_cap = std::max(list_cap, (int64_t)(lists_held / walk_pool_bytes(1, kWalkChunk)));
+        task_cap = std::max(task_cap, (int64_t)(f->tasks.cap / walk_pool_bytes(1, kWalkTaskChunk)));
         g.nnode = nnode;
         g.nleaf = nleaf;
         g.node_first = t->node_first;
@@ -555,7 +557,7 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
         g.items[0] = (WalkItem *)f->items.p;
         g.items[1] = g.items[0] + nleaf;
         g.ctrl = (WalkCtrl *)f->walk_ctrl.p;
-        const int depths = f->limits.depths ? std::min(f->limits.depths, kWalkLevels) : walk_first_depths(nleaf) + kWalkExtraDepths;
+        const int depths = lim.depths ? std::min(lim.depths, kWalkLevels) : walk_first_depths(nleaf) + kWalkExtraDepths;
         bool by_sink = false;  // a deep tree (walk_sink_kernel)
         int stack_cap = kWalkSinkStack;
         for (;;) {
@@ -594,7 +596,8 @@ P2P_API int p2p_fmm_far(p2p_fmm *f, const p2p_walk_tree *t, int npart, const dou
                 if (status || by_sink || boxes[lv] == 0 || lv == depths) break;
             }
             if (status & ST_WALK_TREE) return report_error(P2P_ERR_ARG, "FMM: a child code outside the tree");
-            if (status & ST_WALK_LONG) return report_error(P2P_ERR_CAPACITY, "FMM walk: a leaf's walk met more pairs than it may");
+            if (status & ST_WALK_LONG)
+                return report_error(P2P_ERR_CAPACITY, "FMM walk: a leaf's walk met more pairs than it may");
             if (!status && (by_sink || boxes[lv] == 0)) {
                 f->levels = by_sink ? boxes[0] : lv - (int)std::count(boxes.begin(), boxes.begin() + lv, 0);
                 break;
